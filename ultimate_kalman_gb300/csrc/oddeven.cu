@@ -18,6 +18,10 @@
  *   solve_kernel     one thread per even step: back-substitution and the
  *                    covariance recurrence (Solve_Estimates 614-975)
  *
+ * These are the FP32 kernels and, in FP64 and double-float, those of shapes
+ * with more observation rows than states; up to 8 states FP64 and double-float
+ * run oddeven_small.cuh, from 9 on every form runs oddeven_cta.cuh.
+ *
  * Every "QR, then apply Q^T" of the reference is a Householder triangularization
  * of the pivot block whose reflectors are then streamed over the other columns
  * one column at a time (LAPACK dlarfg sign convention, so R equals LAPACK's up to
@@ -1720,167 +1724,6 @@ __global__ void __launch_bounds__(BS ? BS : 1024) solve_kernel(Args<T, T> a, int
 }
 
 /* ---------------------------------------------------------------------------
- * back-substitution with covariances, register-tiled (n = 4, 6)
- *
- * The same arithmetic as solve_kernel with want_cov, in the same order (the
- * results are equal bit for bit), but R, the reciprocals of its diagonal and
- * the n x n accumulator M live in registers; only F~ and Y (2 n^2 entries) use
- * the thread's shared-memory slice.  solve_kernel's slices (4 n^2 + 4 n
- * entries) hold four warps per SM; here about ten fit, which the FP64 pipe and
- * the double-float arithmetic both need to hide their latencies.
- * ------------------------------------------------------------------------ */
-template <typename T, int N, int BS>
-__global__ void __launch_bounds__(BS) solve_cov_reg_kernel(Args<T, T> a)
-{
-  extern __shared__ unsigned char smem_raw[];
-  T* smem = reinterpret_cast<T*>(smem_raw);
-  const int64_t item = (int64_t)blockIdx.x * BS + threadIdx.x;
-  if (item >= a.ct.nsolve) return;
-  constexpr int nn = N * N;
-  const Rec<T>& Rr = a.cr;
-  const int t = find_track(a.ct.solve, a.ntracks, item);
-  const int64_t e = item - a.ct.solve[t];
-  const int64_t j = 2 * e, L = a.ct.L[t];
-  const bool hp = j > 0, hn = j + 1 < L;
-  const int64_t se = item;
-  const int64_t oj = orig_step(a.track_start, a.level, t, j);
-  const int64_t om = hp ? orig_step(a.track_start, a.level, t, j - 1) : 0;
-  const int64_t op = hn ? orig_step(a.track_start, a.level, t, j + 1) : 0;
-  PVc<T, BS> Fs{smem + threadIdx.x}, Ys = Fs + nn;
-  T R[N][N], dv[N];
-  bool bad = false;
-#pragma unroll
-  for (int c = 0; c < N; ++c)
-#pragma unroll
-    for (int i = 0; i <= c; ++i) R[i][c] = Rr.R.at(c * N + i, se);
-  for (int k = 0; k < nn; ++k) {
-    Fs[k] = hp ? Rr.Ft.at(k, se) : T(0);
-    Ys[k] = hn ? Rr.Y.at(k, se) : T(0);
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    bad |= (R[i][i] == T(0));
-    dv[i] = T(1) / R[i][i];
-  }
-  /* x <- R^{-1} x, the order of solve_upper */
-  auto solve = [&](T (&x)[N]) {
-#pragma unroll
-    for (int jj = N - 1; jj >= 0; --jj) {
-      const T xj = x[jj] * dv[jj];
-      x[jj] = xj;
-#pragma unroll
-      for (int i = 0; i < jj; ++i) x[i] = fma(-xj, R[i][jj], x[i]);
-    }
-  };
-
-  /* state */
-  T pv[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) pv[i] = a.yrhs.p ? a.yrhs.at(i, se) : Rr.rhs.at(i, se);
-  if (hp) {
-    const double* xm = a.state + om * N;
-    for (int k = 0; k < N; ++k) {
-      const T xk = ukg_df::narrow<T>(xm[k]);
-#pragma unroll
-      for (int i = 0; i < N; ++i) pv[i] = fma(-Fs[k * N + i], xk, pv[i]);
-    }
-  }
-  if (hn) {
-    const double* xp = a.state + op * N;
-    for (int k = 0; k < N; ++k) {
-      const T xk = ukg_df::narrow<T>(xp[k]);
-#pragma unroll
-      for (int i = 0; i < N; ++i) pv[i] = fma(-Ys[k * N + i], xk, pv[i]);
-    }
-  }
-  solve(pv);
-  double* xo = a.state + oj * N;
-#pragma unroll
-  for (int i = 0; i < N; ++i) xo[i] = ukg_df::widen(pv[i]);
-
-  const double* Smm = hp ? a.cov + om * nn : nullptr;
-  const double* Spp = hn ? a.cov + op * nn : nullptr;
-  const int64_t smp = (hp && hn) ? a.nt.slot[t] + (j + 1) / 2 : 0; /* U of the next level */
-  T M[N][N]; /* M[c][i]: column c, row i */
-#pragma unroll
-  for (int c = 0; c < N; ++c)
-#pragma unroll
-    for (int i = 0; i < N; ++i) M[c][i] = T(0);
-  const int q0 = hp ? 0 : N, q1 = hn ? 2 * N : N;
-#pragma unroll 1
-  for (int q = q0; q < q1; ++q) {
-    T sg[2 * N];
-    if (q < N) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) sg[i] = ukg_df::narrow<T>(Smm[(int64_t)q * N + i]);
-#pragma unroll
-      for (int i = 0; i < N; ++i) sg[N + i] = hn ? a.nr.U.at(i * N + q, smp) : T(0); /* Smp[q, :] */
-    } else {
-      const int qq = q - N;
-#pragma unroll
-      for (int i = 0; i < N; ++i) sg[i] = hp ? a.nr.U.at(qq * N + i, smp) : T(0);
-#pragma unroll
-      for (int i = 0; i < N; ++i) sg[N + i] = ukg_df::narrow<T>(Spp[(int64_t)qq * N + i]);
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) pv[i] = T(0);
-    if (hp)
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const T sk = sg[k];
-#pragma unroll
-        for (int i = 0; i < N; ++i) pv[i] = fma(Fs[k * N + i], sk, pv[i]);
-      }
-    if (hn)
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const T sk = sg[N + k];
-#pragma unroll
-        for (int i = 0; i < N; ++i) pv[i] = fma(Ys[k * N + i], sk, pv[i]);
-      }
-    PVc<T, BS> bq = q < N ? Fs + q * N : Ys + (q - N) * N; /* column q of B = [F~ | Y] */
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-      const T bc = bq[c];
-#pragma unroll
-      for (int i = 0; i < N; ++i) M[c][i] = fma(pv[i], bc, M[c][i]);
-    }
-    if (a.level == 0) continue; /* level 0's off-diagonal blocks are not needed */
-    solve(pv);
-    if (q < N) { /* cov(x_{j-1}, x_j) = cov(x_j, x_{j-1})^T: row q */
-      const int64_t sU = a.ct.slot[t] + j;
-#pragma unroll
-      for (int i = 0; i < N; ++i) Rr.U.at(i * N + q, sU) = -pv[i];
-    } else {
-      const int64_t sU = a.ct.slot[t] + j + 1;
-#pragma unroll
-      for (int i = 0; i < N; ++i) Rr.U.at((q - N) * N + i, sU) = -pv[i];
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) M[i][i] += T(1);
-  /* S = R^{-1} M R^{-T}: solve the columns, transpose, solve again, transpose */
-#pragma unroll
-  for (int c = 0; c < N; ++c) solve(M[c]);
-#pragma unroll
-  for (int c = 0; c < N; ++c)
-#pragma unroll
-    for (int i = c + 1; i < N; ++i) {
-      const T tmp = M[c][i];
-      M[c][i] = M[i][c];
-      M[i][c] = tmp;
-    }
-#pragma unroll
-  for (int c = 0; c < N; ++c) solve(M[c]);
-  double* So = a.cov + oj * nn;
-#pragma unroll
-  for (int c = 0; c < N; ++c)
-#pragma unroll
-    for (int i = 0; i < N; ++i) So[(int64_t)c * N + i] = ukg_df::widen(M[i][c]);
-  if (bad) atomicOr(a.flag, 2);
-}
-
-/* ---------------------------------------------------------------------------
  * refinement sweep kernels (FP32 factors, FP64 residual)
  * ------------------------------------------------------------------------ */
 
@@ -2349,6 +2192,7 @@ __global__ void add_kernel(double* x, const double* d, int64_t count)
 }
 
 #include "oddeven_cta.cuh"
+#include "oddeven_small.cuh"
 
 /* ---------------------------------------------------------------------------
  * host side: plan, workspace, launches
@@ -2545,14 +2389,14 @@ Eq<T> eq_at(char* B, size_t off, size_t off_m, int64_t stride, int n, int mx)
   return d;
 }
 
-/* The pair and solve kernels used for a state dimension: instantiations with
- * compile-time n, mx and block size for the common small shapes, the
- * runtime-dimension kernels otherwise.                                       */
+/* The pair and solve kernels used for a state dimension: FP32 instantiations
+ * with compile-time n, mx and block size for the common small shapes, the
+ * runtime-dimension kernels otherwise (FP64 and double-float up to 8 states
+ * have their own, SmallKernels below).                                       */
 template <typename T>
 struct Kernels {
   void (*pair)(Args<T, T>, int) = nullptr;
   void (*solve)(Args<T, T>, int) = nullptr;
-  void (*solve_cov)(Args<T, T>) = nullptr; /* register-tiled back-substitution with covariances */
   int bp = 0, bs = 0;     /* fixed block sizes of the specialised kernels (0: pick) */
   size_t pair_smem = 0;   /* dynamic shared memory of the pair kernel (0: per-thread workspace) */
 };
@@ -2573,29 +2417,85 @@ Kernels<T> choose_kernels(int n, int mx, int pair_bp = kPairSsBP)
       k.pair_smem = (size_t)pair_bp * sizeof(float) * (n == 6 ? PairSlice<6, 64>::width : PairSlice<4, 64>::width);
       return k;
     }
+    if (n == mx && n == 8) {
+      k.pair = pair_kernel<T, T, 8, 8, 128>;
+      k.solve = solve_kernel<T, 8, 64>;
+      k.bp = 128;
+      k.bs = 64;
+      return k;
+    }
   }
-  if (n == mx && n == 6) {
-    k.pair = pair_kernel<T, T, 6, 6, 128>;
-    k.solve = solve_kernel<T, 6, 64>;
-    if constexpr (sizeof(T) != sizeof(float)) k.solve_cov = solve_cov_reg_kernel<T, 6, 64>;
-    k.bp = 128;
-    k.bs = 64;
-  } else if (n == mx && n == 4) {
-    k.pair = pair_kernel<T, T, 4, 4, 128>;
-    k.solve = solve_kernel<T, 4, 64>;
-    if constexpr (sizeof(T) != sizeof(float)) k.solve_cov = solve_cov_reg_kernel<T, 4, 64>;
-    k.bp = 128;
-    k.bs = 64;
-  } else if (n == mx && n == 8) {
-    k.pair = pair_kernel<T, T, 8, 8, 128>;
-    k.solve = solve_kernel<T, 8, 64>; /* the register-tiled form spills at n = 8 */
-    k.bp = 128;
-    k.bs = 64;
-  } else {
-    k.pair = pair_kernel<T, T>;
-    k.solve = solve_kernel<T>;
-  }
+  k.pair = pair_kernel<T, T>;
+  k.solve = solve_kernel<T>;
   return k;
+}
+
+/* The FP64 and double-float kernels for n <= 8 and mx == n (oddeven_small.cuh):
+ * lanes or threads per item, by the number of items of a level.             */
+template <typename T>
+struct SmallKernels {
+  void (*pair32)(Args<T, T>) = nullptr;
+  void (*pair8)(Args<T, T>) = nullptr;
+  void (*pair1)(Args<T, T>) = nullptr; /* null: eight lanes at every larger size */
+  void (*tail)(Args<T, T>) = nullptr;
+  void (*solve32)(Args<T, T>) = nullptr;
+  void (*solve1)(Args<T, T>) = nullptr;
+  void (*state)(Args<T, T>) = nullptr;
+};
+constexpr int kPairThreadBS = 128, kSolveThreadBS = 64;
+
+/* The number of items up to which a level takes 32 lanes, then eight, then
+ * one thread per item (n = 6, level time in us against pairs in the level):
+ *   FP64          608   1216   2432   4864   7296   9728  19456
+ *     32 lanes     23     40     70    105    170      -      -
+ *     8 lanes      37     37     40     70    105    130    310
+ *     thread      120    120    120    120    120    125    175
+ *   double-float
+ *     32 lanes     16     19     25     43     65     80    160
+ *     8 lanes      23     23     24     33     40     58    125
+ * (the kernels they replaced, a thread per pair in shared memory: 215-230 and
+ * 150-165).  Steps of 608 = 152 SMs x 4 schedulers: a warp more on a scheduler
+ * is a whole round more of FP64 instructions.  Even steps with covariances:
+ * 32 lanes 14 to 120 us from 608 to 7296, thread 64 throughout.  At n = 7 and
+ * 8 a thread's pivot block does not fit its registers; in double-float eight
+ * lanes stay the fastest at every size (3.8 million pairs: 16.7 ms, against
+ * 19.7 by threads in registers and 21.9 in shared memory).                  */
+template <typename T>
+struct SmallLimits {
+  static constexpr int64_t pair32 = 2432, pair8 = INT64_MAX, solve32 = 7296;
+};
+template <>
+struct SmallLimits<double> {
+  static constexpr int64_t pair32 = 1216, pair8 = 7296, solve32 = 7296;
+};
+
+template <typename T, int N>
+SmallKernels<T> small_kernels_n()
+{
+  SmallKernels<T> k;
+  k.pair32 = small::pair_lanes<T, N, 32>;
+  k.pair8 = small::pair_lanes<T, N, 8>;
+  if constexpr (std::is_same<T, double>::value && N <= 6) k.pair1 = small::pair_thread<T, N, kPairThreadBS, 2>;
+  k.tail = small::tail_lanes<T, N>;
+  k.solve32 = small::solve_lanes<T, N>;
+  k.solve1 = small::solve_thread<T, N, kSolveThreadBS>;
+  k.state = small::solve_state<T, N>;
+  return k;
+}
+template <typename T>
+SmallKernels<T> small_kernels(int n, int mx)
+{
+  if (n != mx) return SmallKernels<T>();
+  switch (n) {
+    case 2: return small_kernels_n<T, 2>();
+    case 3: return small_kernels_n<T, 3>();
+    case 4: return small_kernels_n<T, 4>();
+    case 5: return small_kernels_n<T, 5>();
+    case 6: return small_kernels_n<T, 6>();
+    case 7: return small_kernels_n<T, 7>();
+    case 8: return small_kernels_n<T, 8>();
+    default: return SmallKernels<T>();
+  }
 }
 
 /* Uploads the tables, runs every kernel of the smoother on stream st using
@@ -2608,6 +2508,23 @@ __global__ void upload_tables_kernel(int64_t* __restrict__ dst, const int64_t* _
 {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = src[i];
+}
+
+/* waits for the smoother's kernels and reports its flags */
+int finish_plan(cudaStream_t st, int* dflag)
+{
+  int hflag = 0;
+  cudaMemcpyAsync(&hflag, dflag, sizeof(int), cudaMemcpyDeviceToHost, st);
+  cudaError_t e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return ukg_set_error(KALMAN_GPU_ECUDA, "odd-even smoother: %s", cudaGetErrorString(e));
+  ukg_prof_collect();
+  if (hflag & 8) return ukg_set_error(KALMAN_GPU_ECUDA, "a bulk copy into shared memory did not complete in time");
+  if (hflag & 4) return ukg_set_error(KALMAN_GPU_EINVAL, "malformed input: observation rows outside [0, mmax] or an "
+                                     "unknown covariance type");
+  if (hflag & 1) return ukg_set_error(KALMAN_GPU_ESINGULAR, "a covariance factor is not positive definite");
+  if (hflag & 2) return ukg_set_error(KALMAN_GPU_ESINGULAR, "zero pivot: the smoothing problem is not observable");
+  return 0;
 }
 
 /* tab_dev: the device address of tab when tab is page-locked and mapped (the
@@ -2769,6 +2686,46 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     a.flag = dflag;
     a.baseR = baseR;
   };
+  /* ---- FP64 and double-float, n <= 8: lane and thread kernels ---- */
+  if constexpr (sizeof(T) != sizeof(float)) {
+    const SmallKernels<T> SK = small_kernels<T>(n, mx);
+    if (SK.pair32) {
+      const int lw = small::kLaneWarps, lt = 32 * lw;
+      for (int l = 0; l < nlev; ++l) {
+        Args<T, T> a;
+        memset(&a, 0, sizeof(a));
+        common(a, l);
+        a.ce = l == 0 ? eq0() : eqT(l);
+        if (l + 1 < nlev) a.ne = eqT(l + 1);
+        const int64_t np = lp[l].npairs;
+        if (np > 0) {
+          if (np <= SmallLimits<T>::pair32)
+            UKG_LAUNCH(kPair, st, (SK.pair32<<<grid(np, lw), lt, 0, st>>>(a)));
+          else if (np <= SmallLimits<T>::pair8 || !SK.pair1)
+            UKG_LAUNCH(kPair, st, (SK.pair8<<<grid(np, 4 * lw), lt, 0, st>>>(a)));
+          else
+            UKG_LAUNCH(kPair, st, (SK.pair1<<<grid(np, kPairThreadBS), kPairThreadBS, 0, st>>>(a)));
+        }
+        if (lp[l].ntail > 0) UKG_LAUNCH(kTail, st, (SK.tail<<<grid(lp[l].ntail, lw), lt, 0, st>>>(a)));
+      }
+      const size_t smem_cov = (size_t)kSolveThreadBS * 2 * nn * ts;
+      ukg_allow_dynamic_smem((const void*)SK.solve1);
+      for (int l = nlev - 2; l >= 0; --l) {
+        Args<T, T> a;
+        memset(&a, 0, sizeof(a));
+        common(a, l);
+        const int64_t ns = lp[l].nsolve;
+        if (ns == 0) continue;
+        if (!want_cov)
+          UKG_LAUNCH(kSolve, st, (SK.state<<<grid(ns, 64), 64, 0, st>>>(a)));
+        else if (ns <= SmallLimits<T>::solve32)
+          UKG_LAUNCH(kSolve, st, (SK.solve32<<<grid(ns, lw), lt, 0, st>>>(a)));
+        else
+          UKG_LAUNCH(kSolve, st, (SK.solve1<<<grid(ns, kSolveThreadBS), kSolveThreadBS, smem_cov, st>>>(a)));
+      }
+      return enqueue_only ? 0 : finish_plan(st, dflag);
+    }
+  }
   /* ---- forward elimination ---- */
   for (int l = 0; l < nlev; ++l) {
     Args<T, T> a;
@@ -2803,12 +2760,6 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
         UKG_LAUNCH(kSolve, st, (RS.solve<<<grid(lp[l].nsolve, 128), 128, 0, st>>>(a)));
         continue;
       }
-    }
-    if (want_cov && K.solve_cov) {
-      const size_t smem_cov = (size_t)64 * 2 * nn * ts;
-      ukg_allow_dynamic_smem((const void*)K.solve_cov);
-      UKG_LAUNCH(kSolve, st, (K.solve_cov<<<grid(lp[l].nsolve, 64), 64, smem_cov, st>>>(a)));
-      continue;
     }
     UKG_LAUNCH(kSolve, st, (K.solve<<<grid(lp[l].nsolve, bs), bs, bs * pt_solve, st>>>(a, want_cov ? 1 : 0)));
   }
@@ -2881,19 +2832,7 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
       UKG_LAUNCH(UKG_K_REFINE, st, (add_kernel<<<grid(cnt, 256), 256, 0, st>>>(p->state, dx, cnt)));
     }
   }
-  if (enqueue_only) return 0;
-  int hflag = 0;
-  cudaMemcpyAsync(&hflag, dflag, sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaError_t e = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess) return ukg_set_error(KALMAN_GPU_ECUDA, "odd-even smoother: %s", cudaGetErrorString(e));
-  ukg_prof_collect();
-  if (hflag & 8) return ukg_set_error(KALMAN_GPU_ECUDA, "a bulk copy into shared memory did not complete in time");
-  if (hflag & 4) return ukg_set_error(KALMAN_GPU_EINVAL, "malformed input: observation rows outside [0, mmax] or an "
-                                     "unknown covariance type");
-  if (hflag & 1) return ukg_set_error(KALMAN_GPU_ESINGULAR, "a covariance factor is not positive definite");
-  if (hflag & 2) return ukg_set_error(KALMAN_GPU_ESINGULAR, "zero pivot: the smoothing problem is not observable");
-  return 0;
+  return enqueue_only ? 0 : finish_plan(st, dflag);
 }
 
 /* cached device workspace and plan tables of the ordinary entry point */
