@@ -83,3 +83,40 @@ def test_states_only_and_undetermined_steps():
     X = D.state.cpu().numpy()
     assert np.isnan(X[:2]).all()
     assert np.isfinite(X[2:]).all()
+
+
+@pytest.mark.parametrize("n,m,mmax,kt,ct", [(1, 1, 1, "C", "C"), (3, 2, 8, "w", "F"), (5, 2, 5, "F", "W"),
+                                            (7, 8, 8, "C", "w"), (8, 4, 8, "W", "C")])
+def test_small_states_in_rounds(n, m, mmax, kt, ct):
+    """Up to 8 states the tracks are filtered a round of steps at a time (128 MiB
+    of weighed equations): one track alone (one round) equals the oracle's
+    prefix smoothing, and enough copies of it for several rounds give the
+    same bits."""
+    _cuda()
+    P = pb.random_dynamics([41], n, m, seed=n + 50, per_step=True, missing=0.2, K_type=kt, C_type=ct)
+    if P.mmax < mmax:
+        g = np.zeros((41, n, mmax))
+        g[:, :, :P.mmax] = P.G
+        o = np.zeros((41, mmax))
+        o[:, :P.mmax] = P.o
+        c = np.zeros((41, mmax, mmax))
+        for s in range(41):
+            if P.C_type[s] == ord("w"):
+                c[s].reshape(-1)[:P.mmax] = P.C[s].reshape(-1)[:P.mmax]
+            else:
+                c[s, :P.mmax, :P.mmax] = P.C[s]
+        P = pb.PackedProblem(n, mmax, P.track_start, P.H, P.F, P.c, P.K, P.K_type, g, o, c, P.C_type, P.obs_rows)
+    D = native.DeviceProblem(P, covariance=True)
+    D.filter()
+    X, S = D.results()
+    Q, last = prefixes(P)
+    st, Xo, So = oracle.smooth(Q, "oddeven", covariance=True)
+    assert st == 0
+    assert oracle.rel_err_states(X, Xo[last]) < TOL
+    assert oracle.rel_err_covs(S, So[last]) < TOL
+    T = int((128 << 20) // (8 * ((2 * n + 1) * n + (n + 1) * mmax) * 41)) * 5 // 2 if n >= 7 else 50
+    B = P.select_tracks([0] * T)
+    D = native.DeviceProblem(B, covariance=True)
+    D.filter()
+    Xb, Sb = D.results()
+    assert (Xb.reshape(T, 41, n) == X).all() and (Sb.reshape(T, 41, n, n) == S).all()

@@ -23,11 +23,13 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include <cuda_runtime.h>
 
 #include "cta_linalg.cuh"
+#include "lanes.cuh"
 #include "profiling.h"
 #include "ukgpu_internal.h"
 
@@ -162,269 +164,344 @@ __global__ void __launch_bounds__(NT) filter_cta(FilterArgs a)
 }
 
 /* ---------------------------------------------------------------------------
- * Small states (n, mmax <= 8): one warp per track, lane j holding column j of
- * the current panel in registers (fixed shapes, unused rows exactly zero, so
- * no row counts reach register indices):
- *   evolve panel  rows 0..N-1 the weighed [-F | H | c], rows N..2N-1 the
- *                 carried [R | 0 | y] (zero rows past z), N pivots; rows
- *                 N..2N-1 of columns N..2N are the information on x_i
- *   observe panel rows 0..N-1 that information (shifted to lanes 0..N), rows
- *                 N..N+7 the weighed [G | o] (zero past m), N pivots
- * Reflectors are formed by the pivot column's lane and broadcast by shuffles.
- * Weighing factors, R and R^{-1} for the estimate go through a small
- * per-warp shared-memory area.
+ * Small states (n, mmax <= 8), in three kernels.  Only the QR reductions
+ * depend on the step before; weighing the equations and turning a factor into
+ * an estimate do not, so they run with a thread per step over all tracks and
+ * steps, and the chain that is left is two QR reductions a step:
+ *   filter_weigh     V [-F | H | c] and W [G | o] of every step
+ *   filter_chain     one warp per track, a panel column per lane:
+ *                    evolve  [R 0 y; -VF VH Vc] -> the information on x_i
+ *                    observe [that; WG Wo] -> R, y
+ *   filter_estimate  x = R^{-1} y, P = R^{-1} R^{-T}, in place of the factor
+ * A chain step is n reflectors of 27 FP64 instructions and n of 32 at n = 6,
+ * at 64 to 76 cycles each: 11 to 13 us, and 16 us with the shuffles between
+ * them; with the weighing and the estimate inside the chain it was 42 us.  512
+ * tracks of 50 to 500 steps: 21.2 ms before, 8.2 ms now.
+ *
+ * Tracks are taken kc steps at a time (the weighed equations of a round must
+ * fit the workspace); the factor is carried over between rounds.
  * ------------------------------------------------------------------------ */
 constexpr int kWarpsPerBlock = 4;
-constexpr int kWarpMaxN = 8;
+constexpr int kSmallN = 8;
+constexpr int64_t kRoundBytes = (int64_t)128 << 20; /* 140,000 steps of 6 states: about what L2 holds */
 
-/* QR with NP pivots of the panel held as one column per lane (R rows, NC
- * columns: lanes from NC on hold nothing and stay idle) */
-template <int R, int NP, int NC>
-__device__ __forceinline__ void warp_qr(double (&col)[R], int lane)
-{
-#pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    double tail = 0.0;
-#pragma unroll
-    for (int i = k + 1; i < R; ++i) tail = fma(col[i], col[i], tail);
-    tail = __shfl_sync(0xffffffffu, tail, k);
-    const double alpha = __shfl_sync(0xffffffffu, col[k], k);
-    if (tail == 0.0) continue; /* identity reflector: uniform over the warp */
-    const double beta = -copysign(sqrt(fma(alpha, alpha, tail)), alpha);
-    const double amb = alpha - beta;
-    const double inv = 1.0 / (beta * amb);
-    const double t = -(amb * amb) * inv, scale = beta * inv;
-    double v[R];
-#pragma unroll
-    for (int i = k + 1; i < R; ++i) v[i] = __shfl_sync(0xffffffffu, col[i], k) * scale;
-    if (lane == k) {
-      col[k] = beta;
-#pragma unroll
-      for (int i = k + 1; i < R; ++i) col[i] = v[i];
-    } else if (lane > k && lane < NC) {
-      double d = col[k];
-#pragma unroll
-      for (int i = k + 1; i < R; ++i) d = fma(v[i], col[i], d);
-      d *= t;
-      col[k] -= d;
-#pragma unroll
-      for (int i = k + 1; i < R; ++i) col[i] = fma(-d, v[i], col[i]);
-    }
-  }
-}
+/* entries of a step's weighed equations: columns of [-F | H | c], n rows each,
+ * then columns of [G | o], mmax rows each (zero past the step's rows) */
+__host__ __device__ constexpr int step_entries(int n, int mmax) { return (2 * n + 1) * n + (n + 1) * mmax; }
 
-/* rows r0 .. r0+rows-1 of this lane's column <- V (those rows) for the factor
- * of a covariance (column-major, ld ldc): 'W' W x, 'w' diag x, 'C'
- * chol(cov)^{-1} x, 'U'/'F' tril(cov)^{-1} x.  sL: rows^2 doubles of the
- * warp's shared area.  Returns false for a factor that is not positive
- * definite or has a zero pivot (the same in every lane). */
-template <int R, int R0, int MAXR>
-__device__ __forceinline__ bool warp_weigh(double (&col)[R], char type, const double* cov, int ldc, int rows,
-                                           double* sL, double* sInv, int lane, int ncols)
-{
-  bool ok = true;
-  const bool act = lane < ncols; /* lanes past the panel's columns hold zeros */
-  if (type == 'w') {
+struct SmallArgs {
+  double* weighed;  /* [ntracks][kc][step_entries] */
+  double* factor;   /* [ntracks][kc][n * n] where no covariances are asked for, else null: in place of P */
+  double* carry;    /* [ntracks][(n + 1) * n] */
+  int* carry_rows;  /* [ntracks] */
+  int64_t first, kc; /* steps first .. first + kc - 1 of every track */
+};
+
+/* Weighing of one covariance factor by one thread: the lower factor L and the
+ * reciprocals d of its diagonal ('C' Cholesky, 'U'/'F' the lower triangle),
+ * the matrix ('W') or the weights ('w', in d); rows <= R.                    */
+template <int R>
+struct ThreadWeights {
+  double L[R][R], d[R]; /* L[j][i]: column j, row i */
+  char type;
+
+  __device__ __forceinline__ bool prepare(char t, const double* cov, int ld, int rows)
+  {
+    type = t;
+    bool ok = true;
+    if (t == 'w') {
 #pragma unroll
-    for (int i = 0; i < MAXR; ++i)
-      if (act && i < rows) col[R0 + i] *= cov[i];
-    return true;
-  }
-  if (type == 'W') {
-    if (!act) return true;
-    double x[MAXR];
-#pragma unroll
-    for (int i = 0; i < MAXR; ++i) {
-      double sm = 0.0;
-#pragma unroll
-      for (int k = 0; k < MAXR; ++k)
-        if (i < rows && k < rows) sm = fma(cov[(int64_t)k * ldc + i], col[R0 + k], sm);
-      x[i] = sm;
+      for (int i = 0; i < R; ++i) d[i] = i < rows ? cov[i] : 0.0;
+      return true;
     }
 #pragma unroll
-    for (int i = 0; i < MAXR; ++i)
-      if (i < rows) col[R0 + i] = x[i];
-    return true;
-  }
-  if (type != 'C' && type != 'U' && type != 'F') return true;
-  /* the factor, column-major rows x rows, lower triangle */
-  for (int e = lane; e < rows * rows; e += 32) {
-    const int j = e / rows, i = e - j * rows;
-    sL[e] = i >= j ? cov[(int64_t)j * ldc + i] : 0.0;
-  }
-  __syncwarp();
-  if (type == 'C') {
-    if (lane == 0) /* Cholesky by one lane: at most 8 x 8; one division per column */
-      for (int j = 0; j < rows; ++j) {
-        double d = sL[j * rows + j];
-        for (int k = 0; k < j; ++k) d = fma(-sL[k * rows + j], sL[k * rows + j], d);
-        const bool pd = d > 0.0;
-        const double ljj = pd ? sqrt(d) : 1.0;
-        const double ri = 1.0 / ljj;
-        sL[j * rows + j] = pd ? ljj : -1.0; /* -1 marks a failed pivot (sqrt >= 0 otherwise) */
-        sInv[j] = ri;
-        for (int i = j + 1; i < rows; ++i) {
-          double x = sL[j * rows + i];
-          for (int k = 0; k < j; ++k) x = fma(-sL[k * rows + i], sL[k * rows + j], x);
-          sL[j * rows + i] = x * ri;
+    for (int j = 0; j < R; ++j)
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        L[j][i] = i < rows && j < rows && (t == 'W' || i >= j) ? cov[(int64_t)j * ld + i] : 0.0;
+    if (t == 'W') return true;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      if (t == 'C') {
+        double s = L[j][j];
+#pragma unroll
+        for (int k = 0; k < j; ++k) s = fma(-L[k][j], L[k][j], s);
+        const bool pd = s > 0.0;
+        if (j < rows && !pd) ok = false;
+        d[j] = !pd ? 1.0 : lanes::series_range(s) ? lanes::rsqrt_series(s) : 1.0 / sqrt(s);
+#pragma unroll
+        for (int i = j + 1; i < R; ++i) {
+          double x = L[j][i];
+#pragma unroll
+          for (int k = 0; k < j; ++k) x = fma(-L[k][i], L[k][j], x);
+          L[j][i] = x * d[j];
         }
+      } else {
+        if (j < rows && L[j][j] == 0.0) ok = false;
+        d[j] = j < rows ? lanes::recip(L[j][j]) : 1.0;
       }
-    __syncwarp();
-    for (int j = 0; j < rows; ++j)
-      if (sL[j * rows + j] < 0.0) ok = false;
-  } else {
-    if (lane < rows) sInv[lane] = 1.0 / sL[lane * rows + lane];
-    __syncwarp();
-    for (int j = 0; j < rows; ++j)
-      if (sL[j * rows + j] == 0.0) ok = false;
-  }
-  /* forward substitution on this lane's rows */
-#pragma unroll
-  for (int i = 0; i < MAXR; ++i)
-    if (act && i < rows) {
-      double x = col[R0 + i];
-#pragma unroll
-      for (int k = 0; k < MAXR; ++k)
-        if (k < i) x = fma(-sL[k * rows + i], col[R0 + k], x);
-      col[R0 + i] = x * sInv[i];
     }
-  __syncwarp();
-  return ok;
-}
+    return ok;
+  }
+  __device__ __forceinline__ void apply(double (&x)[R]) const
+  {
+    if (type == 'w') {
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[i] *= d[i];
+    } else if (type == 'W') {
+      double y[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        y[i] = 0.0;
+#pragma unroll
+        for (int k = 0; k < R; ++k) y[i] = fma(L[k][i], x[k], y[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[i] = y[i];
+    } else if (type == 'C' || type == 'U' || type == 'F') {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        x[j] *= d[j];
+#pragma unroll
+        for (int i = j + 1; i < R; ++i) x[i] = fma(-x[j], L[j][i], x[i]);
+      }
+    }
+  }
+};
 
-template <int N>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_warp(FilterArgs a)
+template <int N, int M>
+__global__ void __launch_bounds__(64) filter_weigh(FilterArgs a, SmallArgs w)
 {
-  constexpr int RE = 2 * N, RO = N + kWarpMaxN;
-  __shared__ double area[kWarpsPerBlock][kWarpMaxN * kWarpMaxN + 2 * N * N + N + kWarpMaxN + N];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int t = blockIdx.x * kWarpsPerBlock + w;
-  if (t >= a.ntracks) return; /* uniform over the warp */
-  double* sL = area[w];
-  double* sR = sL + kWarpMaxN * kWarpMaxN; /* R, column-major N x N */
-  double* sRi = sR + N * N;                 /* R^{-1}, column-major */
-  double* sy = sRi + N * N;
-  double* sInv = sy + N;          /* reciprocal pivots of the weighing factor */
-  double* sInvR = sInv + kWarpMaxN; /* reciprocal diagonal of R */
+  const int64_t e = (int64_t)blockIdx.x * 64 + threadIdx.x;
+  const int t = (int)(e / w.kc);
+  if (t >= a.ntracks) return;
+  const int64_t s0 = a.track_start[t], s = s0 + w.first + (e - t * w.kc);
+  if (s >= a.track_start[t + 1]) return;
   const int mm = a.mmax;
   const int64_t nn = (int64_t)N * N;
-  const int64_t s0 = a.track_start[t], s1 = a.track_start[t + 1];
-  double Rc[N]; /* this lane's column of the carried [R | y] (lanes 0..N), zero rows past z */
-#pragma unroll
-  for (int r = 0; r < N; ++r) Rc[r] = 0.0;
-  int z = 0;
+  double* out = w.weighed + e * step_entries(N, mm);
   int flag = 0;
-  for (int64_t s = s0; s < s1; ++s) {
-    double oc[RO]; /* the observe panel: lanes 0..N-1 R~'s columns, lane N y~ */
-    if (s > s0) {
-      double ec[RE];
-      /* rows 0..N-1: [-F | H | c] of step s; rows N..2N-1: [R | 0 | y] */
+  if (s > s0) {
+    ThreadWeights<N> V;
+    const char kt = a.K_type[s];
+    if (!cta::valid_cov_type(kt)) flag |= 4;
+    if (!V.prepare(kt, a.K + s * nn, N, N)) flag |= 1;
+#pragma unroll 1
+    for (int c = 0; c <= 2 * N; ++c) {
+      const double* src = c < N ? a.F + s * nn + c * N : c < 2 * N ? a.H + s * nn + (c - N) * N : a.c + s * N;
+      double x[N];
 #pragma unroll
-      for (int r = 0; r < N; ++r) {
-        double v = 0.0;
-        if (lane < N) v = -a.F[s * nn + (int64_t)lane * N + r];
-        else if (lane < 2 * N) v = a.H[s * nn + (int64_t)(lane - N) * N + r];
-        else if (lane == 2 * N) v = a.c[s * N + r];
-        ec[r] = v;
-      }
+      for (int i = 0; i < N; ++i) x[i] = c < N ? -src[i] : src[i];
+      V.apply(x);
 #pragma unroll
-      for (int r = 0; r < N; ++r) {
-        const double yr = __shfl_sync(0xffffffffu, Rc[r], N);
-        ec[N + r] = lane < N ? Rc[r] : lane == 2 * N ? yr : 0.0;
-      }
-      const char kt = a.K_type[s];
-      if (!cta::valid_cov_type(kt)) flag |= 4;
-      if (!warp_weigh<RE, 0, N>(ec, kt, a.K + s * nn, N, N, sL, sInv, lane, 2 * N + 1)) flag |= 1;
-      warp_qr<RE, N, 2 * N + 1>(ec, lane);
-      /* rows N..2N-1 of lanes N..2N -> lanes 0..N */
-#pragma unroll
-      for (int r = 0; r < N; ++r) oc[r] = __shfl_sync(0xffffffffu, ec[N + r], (lane + N) & 31);
-      if (lane > N) {
-#pragma unroll
-        for (int r = 0; r < N; ++r) oc[r] = 0.0;
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < N; ++r) oc[r] = 0.0;
+      for (int i = 0; i < N; ++i) out[c * N + i] = x[i];
     }
-    int m = a.obs_rows[s];
-    if (m < 0 || m > mm || m > kWarpMaxN) {
-      flag |= 4;
-      m = 0;
-    }
-#pragma unroll
-    for (int r = 0; r < kWarpMaxN; ++r) {
-      double v = 0.0;
-      if (r < m) {
-        if (lane < N) v = a.G[s * (int64_t)mm * N + (int64_t)lane * mm + r];
-        else if (lane == N) v = a.o[s * mm + r];
-      }
-      oc[N + r] = v;
-    }
-    if (m > 0) {
-      const char ct = a.C_type[s];
-      if (!cta::valid_cov_type(ct)) flag |= 4;
-      if (!warp_weigh<RO, N, kWarpMaxN>(oc, ct, a.C + s * (int64_t)mm * mm, mm, m, sL, sInv, lane, N + 1)) flag |= 1;
-    }
-    warp_qr<RO, N, N + 1>(oc, lane);
-#pragma unroll
-    for (int r = 0; r < N; ++r) Rc[r] = (lane <= N && (lane == N || r <= lane)) ? oc[r] : 0.0;
-    z = z + m < N ? z + m : N;
-    /* estimate */
-    double* x = a.state + s * N;
-    double* P = a.cov ? a.cov + s * nn : nullptr;
-    bool det = z == N;
-    if (lane < N) {
-#pragma unroll
-      for (int r = 0; r < N; ++r) sR[lane * N + r] = Rc[r];
-    } else if (lane == N) {
-#pragma unroll
-      for (int r = 0; r < N; ++r) sy[r] = Rc[r];
-    }
-    __syncwarp();
-    for (int i = 0; i < N; ++i)
-      if (sR[i * N + i] == 0.0) det = false;
-    if (!det) {
-      if (lane < N) x[lane] = NAN;
-      if (P)
-        for (int e = lane; e < N * N; e += 32) P[e] = NAN;
-      flag |= 1;
-      __syncwarp();
-      continue;
-    }
-    if (lane < N) sInvR[lane] = 1.0 / sR[lane * N + lane];
-    __syncwarp();
-    if (lane < N) { /* column lane of R^{-1}: R u = e_lane */
-      double u[N];
-#pragma unroll
-      for (int i = N - 1; i >= 0; --i) {
-        double v = i == lane ? 1.0 : 0.0;
-#pragma unroll
-        for (int k = i + 1; k < N; ++k) v = fma(-sR[k * N + i], u[k], v);
-        u[i] = v * sInvR[i];
-      }
-#pragma unroll
-      for (int i = 0; i < N; ++i) sRi[lane * N + i] = u[i];
-    }
-    __syncwarp();
-    if (lane < N) {
-      double xi = 0.0;
-#pragma unroll
-      for (int k = 0; k < N; ++k) xi = fma(sRi[k * N + lane], sy[k], xi);
-      x[lane] = xi;
-      if (P) { /* P(:, lane) = sum_k Ri(:, k) Ri(lane, k) */
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-          double sm = 0.0;
-#pragma unroll
-          for (int k = 0; k < N; ++k) sm = fma(sRi[k * N + i], sRi[k * N + lane], sm);
-          P[(int64_t)lane * N + i] = sm;
-        }
-      }
-    }
-    __syncwarp();
   }
-  if (flag && lane == 0) atomicOr(a.flag, flag);
+  int m = a.obs_rows[s];
+  if (m < 0 || m > mm) {
+    flag |= 4;
+    m = 0;
+  }
+  out += (2 * N + 1) * N;
+  if (m == 0) { /* the chain reads all mmax rows */
+    for (int i = 0; i < (N + 1) * mm; ++i) out[i] = 0.0;
+  } else {
+    ThreadWeights<M> W;
+    const char ct = a.C_type[s];
+    if (!cta::valid_cov_type(ct)) flag |= 4;
+    if (!W.prepare(ct, a.C + s * (int64_t)mm * mm, mm, m)) flag |= 1;
+#pragma unroll 1
+    for (int c = 0; c <= N; ++c) {
+      const double* src = c < N ? a.G + s * (int64_t)mm * N + (int64_t)c * mm : a.o + s * mm;
+      double x[M];
+#pragma unroll
+      for (int i = 0; i < M; ++i) x[i] = i < m ? src[i] : 0.0;
+      W.apply(x);
+#pragma unroll
+      for (int i = 0; i < M; ++i)
+        if (i < mm) out[c * mm + i] = i < m ? x[i] : 0.0;
+    }
+  }
+  if (flag) atomicOr(a.flag, flag);
+}
+
+/* The factor's z rows (all n in the usual case) are carried on lanes 0..N
+ * ([R | y], zero rows past z).  With z = n the triangle R is on top of the
+ * weighed evolution; before that the evolution is on top and R's rows below,
+ * whose zero rows stay exactly zero.  Either way the lower rows of the columns
+ * N..2N become the information on x_i.                                       */
+template <int N, int M>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a, SmallArgs w)
+{
+  const int lane = threadIdx.x & 31;
+  const int t = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (t >= a.ntracks) return; /* the whole warp */
+  const unsigned all = 0xffffffffu;
+  const int mm = a.mmax, per = step_entries(N, mm);
+  const int64_t s0 = a.track_start[t] + w.first;
+  const int64_t cnt = a.track_start[t + 1] - s0 < w.kc ? a.track_start[t + 1] - s0 : w.kc;
+  if (cnt <= 0) return;
+  double R[N]; /* this lane's column of [R | y] */
+  int z = 0;
+#pragma unroll
+  for (int r = 0; r < N; ++r) R[r] = 0.0;
+  if (w.first > 0) {
+    z = w.carry_rows[t];
+    if (lane <= N)
+#pragma unroll
+      for (int r = 0; r < N; ++r) R[r] = w.carry[((int64_t)t * (N + 1) + lane) * N + r];
+  }
+  const double* in = w.weighed + (int64_t)t * w.kc * per;
+  const int64_t nn = (int64_t)N * N;
+  double e[N], g[M]; /* the step's columns, loaded a step ahead */
+  int m = 0;
+  auto load = [&](int64_t q) {
+    const double* p = in + q * per;
+    if (lane <= 2 * N && (w.first > 0 || q > 0))
+#pragma unroll
+      for (int r = 0; r < N; ++r) e[r] = p[lane * N + r];
+    if (lane <= N)
+#pragma unroll
+      for (int r = 0; r < M; ++r)
+        if (r < mm) g[r] = p[(2 * N + 1) * N + lane * mm + r];
+    m = a.obs_rows[s0 + q];
+    if (m < 0 || m > mm) m = 0; /* reported by the weighing */
+  };
+#pragma unroll
+  for (int r = 0; r < N; ++r) e[r] = 0.0;
+#pragma unroll
+  for (int r = 0; r < M; ++r) g[r] = 0.0;
+  load(0);
+  for (int64_t q = 0; q < cnt; ++q) {
+    double tp[1][N], bt[1][N], bo[1][M];
+    const int mq = m;
+    const bool tri = z == N;
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      const double y = __shfl_sync(all, R[r], N);
+      const double c = lane < N ? R[r] : lane == 2 * N ? y : 0.0;
+      tp[0][r] = tri ? c : e[r];
+      bt[0][r] = tri ? e[r] : c;
+    }
+#pragma unroll
+    for (int r = 0; r < M; ++r) bo[0][r] = g[r];
+    if (q + 1 < cnt) load(q + 1);
+    if (w.first + q > 0) {
+      if (tri) lanes::lanes_qr_tri<double, N, 32, 1>(tp, bt, all, lane, 0, N);
+      else lanes::lanes_qr_full<double, N, 32, 1, N>(tp, bt, all, lane, 0, N);
+#pragma unroll
+      for (int r = 0; r < N; ++r) {
+        const double v = __shfl_sync(all, bt[0][r], (lane + N) & 31);
+        tp[0][r] = lane <= N ? v : 0.0;
+      }
+    } else { /* a track's first step has no evolution */
+#pragma unroll
+      for (int r = 0; r < N; ++r) tp[0][r] = 0.0;
+    }
+    z = z + mq < N ? z + mq : N;
+    lanes::lanes_qr_full<double, N, 32, 1, M>(tp, bo, all, lane, 0, z);
+    double* Ro = a.cov ? a.cov + (s0 + q) * nn : w.factor + ((int64_t)t * w.kc + q) * nn;
+#pragma unroll
+    for (int r = 0; r < N; ++r) R[r] = lane <= N && r <= lane && r < z ? tp[0][r] : 0.0;
+    double* out = lane < N ? Ro + lane * N : a.state + (s0 + q) * N;
+    if (lane <= N)
+#pragma unroll
+      for (int r = 0; r < N; ++r) out[r] = R[r];
+  }
+  if (lane <= N)
+#pragma unroll
+    for (int r = 0; r < N; ++r) w.carry[((int64_t)t * (N + 1) + lane) * N + r] = R[r];
+  if (lane == 0) w.carry_rows[t] = z;
+}
+
+/* x = R^{-1} y and P = R^{-1} R^{-T} of a step, over the factor that the chain
+ * left in the outputs; a zero on R's diagonal (fewer than n rows, or a zero
+ * pivot) is an undetermined state                                           */
+template <int N>
+__global__ void __launch_bounds__(64) filter_estimate(FilterArgs a, SmallArgs w)
+{
+  const int64_t e = (int64_t)blockIdx.x * 64 + threadIdx.x;
+  const int t = (int)(e / w.kc);
+  if (t >= a.ntracks) return;
+  const int64_t s = a.track_start[t] + w.first + (e - t * w.kc);
+  if (s >= a.track_start[t + 1]) return;
+  const int64_t nn = (int64_t)N * N;
+  double* P = a.cov ? a.cov + s * nn : nullptr;
+  const double* Rp = P ? P : w.factor + e * nn;
+  double* x = a.state + s * N;
+  double R[N][N], d[N], y[N]; /* R[j][i]: column j, row i <= j */
+  bool det = true;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    y[j] = x[j];
+#pragma unroll
+    for (int i = 0; i <= j; ++i) R[j][i] = Rp[j * N + i];
+    det = det && R[j][j] != 0.0;
+  }
+  if (!det) {
+    for (int i = 0; i < N; ++i) x[i] = NAN;
+    if (P)
+      for (int i = 0; i < N * N; ++i) P[i] = NAN;
+    atomicOr(a.flag, 1);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) d[j] = lanes::recip(R[j][j]);
+#pragma unroll
+  for (int j = N - 1; j >= 0; --j) {
+    y[j] *= d[j];
+#pragma unroll
+    for (int i = 0; i < j; ++i) y[i] = fma(-y[j], R[j][i], y[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = y[i];
+  if (!P) return;
+  /* R <- R^{-1} column by column (column j of the inverse needs R's columns up to j), last column first */
+#pragma unroll
+  for (int j = N - 1; j >= 0; --j) {
+    double u[N];
+    u[j] = d[j];
+#pragma unroll
+    for (int i = 0; i < j; ++i) u[i] = -R[j][i] * d[j];
+#pragma unroll
+    for (int k = j - 1; k >= 0; --k) {
+      u[k] *= d[k];
+#pragma unroll
+      for (int i = 0; i < k; ++i) u[i] = fma(-u[k], R[k][i], u[i]);
+    }
+#pragma unroll
+    for (int i = 0; i <= j; ++i) R[j][i] = u[i];
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int i = j; i < N; ++i) {
+      double sm = 0.0;
+#pragma unroll
+      for (int k = i; k < N; ++k) sm = fma(R[k][i], R[k][j], sm);
+      P[j * N + i] = sm;
+      P[i * N + j] = sm;
+    }
+}
+
+template <int N, int M>
+void filter_small_nm(const FilterArgs& a, SmallArgs w, int64_t longest, cudaStream_t st)
+{
+  const unsigned chain = (unsigned)((a.ntracks + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  const unsigned steps = (unsigned)((a.ntracks * w.kc + 63) / 64);
+  for (w.first = 0; w.first < longest; w.first += w.kc) {
+    UKG_LAUNCH(UKG_K_FILTER, st, (filter_weigh<N, M><<<steps, 64, 0, st>>>(a, w)));
+    UKG_LAUNCH(UKG_K_FILTER, st, (filter_chain<N, M><<<chain, 32 * kWarpsPerBlock, 0, st>>>(a, w)));
+    UKG_LAUNCH(UKG_K_FILTER, st, (filter_estimate<N><<<steps, 64, 0, st>>>(a, w)));
+  }
+}
+/* observation rows in registers: half of n, n or 8 */
+template <int N>
+void filter_small_n(const FilterArgs& a, const SmallArgs& w, int64_t longest, cudaStream_t st)
+{
+  if (a.mmax <= (N + 1) / 2) filter_small_nm<N, (N + 1) / 2>(a, w, longest, st);
+  else if (a.mmax <= N) filter_small_nm<N, N>(a, w, longest, st);
+  else filter_small_nm<N, kSmallN>(a, w, longest, st);
 }
 
 struct Workspace {
@@ -448,6 +525,8 @@ int ensure(size_t bytes)
 }
 
 }  // namespace
+
+extern "C" int64_t ukg_filter_workspace_held(void) { return (int64_t)tl_ws.bytes; }
 
 extern "C" void ukg_release_filter_workspace(void)
 {
@@ -473,7 +552,22 @@ extern "C" int kalman_gpu_filter_packed(uint32_t options, const kalman_gpu_probl
   const int ncta = p->ntracks < sms * 4 ? p->ntracks : sms * 4;
   const int64_t per = filter_scratch(p->n, p->mmax);
   const size_t tab = ((size_t)(p->ntracks + 1) * sizeof(int64_t) + 255) / 256 * 256;
-  if (int e = ensure(tab + 256 + (size_t)ncta * per * sizeof(double))) return e;
+  const bool small = p->n <= kSmallN && p->mmax <= kSmallN;
+  SmallArgs w;
+  memset(&w, 0, sizeof(w));
+  int64_t longest = 0;
+  size_t scratch = (size_t)ncta * per;
+  if (small) { /* steps of every track at a time: at most kRoundBytes of weighed equations */
+    for (int t = 0; t < p->ntracks; ++t) {
+      const int64_t k = p->track_start[t + 1] - p->track_start[t];
+      longest = k > longest ? k : longest;
+    }
+    const int64_t step = step_entries(p->n, p->mmax) + (want_cov ? 0 : p->n * p->n);
+    w.kc = kRoundBytes / ((int64_t)sizeof(double) * step * p->ntracks);
+    w.kc = w.kc < 1 ? 1 : w.kc < longest ? w.kc : longest;
+    scratch = (size_t)p->ntracks * (w.kc * step + (p->n + 1) * p->n + 1);
+  }
+  if (int e = ensure(tab + 256 + scratch * sizeof(double))) return e;
   char* base = (char*)tl_ws.p;
   int64_t* dts = (int64_t*)base;
   int* dflag = (int*)(base + tab);
@@ -499,18 +593,21 @@ extern "C" int kalman_gpu_filter_packed(uint32_t options, const kalman_gpu_probl
   a.scratch = (double*)(base + tab + 256);
   a.per_cta = per;
   a.flag = dflag;
-  if (p->n <= kWarpMaxN && p->mmax <= kWarpMaxN) {
-    const unsigned blocks = (unsigned)((p->ntracks + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    const int bs = 32 * kWarpsPerBlock;
+  if (small) {
+    const int64_t T = p->ntracks;
+    w.weighed = a.scratch;
+    w.carry = w.weighed + T * w.kc * step_entries(p->n, p->mmax);
+    w.factor = w.carry + T * (p->n + 1) * p->n;
+    w.carry_rows = (int*)(w.factor + (want_cov ? 0 : T * w.kc * p->n * p->n));
     switch (p->n) {
-      case 1: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<1><<<blocks, bs, 0, st>>>(a))); break;
-      case 2: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<2><<<blocks, bs, 0, st>>>(a))); break;
-      case 3: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<3><<<blocks, bs, 0, st>>>(a))); break;
-      case 4: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<4><<<blocks, bs, 0, st>>>(a))); break;
-      case 5: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<5><<<blocks, bs, 0, st>>>(a))); break;
-      case 6: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<6><<<blocks, bs, 0, st>>>(a))); break;
-      case 7: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<7><<<blocks, bs, 0, st>>>(a))); break;
-      default: UKG_LAUNCH(UKG_K_FILTER, st, (filter_warp<8><<<blocks, bs, 0, st>>>(a))); break;
+      case 1: filter_small_n<1>(a, w, longest, st); break;
+      case 2: filter_small_n<2>(a, w, longest, st); break;
+      case 3: filter_small_n<3>(a, w, longest, st); break;
+      case 4: filter_small_n<4>(a, w, longest, st); break;
+      case 5: filter_small_n<5>(a, w, longest, st); break;
+      case 6: filter_small_n<6>(a, w, longest, st); break;
+      case 7: filter_small_n<7>(a, w, longest, st); break;
+      default: filter_small_n<8>(a, w, longest, st); break;
     }
   } else {
     UKG_LAUNCH(UKG_K_FILTER, st, (filter_cta<<<ncta, NT, 0, st>>>(a)));

@@ -417,6 +417,7 @@ extern "C" void ukg_release_oddeven_workspace(void);
 extern "C" void ukg_release_associative_workspace(void);
 extern "C" int64_t ukg_oddeven_workspace_held(void);
 extern "C" int64_t ukg_associative_workspace_held(void);
+extern "C" int64_t ukg_filter_workspace_held(void);
 
 extern "C" void ukg_allow_dynamic_smem(const void* kernel)
 {
@@ -462,8 +463,8 @@ extern "C" int ukg_malloc_async(void** ptr, size_t bytes, void* cuda_stream)
 
 extern "C" int64_t kalman_gpu_workspace_held(void)
 {
-  return ukg_oddeven_workspace_held() + ukg_associative_workspace_held() + (int64_t)tl_stage.bytes +
-         (int64_t)tl_pad.bytes;
+  return ukg_oddeven_workspace_held() + ukg_associative_workspace_held() + ukg_filter_workspace_held() +
+         (int64_t)tl_stage.bytes + (int64_t)tl_pad.bytes;
 }
 
 namespace {
