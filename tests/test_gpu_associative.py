@@ -121,3 +121,19 @@ def test_n48_m24_long_track_with_missing_observations(parity_log):
     assert (P.obs_rows[1:] == 0).sum() > 50
     X, S = native.smooth(P, algorithm="associative")
     check(P, X, S, parity_log, "n=48 k=2000 5% missing")
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (2, 1), (3, 3), (5, 2), (7, 4), (8, 4)])
+@pytest.mark.parametrize("k", [2, 3, 6, 33])
+def test_small_states_all_lengths(n, m, k):
+    """The warp-per-combine scans at every group width (n = 8 fills the warp)
+    and at lengths with and without carried elements, alone and among others."""
+    P = pb.random_dynamics([k], n, m, seed=n + 10 * k, per_step=True, missing=0.2)
+    X, S = native.smooth(P, "associative")
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    assert oracle.rel_err_states(X, Xo) < 1e-11
+    assert oracle.rel_err_covs(S, So) < 1e-11
+    Xb, Sb = native.smooth(P.select_tracks([0] * 37), "associative")
+    np.testing.assert_array_equal(Xb[36 * k:], X)
+    np.testing.assert_array_equal(Sb[36 * k:], S)

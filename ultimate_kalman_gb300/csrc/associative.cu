@@ -23,9 +23,10 @@
  * e = 0, J = 0 (the reference dereferences NULL); an unobserved step 1 gets
  * b = F m0 + c (the reference computes m0 + c).
  *
- * One thread per item; its n x n temporaries live in shared memory,
- * interleaved across the block's threads (element e of thread t at
- * smem[e*blockDim + t]).  Element arrays are element-major (SoA) so that
+ * Up to 8 states an element is built by one thread, its n x n temporaries in
+ * shared memory, interleaved across the block's threads (element e of thread t
+ * at smem[e*blockDim + t]), and combined by a warp (associative_small.cuh);
+ * from 9 on a thread block takes an item (associative_cta.cuh).  Element arrays are element-major (SoA) so that
  * consecutive threads touch consecutive addresses.
  */
 #include <cuda_runtime.h>
@@ -37,6 +38,7 @@
 
 #include "profiling.h"
 #include "cta_linalg.cuh"
+#include "lanes.cuh"
 #include "ukgpu_internal.h"
 
 namespace {
@@ -466,166 +468,6 @@ __global__ void element_kernel(Args a, Raw raw, FElems out, const int64_t* seq_s
   if (bad) atomicOr(a.flag, 2);
 }
 
-/* ---------------------------------------------------------------------------
- * the two associative operations.  `out` may alias `sj` (never `si`): every
- * entry of sj is read before the entry of out at the same place is written.
- * ------------------------------------------------------------------------ */
-__device__ bool combine_filter(int n, const FElems& Xi, int64_t i, const FElems& Xj, int64_t j, const FElems& O,
-                               int64_t o, PV ws)
-{
-  /* ws: W (2n*n) | Xm (n*n) | Ym (n*n) | T (n*n) | v (n) */
-  PV W = ws, Xm = ws + 2 * n * n, Ym = Xm + n * n, T = Ym + n * n, v = T + n * n;
-  bool bad = false;
-  /* W = [(I + Zi Jj)^T | Aj^T]; the solve leaves X^T = (I + Zi Jj)^{-T} Aj^T */
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = (p == q) ? 1.0 : 0.0; /* (I + Zi Jj)(q, p) */
-      for (int k = 0; k < n; ++k) s = fma(Xi.Z.at(k * n + q, i), Xj.J.at(p * n + k, j), s);
-      W[q * n + p] = s;                           /* W(p, q) = M(q, p) */
-      W[(n + q) * n + p] = Xj.A.at(p * n + q, j); /* Aj^T(p, q)        */
-    }
-  bad |= solve_square(W, n, n);
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) Xm[q * n + p] = W[(n + p) * n + q]; /* X = (X^T)^T */
-  /* W = [(I + Jj Zi)^T | Ai]; the solve leaves Y^T = (I + Jj Zi)^{-T} Ai */
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = (p == q) ? 1.0 : 0.0; /* (I + Jj Zi)(q, p) */
-      for (int k = 0; k < n; ++k) s = fma(Xj.J.at(k * n + q, j), Xi.Z.at(p * n + k, i), s);
-      W[q * n + p] = s;
-      W[(n + q) * n + p] = Xi.A.at(q * n + p, i); /* Ai(p, q) */
-    }
-  bad |= solve_square(W, n, n);
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) Ym[q * n + p] = W[(n + p) * n + q];
-  /* Z = (X Zi) Aj^T + Zj (reads Aj and Zj before they are overwritten) */
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = 0.0;
-      for (int k = 0; k < n; ++k) s = fma(Xm[k * n + p], Xi.Z.at(q * n + k, i), s);
-      T[q * n + p] = s;
-    }
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = Xj.Z.at(q * n + p, j);
-      for (int k = 0; k < n; ++k) s = fma(T[k * n + p], Xj.A.at(k * n + q, j), s);
-      O.Z.at(q * n + p, o) = s;
-    }
-  /* b = X (bi + Zi ej) + bj */
-  for (int p = 0; p < n; ++p) {
-    double s = Xi.b.at(p, i);
-    for (int k = 0; k < n; ++k) s = fma(Xi.Z.at(k * n + p, i), Xj.e.at(k, j), s);
-    v[p] = s;
-  }
-  for (int p = 0; p < n; ++p) {
-    double s = Xj.b.at(p, j);
-    for (int k = 0; k < n; ++k) s = fma(Xm[k * n + p], v[k], s);
-    O.b.at(p, o) = s;
-  }
-  /* e = Y (ej - Jj bi) + ei */
-  for (int p = 0; p < n; ++p) {
-    double s = Xj.e.at(p, j);
-    for (int k = 0; k < n; ++k) s = fma(-Xj.J.at(k * n + p, j), Xi.b.at(k, i), s);
-    v[p] = s;
-  }
-  for (int p = 0; p < n; ++p) {
-    double s = Xi.e.at(p, i);
-    for (int k = 0; k < n; ++k) s = fma(Ym[k * n + p], v[k], s);
-    O.e.at(p, o) = s;
-  }
-  /* J = Y (Jj Ai) + Ji */
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = 0.0;
-      for (int k = 0; k < n; ++k) s = fma(Xj.J.at(k * n + p, j), Xi.A.at(q * n + k, i), s);
-      T[q * n + p] = s;
-    }
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = Xi.J.at(q * n + p, i);
-      for (int k = 0; k < n; ++k) s = fma(Ym[k * n + p], T[q * n + k], s);
-      O.J.at(q * n + p, o) = s;
-    }
-  /* A = X Ai (last: overwrites Aj) */
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = 0.0;
-      for (int k = 0; k < n; ++k) s = fma(Xm[k * n + p], Xi.A.at(q * n + k, i), s);
-      T[q * n + p] = s;
-    }
-  for (int e = 0; e < n * n; ++e) O.A.at(e, o) = T[e];
-  return bad;
-}
-
-__device__ bool combine_smooth(int n, const SElems& Xi, int64_t i, const SElems& Xj, int64_t j, const SElems& O,
-                               int64_t o, PV ws)
-{
-  /* E = Ej Ei, g = Ej gi + gj, L = Ej Li Ej^T + Lj */
-  PV T = ws, U = ws + n * n;
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = 0.0, u = 0.0;
-      for (int k = 0; k < n; ++k) {
-        s = fma(Xj.E.at(k * n + p, j), Xi.L.at(q * n + k, i), s);
-        u = fma(Xj.E.at(k * n + p, j), Xi.E.at(q * n + k, i), u);
-      }
-      T[q * n + p] = s; /* Ej Li */
-      U[q * n + p] = u; /* Ej Ei */
-    }
-  for (int q = 0; q < n; ++q)
-    for (int p = 0; p < n; ++p) {
-      double s = Xj.L.at(q * n + p, j);
-      for (int k = 0; k < n; ++k) s = fma(T[k * n + p], Xj.E.at(k * n + q, j), s);
-      O.L.at(q * n + p, o) = s;
-    }
-  for (int p = 0; p < n; ++p) {
-    double s = Xj.g.at(p, j);
-    for (int k = 0; k < n; ++k) s = fma(Xj.E.at(k * n + p, j), Xi.g.at(k, i), s);
-    T[p] = s;
-  }
-  for (int p = 0; p < n; ++p) O.g.at(p, o) = T[p];
-  for (int e = 0; e < n * n; ++e) O.E.at(e, o) = U[e];
-  return false;
-}
-
-template <class El>
-__device__ void copy_elem(int n, const El& X, int64_t i, const El& O, int64_t o);
-
-template <>
-__device__ void copy_elem<FElems>(int n, const FElems& X, int64_t i, const FElems& O, int64_t o)
-{
-  for (int e = 0; e < n * n; ++e) {
-    O.A.at(e, o) = X.A.at(e, i);
-    O.Z.at(e, o) = X.Z.at(e, i);
-    O.J.at(e, o) = X.J.at(e, i);
-  }
-  for (int e = 0; e < n; ++e) {
-    O.b.at(e, o) = X.b.at(e, i);
-    O.e.at(e, o) = X.e.at(e, i);
-  }
-}
-
-template <>
-__device__ void copy_elem<SElems>(int n, const SElems& X, int64_t i, const SElems& O, int64_t o)
-{
-  for (int e = 0; e < n * n; ++e) {
-    O.E.at(e, o) = X.E.at(e, i);
-    O.L.at(e, o) = X.L.at(e, i);
-  }
-  for (int e = 0; e < n; ++e) O.g.at(e, o) = X.g.at(e, i);
-}
-
-__device__ __forceinline__ bool combine(int n, const FElems& Xi, int64_t i, const FElems& Xj, int64_t j,
-                                        const FElems& O, int64_t o, PV ws)
-{
-  return combine_filter(n, Xi, i, Xj, j, O, o, ws);
-}
-__device__ __forceinline__ bool combine(int n, const SElems& Xi, int64_t i, const SElems& Xj, int64_t j,
-                                        const SElems& O, int64_t o, PV ws)
-{
-  return combine_smooth(n, Xi, i, Xj, j, O, o, ws);
-}
-
 /* level tables of a scan: per track, the sequence length L and start at each
  * level, and prefix sums of items (ceil(L/2) for tracks with L >= 2 in the
  * up-sweep, ceil(L/2) for tracks with L >= 1 in the down-sweep)             */
@@ -638,42 +480,7 @@ struct ScanLevel {
 };
 
 #include "associative_cta.cuh"
-
-/* up-sweep: level d+1 element p = a_{2p} (x) a_{2p+1}, or a_{2p} alone */
-template <class El>
-__global__ void up_kernel(int n, int T, ScanLevel lv, ScanLevel nx, El cur, El nxt, int* flag)
-{
-  extern __shared__ double smem[];
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= lv.nup) return;
-  PV ws{smem + threadIdx.x, (int)blockDim.x};
-  const int t = find_track(lv.up_items, T, item);
-  const int64_t p = item - lv.up_items[t];
-  const int64_t s0 = lv.start[t] + 2 * p, o = nx.start[t] + p;
-  if (2 * p + 1 < lv.L[t]) {
-    if (combine(n, cur, s0, cur, s0 + 1, nxt, o, ws)) atomicOr(flag, 2);
-  } else {
-    copy_elem(n, cur, s0, nxt, o);
-  }
-}
-
-/* down-sweep: with level d+1 already inclusive prefixes B,
- * A_{2p+1} = B_p, A_{2p} = B_{p-1} (x) a_{2p} (A_0 = a_0), in place          */
-template <class El>
-__global__ void down_kernel(int n, int T, ScanLevel lv, ScanLevel nx, El cur, El nxt, int* flag)
-{
-  extern __shared__ double smem[];
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= lv.ndown) return;
-  PV ws{smem + threadIdx.x, (int)blockDim.x};
-  const int t = find_track(lv.down_items, T, item);
-  const int64_t p = item - lv.down_items[t];
-  const int64_t L = lv.L[t];
-  if (L < 2) return; /* a one-element sequence is its own prefix */
-  const int64_t s0 = lv.start[t] + 2 * p, b0 = nx.start[t] + p;
-  if (2 * p + 1 < L) copy_elem(n, nxt, b0, cur, s0 + 1);
-  if (p > 0 && combine(n, nxt, b0 - 1, cur, s0, cur, s0, ws)) atomicOr(flag, 2);
-}
+#include "associative_small.cuh"
 
 /* filtered estimates: step i >= 1 of each track gets (b, Z) of prefix i-1   */
 __global__ void filtered_out_kernel(Args a, FElems el, const int64_t* seq_start, int64_t nsteps)
@@ -1081,20 +888,17 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
   const size_t sc_obs = 3 * (size_t)mx * mx + (size_t)mx * (mx + n) + 2 * (size_t)n * mx + mx + n + nn;
   const size_t sc_elem = std::max<size_t>(std::max<size_t>((size_t)n * (n + 1) + nn + n, 2 * nn), sc_obs);
   const size_t pt_elem = ((size_t)n + 2 * nn + sc_elem + 8) * 8;
-  const size_t pt_comb = (size_t)(5 * nn + n + 8) * 8;
   const size_t pt_selem = (size_t)(6 * nn + n + 8) * 8;
-  int be, bc, bsm;
-  if (pick_block(pt_elem, 64, &be) || pick_block(pt_comb, 64, &bc) || pick_block(pt_selem, 64, &bsm))
+  int be, bsm;
+  if (pick_block(pt_elem, 64, &be) || pick_block(pt_selem, 64, &bsm))
     return ukg_set_error(KALMAN_GPU_EINVAL, "state dimension %d needs more shared memory per thread than this build "
                          "of the associative kernels uses", n);
   ukg_allow_dynamic_smem((const void*)element_kernel);
-  ukg_allow_dynamic_smem((const void*)up_kernel<FElems>);
-  ukg_allow_dynamic_smem((const void*)down_kernel<FElems>);
-  ukg_allow_dynamic_smem((const void*)up_kernel<SElems>);
-  ukg_allow_dynamic_smem((const void*)down_kernel<SElems>);
   ukg_allow_dynamic_smem((const void*)smooth_element_kernel);
   auto grid = [](int64_t items, int block) { return (unsigned)((items + block - 1) / block); };
   const int ew = 128;
+  const asmall::Scans sc = asmall::scans(n); /* n <= 8 here */
+  const int bc = 32 * asmall::kWarps;
 
   /* filtering elements and the forward scan */
   const int64_t* fstart0 = dtab + fp.off_start[0];
@@ -1103,13 +907,13 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
   for (int l = 0; l + 1 < fp.nlev; ++l)
     if (fp.nup[l] > 0)
       UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (up_kernel<FElems><<<grid(fp.nup[l], bc), bc, bc * pt_comb, st>>>(
-                     n, T, level(fp, l), level(fp, l + 1), felems(l), felems(l + 1), dflag)));
+                 (sc.up_f<<<grid(fp.nup[l], asmall::kWarps), bc, 0, st>>>(T, level(fp, l), level(fp, l + 1), felems(l),
+                                                                          felems(l + 1), dflag)));
   for (int l = fp.nlev - 2; l >= 0; --l)
     if (fp.ndown[l] > 0)
       UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (down_kernel<FElems><<<grid(fp.ndown[l], bc), bc, bc * pt_comb, st>>>(
-                     n, T, level(fp, l), level(fp, l + 1), felems(l), felems(l + 1), dflag)));
+                 (sc.down_f<<<grid(fp.ndown[l], asmall::kWarps), bc, 0, st>>>(T, level(fp, l), level(fp, l + 1),
+                                                                              felems(l), felems(l + 1), dflag)));
   UKG_LAUNCH(UKG_K_AS_ELEMENT, st, (filtered_out_kernel<<<grid(N, ew), ew, 0, st>>>(a, felems(0), fstart0, N)));
   /* smoothing elements and the reverse scan */
   const int64_t* sstart0 = dtab + sp.off_start[0];
@@ -1118,13 +922,13 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
   for (int l = 0; l + 1 < sp.nlev; ++l)
     if (sp.nup[l] > 0)
       UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (up_kernel<SElems><<<grid(sp.nup[l], bc), bc, bc * pt_comb, st>>>(
-                     n, T, level(sp, l), level(sp, l + 1), selems(l), selems(l + 1), dflag)));
+                 (sc.up_s<<<grid(sp.nup[l], sc.smooth_per_block), bc, 0, st>>>(T, level(sp, l), level(sp, l + 1),
+                                                                               selems(l), selems(l + 1))));
   for (int l = sp.nlev - 2; l >= 0; --l)
     if (sp.ndown[l] > 0)
       UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (down_kernel<SElems><<<grid(sp.ndown[l], bc), bc, bc * pt_comb, st>>>(
-                     n, T, level(sp, l), level(sp, l + 1), selems(l), selems(l + 1), dflag)));
+                 (sc.down_s<<<grid(sp.ndown[l], sc.smooth_per_block), bc, 0, st>>>(T, level(sp, l), level(sp, l + 1),
+                                                                                   selems(l), selems(l + 1))));
   UKG_LAUNCH(UKG_K_AS_SMOOTH, st, (smoothed_out_kernel<<<grid(N, ew), ew, 0, st>>>(a, selems(0), sstart0, N)));
 
   return finish(st, dflag);
