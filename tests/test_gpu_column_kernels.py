@@ -1,0 +1,47 @@
+"""The thread-per-column kernels (9 to 64 states, 96 in the precision form) at
+the edges of their register sizes (12, 16, 24, 32, 48, 64, 96 rows) against
+the oracle: every covariance type, unobserved steps (the trapezoids then run
+out of rows), odd and even lengths.  Bars as elsewhere: 1e-11 in FP64, 1e-9
+in the precision form and in double-float."""
+import pytest
+
+import oracle
+from ultimate_kalman_gb300 import native, problem as pb
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    native.load()
+
+
+@pytest.mark.parametrize("n,m,cov", [(9, 4, "C"), (12, 12, "W"), (13, 1, "w"), (16, 7, "F"), (17, 17, "C"),
+                                     (24, 11, "W"), (25, 12, "F"), (31, 30, "C"), (32, 9, "w"), (33, 16, "C"),
+                                     (48, 47, "F"), (49, 20, "W"), (63, 5, "C"), (64, 32, "C"), (65, 31, "C"),
+                                     (96, 40, "C"), (97, 33, "F")])
+def test_register_sizes(n, m, cov):
+    P = pb.random_dynamics([1, 2, 11, 14], n, m, seed=n + m, K_type=cov, C_type=cov, missing=0.3, per_step=True)
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, S = native.smooth(P, "oddeven")
+    assert oracle.rel_err_states(X, Xo) < 1e-11 and oracle.rel_err_covs(S, So) < 1e-11
+    X, _ = native.smooth(P, "oddeven", covariance=False)
+    assert oracle.rel_err_states(X, Xo) < 1e-11
+    X, S = native.smooth(P, "oddeven", fp32_refine=True)
+    assert oracle.rel_err_states(X, Xo) < 1e-9 and oracle.rel_err_covs(S, So) < 1e-9
+    X, _ = native.smooth(P, "oddeven", covariance=False, fp32_refine=True, sweeps=3)
+    assert oracle.rel_err_states(X, Xo) < 1e-9
+
+
+@pytest.mark.parametrize("n", [12, 40])
+def test_unobservable_is_reported(n):
+    P = pb.random_dynamics([9], n, 2, seed=n, fold=False)
+    P.obs_rows[1:] = 0
+    for refine in (False, True):
+        with pytest.raises(native.KalmanError) as e:
+            native.smooth(P, "oddeven", fp32_refine=refine)
+        assert e.value.status == native.KALMAN_GPU_ESINGULAR

@@ -41,6 +41,8 @@ __device__ __forceinline__ bool series_range(double x)
 __device__ __forceinline__ double recip(double d) { return series_range(d) ? rcp_series(d) : 1.0 / d; }
 __device__ __forceinline__ ukg_df::dd recip(ukg_df::dd d) { return ukg_df::dd(1) / d; }
 
+__device__ __forceinline__ float recip(float d) { return 1.0f / d; }
+
 /* The reflector that maps (alpha, x) to (beta, 0), tail = x^T x != 0, as
  * H = I - inv u u^T with u = (amb, x): a column (a_k, a) takes
  * d = inv (x^T a + amb a_k), a_k -= d amb, a -= d x.  x stays unscaled.      */
@@ -73,6 +75,16 @@ __device__ __forceinline__ Refl<ukg_df::dd> reflector(ukg_df::dd alpha, ukg_df::
   r.beta = -copysign(nb, alpha);
   r.amb = alpha - r.beta;
   r.inv = dd(1) / (nb * fabs(r.amb));
+  return r;
+}
+
+__device__ __forceinline__ Refl<float> reflector(float alpha, float tail)
+{
+  Refl<float> r;
+  const float nb = sqrtf(fmaf(alpha, alpha, tail));
+  r.beta = -copysignf(nb, alpha);
+  r.amb = alpha - r.beta;
+  r.inv = 1.0f / (nb * fabsf(r.amb));
   return r;
 }
 

@@ -2194,6 +2194,7 @@ __global__ void add_kernel(double* x, const double* d, int64_t count)
 
 #include "oddeven_cta.cuh"
 #include "oddeven_small.cuh"
+#include "oddeven_cols.cuh"
 
 /* ---------------------------------------------------------------------------
  * host side: plan, workspace, launches
@@ -3036,6 +3037,15 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
   auto grid = [&](int64_t items) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, ncta)); };
   constexpr bool kDD = std::is_same<T, ukg_df::dd>::value; /* double-float: own kernel classes */
   const int kWeigh = kDD ? UKG_K_DF_WEIGH : UKG_K_WEIGH, kTail = kDD ? UKG_K_DF_TAIL : UKG_K_TAIL;
+  /* a thread per column where the columns' registers hold the shape */
+  const cols::Kernels<T> CK = cols::kernels<T>(n, mx);
+  const size_t ck_pair = cols::pair_smem<T>(n), ck_tail = cols::tail_smem<T>(n), ck_solve = cols::solve_smem<T>(n);
+  if (CK.pair) {
+    ukg_allow_dynamic_smem((const void*)CK.weigh);
+    ukg_allow_dynamic_smem((const void*)CK.pair);
+    ukg_allow_dynamic_smem((const void*)CK.tail);
+    if (CK.solve) ukg_allow_dynamic_smem((const void*)CK.solve);
+  }
   const ctak::RawA raw{p->H, p->F, p->c, p->K, p->G, p->o, p->C, p->K_type, p->C_type, p->obs_rows, p->mmax};
   {
     ctak::CArgs<T> a;
@@ -3045,7 +3055,9 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
        CTAs fit one slot, twice as many run (more warps on its latency) */
     const int64_t rmax = std::max(n, p->mmax);
     const int64_t wneed = rmax * rmax + rmax * (2 * n + 1) + rmax * cta::NT;
-    if (2 * wneed <= a.scratch_per_cta) {
+    if (CK.weigh) {
+      UKG_LAUNCH(kWeigh, st, (CK.weigh<<<(unsigned)p->nsteps, CK.threads3, CK.weigh_smem, st>>>(a, raw)));
+    } else if (2 * wneed <= a.scratch_per_cta) {
       a.scratch_per_cta /= 2;
       const unsigned g2 = (unsigned)std::max<int64_t>(1, std::min<int64_t>(p->nsteps, 2 * (int64_t)ncta));
       UKG_LAUNCH(kWeigh, st, (ctak::weigh_cta<T><<<g2, cta::NT, 0, st>>>(a, raw, p->nsteps)));
@@ -3060,6 +3072,12 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     common(a, l);
     a.ce = eq_level(l);
     if (l + 1 < nlev) a.ne = eq_level(l + 1);
+    if (CK.pair) {
+      if (lp[l].npairs > 0)
+        UKG_LAUNCH(kPair, st, (CK.pair<<<(unsigned)lp[l].npairs, CK.threads, ck_pair, st>>>(a)));
+      if (lp[l].ntail > 0) UKG_LAUNCH(kTail, st, (CK.tail<<<(unsigned)lp[l].ntail, CK.threads, ck_tail, st>>>(a)));
+      continue;
+    }
     if (lp[l].npairs > 0) {
       if (n >= cta::kBlockedMinN)
         UKG_LAUNCH(kPair, st, (ctak::pair_cta<T, true><<<grid(lp[l].npairs), cta::NT, 0, st>>>(a)));
@@ -3076,7 +3094,12 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
   for (int l = nlev - 2; l >= 0; --l) {
     ctak::CArgs<T> a;
     common(a, l);
-    if (lp[l].nsolve > 0)
+    if (lp[l].nsolve == 0) continue;
+    if (CK.solve && want_cov)
+      UKG_LAUNCH(kSolve, st, (CK.solve<<<(unsigned)lp[l].nsolve, CK.threads3, ck_solve, st>>>(a)));
+    else if (CK.state && !want_cov)
+      UKG_LAUNCH(kSolve, st, (CK.state<<<(unsigned)((lp[l].nsolve + 3) / 4), 128, 0, st>>>(a)));
+    else
       UKG_LAUNCH(kSolve, st, (ctak::solve_cta<T><<<grid(lp[l].nsolve), cta::NT, 0, st>>>(a, want_cov ? 1 : 0)));
   }
   /* ---- refinement sweeps (FP32 factors): FP64 residual, transpose solves, solves ---- */
@@ -3146,7 +3169,9 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
         a.state = dx;
         a.cov = nullptr;
         a.yrhs = Soa<float>{(float*)(B + P.o_y[l]), std::max<int64_t>(lp[l].E, 1)};
-        if (lp[l].nsolve > 0)
+        if (lp[l].nsolve > 0 && CK.state)
+          UKG_LAUNCH(UKG_K_RSOLVE, st, (CK.state<<<(unsigned)((lp[l].nsolve + 3) / 4), 128, 0, st>>>(a)));
+        else if (lp[l].nsolve > 0)
           UKG_LAUNCH(UKG_K_RSOLVE, st, (ctak::solve_cta<float><<<grid(lp[l].nsolve), cta::NT, 0, st>>>(a, 0)));
       }
       const int64_t cnt = p->nsteps * n;
