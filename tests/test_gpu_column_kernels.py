@@ -45,3 +45,14 @@ def test_unobservable_is_reported(n):
         with pytest.raises(native.KalmanError) as e:
             native.smooth(P, "oddeven", fp32_refine=refine)
         assert e.value.status == native.KALMAN_GPU_ESINGULAR
+
+
+@pytest.mark.parametrize("n,m,cov", [(9, 3, "W"), (12, 6, "C"), (15, 15, "w"), (16, 8, "F"), (24, 10, "C"),
+                                     (31, 8, "U"), (33, 40, "C"), (48, 24, "W"), (50, 20, "C"), (64, 30, "F"),
+                                     (65, 10, "C")])
+def test_associative_register_sizes(n, m, cov):
+    P = pb.random_dynamics([1, 2, 9, 14], n, m, seed=2 * n + m, K_type=cov, C_type=cov, missing=0.3, per_step=True)
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, S = native.smooth(P, "associative")
+    assert oracle.rel_err_states(X, Xo) < 1e-11 and oracle.rel_err_covs(S, So) < 1e-11

@@ -38,6 +38,7 @@
 
 #include "profiling.h"
 #include "cta_linalg.cuh"
+#include "columns.cuh"
 #include "lanes.cuh"
 #include "ukgpu_internal.h"
 
@@ -480,6 +481,7 @@ struct ScanLevel {
 };
 
 #include "associative_cta.cuh"
+#include "associative_cols.cuh"
 #include "associative_small.cuh"
 
 /* filtered estimates: step i >= 1 of each track gets (b, Z) of prefix i-1   */
@@ -754,7 +756,7 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
   /* larger shapes run the CTA kernels, which need per-CTA scratch */
   const bool cta_path = n >= 9 || mx > 8;
   int ncta = 0;
-  int64_t per_cta = 0;
+  int64_t per_cta = 0, xy_items = 1;
   size_t o_scratch = 0;
   if (cta_path) {
     if (mx > 128)
@@ -768,7 +770,10 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
     const int64_t elem = n + 2 * nn + mxr * 2 * n + mxr * (mxr + n + 1) + 2 * mxr * mxr + 2 * n * mxr + 2 * mxr +
                          mxr * acta::NT;
     per_cta = std::max(std::max(elem, 7 * nn + 4 * n), 7 * nn + n) + 32;
+    /* the same region holds the solved systems of a scan level, 2 n^2 entries
+       an item, of as many items as fit (at least one per SM)               */
     o_scratch = take((size_t)ncta * per_cta * sizeof(double));
+    xy_items = (int64_t)ncta * per_cta / (2 * nn);
   }
   void* base = nullptr;
   if (int e = ensure(bytes, &base, st)) return e;
@@ -845,28 +850,63 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
     acta::RawS raw{p->F, p->c, p->K, p->G, p->o, p->C, p->K_type, p->C_type, p->obs_rows, p->mmax};
     auto g = [&](int64_t items) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, ncta)); };
     const int64_t* fstart0 = dtab + fp.off_start[0];
+    const acols::Kernels CK = acols::kernels(n); /* a thread per column where its rows fit the registers */
+    if (CK.smooth_element)
+      for (const void* f : {(const void*)CK.solve[0], (const void*)CK.solve[1], (const void*)CK.products[0],
+                            (const void*)CK.products[1], (const void*)CK.smooth[0], (const void*)CK.smooth[1],
+                            (const void*)CK.smooth_element})
+        ukg_allow_dynamic_smem(f);
+    /* one level of the filtering scan (dir 0: up, 1: down), xy_items at a time */
+    auto filter_level = [&](int dir, int l, int64_t items) {
+      for (int64_t i0 = 0; i0 < items; i0 += xy_items) {
+        const unsigned blocks = 2 * (unsigned)std::min<int64_t>(items - i0, xy_items);
+        UKG_LAUNCH(UKG_K_AS_SCAN, st,
+                   (CK.solve[dir]<<<blocks, CK.threads2, acols::solve_smem(n), st>>>(
+                       n, T, level(fp, l), level(fp, l + 1), fel(l), fel(l + 1), scratch, i0, dflag)));
+        UKG_LAUNCH(UKG_K_AS_SCAN, st,
+                   (CK.products[dir]<<<blocks, CK.threads4, acols::products_smem(n), st>>>(
+                       n, T, level(fp, l), level(fp, l + 1), fel(l), fel(l + 1), scratch, i0)));
+      }
+    };
+    auto smooth_level = [&](int dir, int l, int64_t items) {
+      UKG_LAUNCH(UKG_K_AS_SCAN, st,
+                 (CK.smooth[dir]<<<(unsigned)items, CK.threads4, acols::smooth_smem(n), st>>>(
+                     n, T, level(sp, l), level(sp, l + 1), sel(l), sel(l + 1))));
+    };
     UKG_LAUNCH(UKG_K_AS_ELEMENT, st, (acta::element_cta<<<g(N), acta::NT, 0, st>>>(a, raw, fel(0), fstart0, N)));
     for (int l = 0; l + 1 < fp.nlev; ++l)
-      if (fp.nup[l] > 0)
+      if (fp.nup[l] > 0 && CK.smooth_element)
+        filter_level(0, l, fp.nup[l]);
+      else if (fp.nup[l] > 0)
         UKG_LAUNCH(UKG_K_AS_SCAN, st,
                    (acta::up_cta<acta::FEl><<<g(fp.nup[l]), acta::NT, 0, st>>>(
                        n, T, level(fp, l), level(fp, l + 1), fel(l), fel(l + 1), dflag, scratch, per_cta)));
     for (int l = fp.nlev - 2; l >= 0; --l)
-      if (fp.ndown[l] > 0)
+      if (fp.ndown[l] > 0 && CK.smooth_element)
+        filter_level(1, l, fp.ndown[l]);
+      else if (fp.ndown[l] > 0)
         UKG_LAUNCH(UKG_K_AS_SCAN, st,
                    (acta::down_cta<acta::FEl><<<g(fp.ndown[l]), acta::NT, 0, st>>>(
                        n, T, level(fp, l), level(fp, l + 1), fel(l), fel(l + 1), dflag, scratch, per_cta)));
     UKG_LAUNCH(UKG_K_AS_ELEMENT, st, (acta::filtered_out_cta<<<g(N), 128, 0, st>>>(a, fel(0), fstart0, N)));
     const int64_t* sstart0 = dtab + sp.off_start[0];
-    UKG_LAUNCH(UKG_K_AS_SMOOTH, st,
+    if (CK.smooth_element)
+      UKG_LAUNCH(UKG_K_AS_SMOOTH, st,
+                 (CK.smooth_element<<<(unsigned)N, CK.threads2, acols::element_smem(n), st>>>(a, raw, sel(0), sstart0)));
+    else
+      UKG_LAUNCH(UKG_K_AS_SMOOTH, st,
                (acta::smooth_element_cta<<<g(N), acta::NT, 0, st>>>(a, raw, sel(0), sstart0, N)));
     for (int l = 0; l + 1 < sp.nlev; ++l)
-      if (sp.nup[l] > 0)
+      if (sp.nup[l] > 0 && CK.smooth_element)
+        smooth_level(0, l, sp.nup[l]);
+      else if (sp.nup[l] > 0)
         UKG_LAUNCH(UKG_K_AS_SCAN, st,
                    (acta::up_cta<acta::SEl><<<g(sp.nup[l]), acta::NT, 0, st>>>(
                        n, T, level(sp, l), level(sp, l + 1), sel(l), sel(l + 1), dflag, scratch, per_cta)));
     for (int l = sp.nlev - 2; l >= 0; --l)
-      if (sp.ndown[l] > 0)
+      if (sp.ndown[l] > 0 && CK.smooth_element)
+        smooth_level(1, l, sp.ndown[l]);
+      else if (sp.ndown[l] > 0)
         UKG_LAUNCH(UKG_K_AS_SCAN, st,
                    (acta::down_cta<acta::SEl><<<g(sp.ndown[l]), acta::NT, 0, st>>>(
                        n, T, level(sp, l), level(sp, l + 1), sel(l), sel(l + 1), dflag, scratch, per_cta)));

@@ -1,0 +1,148 @@
+/*
+ * columns.cuh -- dense routines with one matrix column per thread, its rows in
+ * registers (NP of them, n <= NP in use), shared by the odd-even and the
+ * associative smoother for 9 states and more.
+ */
+#pragma once
+#include <cstdint>
+
+#include "lanes.cuh"
+
+namespace columns {
+
+/* b <- n (or `rows`) consecutive entries, zero past them */
+template <typename T, int NP>
+__device__ __forceinline__ void load_rows(const T* p, int rows, bool on, T (&b)[NP])
+{
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    b[i] = T(0);
+    if (on && i < rows) b[i] = p[i];
+  }
+}
+
+/* R x = b by columns: v_j = b_j / R_jj from the last row up, the rows moving
+ * towards the end as they are done.  b is aligned to the end (row n - 1 at
+ * NP - 1); R column-major in shared memory (ld n), dv the reciprocals of its
+ * diagonal; put(j, v_j).                                                     */
+template <typename T, int NP, class PUT>
+__device__ __forceinline__ void back_subst(const T* R, const T* dv, int n, T (&b)[NP], PUT put)
+{
+#pragma unroll 1
+  for (int j = n - 1; j >= 0; --j) {
+    const T v = b[NP - 1] * dv[j];
+    put(j, v);
+    const T* Rj = R + j * n + j - NP; /* row of b[i - 1] is i - NP + j */
+#pragma unroll
+    for (int i0 = NP - 4; i0 >= 0; i0 -= 4)
+      if (i0 + 3 - NP + j >= 0) { /* the same in every thread */
+#pragma unroll
+        for (int u = 3; u >= 0; --u) {
+          const int i = i0 + u;
+          if (i > 0) b[i] = i - NP + j >= 0 ? fma(-v, Rj[i], b[i - 1]) : b[i - 1];
+        }
+      }
+  }
+}
+template <typename T, int NP>
+__device__ __forceinline__ void load_end(const T* p, int n, bool on, T (&b)[NP])
+{
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    b[i] = T(0);
+    if (on && i - NP + n >= 0) b[i] = p[i - NP + n];
+  }
+}
+
+/* b += M s for the column-major M (n x n, ld n) and a vector s given entry by
+ * entry, four at a time, the next four on their way; b from row 0 on          */
+template <int NP, class AT>
+__device__ __forceinline__ void matvec(const double* M, int n, double (&b)[NP], AT at)
+{
+  double s[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) s[u] = u < n ? at(u) : 0.0;
+#pragma unroll 1
+  for (int k = 0; k < n; k += 4) {
+    double next[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) next[u] = k + 4 + u < n ? at(k + 4 + u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u < n) {
+        const double* p = M + (int64_t)(k + u) * n;
+#pragma unroll
+        for (int i = 0; i < NP; i += 4)
+          if (i < n) /* the same in every thread */
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+              if (i + v < n) b[i + v] = fma(p[i + v], s[u], b[i + v]);
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = next[u];
+  }
+}
+
+/* Householder QR of square panels (n x n pivots on the columns 0..n-1 of up to
+ * two panels), FP64.  Row k is the first of b at step k; done, it goes to the
+ * end, so after n steps a column's entries are in order, aligned to the end:
+ * R (whose entries below the diagonal mean nothing) and Q^T of the others.   */
+template <int NP>
+struct SquareShared {
+  double x[2][2][NP], amb[2][2], inv[2][2];
+};
+template <int NP>
+__device__ __forceinline__ void qr_square(SquareShared<NP>& sm, int panel, bool act, int c, int n, double (&b)[NP])
+{
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    const int rows = n - 1 - k, buf = k & 1; /* rows below row k */
+    double t = b[0];
+#pragma unroll
+    for (int i = 0; i + 1 < NP; ++i) b[i] = b[i + 1];
+    double* x = sm.x[buf][panel];
+    const bool pivot = act && c == k;
+    if (pivot)
+#pragma unroll
+      for (int i = 0; i < NP; ++i) x[i] = i < rows ? b[i] : 0.0;
+    __syncthreads();
+    const bool on = act && c >= k; /* whole warps of finished pivots wait */
+    double dot = 0.0;
+    if (on) {
+      double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+      for (int i = 0; i < NP; i += 4)
+        if (i < rows) {
+          d0 = fma(x[i], b[i], d0);
+          d1 = fma(x[i + 1], b[i + 1], d1);
+          d0 = fma(x[i + 2], b[i + 2], d0);
+          d1 = fma(x[i + 3], b[i + 3], d1);
+        }
+      dot = d0 + d1;
+    }
+    if (pivot) {
+      lanes::Refl<double> r;
+      r.beta = t;
+      r.amb = r.inv = 0.0;
+      if (dot != 0.0) r = lanes::reflector(t, dot);
+      sm.amb[buf][panel] = r.amb;
+      sm.inv[buf][panel] = r.inv;
+      t = r.beta;
+    }
+    __syncthreads();
+    const double amb = sm.amb[buf][panel], inv = sm.inv[buf][panel];
+    if (on && !pivot && amb != 0.0) {
+      const double d = fma(amb, t, dot) * inv;
+      t = fma(-d, amb, t);
+#pragma unroll
+      for (int i = 0; i < NP; i += 4)
+        if (i < rows) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) b[i + u] = fma(-d, x[i + u], b[i + u]);
+        }
+    }
+    b[NP - 1] = t;
+  }
+}
+
+}  // namespace columns

@@ -60,6 +60,7 @@
 
 #include "df64.cuh"
 #include "cta_linalg.cuh"
+#include "columns.cuh"
 #include "lanes.cuh"
 
 #include <algorithm>

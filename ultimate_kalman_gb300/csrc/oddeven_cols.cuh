@@ -32,6 +32,9 @@
 namespace cols {
 using ctak::CArgs;
 using ctak::RawA;
+using columns::back_subst;
+using columns::load_end;
+using columns::load_rows;
 using lanes::recip;
 using lanes::Refl;
 using lanes::reflector;
@@ -143,17 +146,6 @@ __device__ __forceinline__ void reduce(QrShared<T, NP>& sm, int panel, bool act,
     next = act && k + 1 < m ? load(k + 1) : T(0);
     tk = step<T, NP>(sm, k, panel, on, c == k, n, tk, b);
     if (on) store(k, tk);
-  }
-}
-
-/* b <- n (or `rows`) consecutive entries, zero past them */
-template <typename T, int NP>
-__device__ __forceinline__ void load_rows(const T* p, int rows, bool on, T (&b)[NP])
-{
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    b[i] = T(0);
-    if (on && i < rows) b[i] = p[i];
   }
 }
 
@@ -454,39 +446,6 @@ __global__ void __launch_bounds__(threads<NP>(), blocks<T, NP>()) pair_cols(CArg
 }
 template <typename T>
 size_t pair_smem(int n) { return (size_t)(n * (2 * n + 1) + (n + 1) * n) * sizeof(T); }
-
-/* R x = b by columns: v_j = b_j / R_jj from the last row up, the rows moving
- * towards the end as they are done.  b is aligned to the end (row n - 1 at
- * NP - 1); R column-major in shared memory (ld n), dv the reciprocals of its
- * diagonal; put(j, v_j).                                                     */
-template <typename T, int NP, class PUT>
-__device__ __forceinline__ void back_subst(const T* R, const T* dv, int n, T (&b)[NP], PUT put)
-{
-#pragma unroll 1
-  for (int j = n - 1; j >= 0; --j) {
-    const T v = b[NP - 1] * dv[j];
-    put(j, v);
-    const T* Rj = R + j * n + j - NP; /* row of b[i - 1] is i - NP + j */
-#pragma unroll
-    for (int i0 = NP - 4; i0 >= 0; i0 -= 4)
-      if (i0 + 3 - NP + j >= 0) { /* the same in every thread */
-#pragma unroll
-        for (int u = 3; u >= 0; --u) {
-          const int i = i0 + u;
-          if (i > 0) b[i] = i - NP + j >= 0 ? fma(-v, Rj[i], b[i - 1]) : b[i - 1];
-        }
-      }
-  }
-}
-template <typename T, int NP>
-__device__ __forceinline__ void load_end(const T* p, int n, bool on, T (&b)[NP])
-{
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    b[i] = T(0);
-    if (on && i - NP + n >= 0) b[i] = p[i - NP + n];
-  }
-}
 
 /* ---------------------------------------------------------------------------
  * odd-length tracks: the single last step and its fix-up, or the base case
