@@ -104,6 +104,7 @@ struct Dot<ukg_df::dd> {
   __device__ __forceinline__ ukg_df::dd value() const { return ukg_df::finish(s); }
 };
 
+__device__ __forceinline__ float shfl(unsigned m, float v, int src, int w) { return __shfl_sync(m, v, src, w); }
 __device__ __forceinline__ double shfl(unsigned m, double v, int src, int w) { return __shfl_sync(m, v, src, w); }
 __device__ __forceinline__ ukg_df::dd shfl(unsigned m, ukg_df::dd v, int src, int w)
 {

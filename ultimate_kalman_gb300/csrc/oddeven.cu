@@ -96,17 +96,6 @@ struct PVc {
   __device__ __forceinline__ PVc operator+(int off) const { return PVc{p + off * BS}; }
 };
 
-template <typename T, int BS>
-struct ViewOf {
-  using type = PVc<T, BS>;
-  static __device__ __forceinline__ type make(T* smem) { return type{smem + threadIdx.x}; }
-};
-template <typename T>
-struct ViewOf<T, 0> {
-  using type = PV<T>;
-  static __device__ __forceinline__ type make(T* smem) { return type{smem + threadIdx.x, (int)blockDim.x}; }
-};
-
 /* Householder triangularization of the rows x cols block W (leading dimension
  * ld) using the first npiv columns as pivots; reflector scalars go to tau
  * (tau[k] = 0 for an identity reflector).  One division per reflector: with
@@ -225,6 +214,7 @@ struct Args {
   int* flag;
   Soa<T> baseR;    /* base-case R per track (refinement), p may be null      */
   Soa<T> yrhs;     /* refinement: right-hand side of the even steps          */
+  double* xadd;    /* refinement: the states that the correction is added to, or null */
 };
 
 /* last t with base[t] <= i (base has T+1 nondecreasing entries, i < base[T]) */
@@ -858,19 +848,16 @@ __global__ void __launch_bounds__(BS, 512 / BS) weigh_df_kernel(Args<float, floa
 /* ---------------------------------------------------------------------------
  * forward elimination of one pair of a level
  * ------------------------------------------------------------------------ */
-/* NT, MT: compile-time n and mx (0: taken from the arguments); BS: the
- * compile-time block size (0: runtime)                                      */
-template <typename T, typename TI, int NT = 0, int MT = 0, int BS = 0>
-__global__ void __launch_bounds__(BS ? BS : 1024) pair_kernel(Args<T, TI> a, int rmax_rt)
+template <typename T, typename TI>
+__global__ void pair_kernel(Args<T, TI> a, int rmax)
 {
   extern __shared__ unsigned char smem_raw[];
   T* smem = reinterpret_cast<T*>(smem_raw);
   const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= a.ct.npairs) return;
-  const int n = NT ? NT : a.n, mx = MT ? MT : a.mx, rmax = MT ? 2 * MT : rmax_rt;
-  using View = typename ViewOf<T, BS>::type;
-  View ws = ViewOf<T, BS>::make(smem);
-  View W = ws, tau = ws + rmax * (n + 1), col = tau + n;
+  const int n = a.n, mx = a.mx;
+  PV<T> ws{smem + threadIdx.x, (int)blockDim.x};
+  PV<T> W = ws, tau = ws + rmax * (n + 1), col = tau + n;
 
   const Eq<TI>& C = a.ce;
   const Eq<T>& N = a.ne;
@@ -958,326 +945,6 @@ __global__ void __launch_bounds__(BS ? BS : 1024) pair_kernel(Args<T, TI> a, int
       for (int i = 0; i < n; ++i) N.H.at(q * n + i, sn) = col[n + i];
     }
   }
-}
-
-/* ---------------------------------------------------------------------------
- * Householder QR and reflector application on register arrays, for the FP32
- * pair kernel below: the row counts of stages A (m_j + n) and C (m_j +
- * m_{j+1}) are dispatched at run time to instantiations in which every loop
- * bound is a compile-time constant, so the pivot block P[col][row], the
- * reflector scalars and the streamed column are register arrays.  Same
- * arithmetic as pair_kernel.
- * ------------------------------------------------------------------------ */
-template <int R, int C>
-__device__ __forceinline__ void hh_reg(float (&P)[C][R], float (&tau)[C])
-{
-#pragma unroll
-  for (int k = 0; k < C; ++k) {
-    tau[k] = 0.0f;
-    if (k >= R) continue;
-    const float alpha = P[k][k];
-    float tail = 0.0f;
-#pragma unroll
-    for (int i = k + 1; i < R; ++i) tail = fmaf(P[k][i], P[k][i], tail);
-    if (tail != 0.0f) {
-      const float beta = -copysignf(sqrtf(fmaf(alpha, alpha, tail)), alpha);
-      const float amb = alpha - beta;
-      const float inv = 1.0f / (beta * amb);
-      const float t = -(amb * amb) * inv;
-      const float scale = beta * inv;
-#pragma unroll
-      for (int i = k + 1; i < R; ++i) P[k][i] *= scale;
-      P[k][k] = beta;
-#pragma unroll
-      for (int j = k + 1; j < C; ++j) {
-        float d = P[j][k];
-#pragma unroll
-        for (int i = k + 1; i < R; ++i) d = fmaf(P[k][i], P[j][i], d);
-        d *= t;
-        P[j][k] -= d;
-#pragma unroll
-        for (int i = k + 1; i < R; ++i) P[j][i] = fmaf(-d, P[k][i], P[j][i]);
-      }
-      tau[k] = t;
-    }
-  }
-}
-
-template <int R, int C>
-__device__ __forceinline__ void apply_reg(const float (&P)[C][R], const float (&tau)[C], float (&col)[R])
-{
-#pragma unroll
-  for (int k = 0; k < C; ++k) {
-    if (k >= R) continue;
-    const float t = tau[k];
-    float d = col[k];
-#pragma unroll
-    for (int i = k + 1; i < R; ++i) d = fmaf(P[k][i], col[i], d);
-    d *= t;
-    col[k] -= d;
-#pragma unroll
-    for (int i = k + 1; i < R; ++i) col[i] = fmaf(-d, P[k][i], col[i]);
-  }
-}
-
-/* ---------------------------------------------------------------------------
- * FP32 pair elimination with the pair's inputs staged asynchronously.
- * Each thread copies its pair's level equations into its own slice of shared
- * memory with 4-byte cp.async copies in four commit groups (stage A's pivot,
- * the H_{j+1} columns, stage C's rows, stage B's blocks), so every input of
- * the pair is in flight at once and stage A starts when its group lands.  The
- * intermediates (R~, rhs~, Y~, H~, o~) stay in the slice, over inputs already
- * consumed; records and the next level are written once.  Element e of
- * thread t's slice is at smem[e * BP + t] (no bank conflicts).
- * ------------------------------------------------------------------------ */
-__device__ __forceinline__ void cp_async4(float* dst, const float* src)
-{
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int G>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(G) : "memory"); }
-
-template <int N, int BP>
-struct PairSlice {
-  static constexpr int NN = N * N, GW = N * N;   /* MX == N */
-  static constexpr int Gj = 0, oj = GW, Hj = GW + N, Fj = Hj + NN, cj = Fj + NN;
-  static constexpr int G1 = cj + N, o1 = G1 + GW, H1 = o1 + N, F1 = H1 + NN, c1 = F1 + NN;
-  static constexpr int width = c1 + N;
-  /* intermediates: R~ over G_j, rhs~ over o_j, Y~ over F_{j+1}, H~ over the
-   * consumed H_{j+1} columns, o~ over c_{j+1} */
-  static constexpr int Rt = Gj, rt = oj, Yt = F1, Ht = H1, ot = c1;
-  float* t0;
-  __device__ __forceinline__ float& operator[](int e) const { return t0[e * BP]; }
-};
-
-/* stage A with RA = m_j + N rows: pivot [G_j; F_{j+1}], rhs [o_j; c_{j+1}] */
-template <int N, int BP, int RA>
-__device__ __forceinline__ void ss_stage_a(const PairSlice<N, BP>& S)
-{
-  using L = PairSlice<N, BP>;
-  constexpr int MJ = RA - N;
-  float P[N][RA], v[RA], tau[N];
-  cp_async_wait<3>();
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-#pragma unroll
-    for (int i = 0; i < MJ; ++i) P[q][i] = S[L::Gj + q * N + i];
-#pragma unroll
-    for (int i = 0; i < N; ++i) P[q][MJ + i] = S[L::F1 + q * N + i];
-  }
-#pragma unroll
-  for (int i = 0; i < MJ; ++i) v[i] = S[L::oj + i];
-#pragma unroll
-  for (int i = 0; i < N; ++i) v[MJ + i] = S[L::c1 + i];
-  hh_reg<RA, N>(P, tau);
-  apply_reg<RA, N>(P, tau, v);
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < N; ++i) S[L::Rt + q * N + i] = (i <= q) ? P[q][i] : 0.0f;
-#pragma unroll
-  for (int i = 0; i < N; ++i) S[L::rt + i] = v[i];
-#pragma unroll
-  for (int i = 0; i < MJ; ++i) S[L::ot + i] = v[N + i];
-  cp_async_wait<2>();
-#pragma unroll 1
-  for (int q = 0; q < N; ++q) { /* not unrolled: keeps the kernel's code small */
-    float col[RA];
-#pragma unroll
-    for (int i = 0; i < MJ; ++i) col[i] = 0.0f;
-#pragma unroll
-    for (int i = 0; i < N; ++i) col[MJ + i] = S[L::H1 + q * N + i];
-    apply_reg<RA, N>(P, tau, col);
-#pragma unroll
-    for (int i = 0; i < N; ++i) S[L::Yt + q * N + i] = col[i];
-#pragma unroll
-    for (int i = 0; i < MJ; ++i) S[L::Ht + q * N + i] = col[N + i];
-  }
-}
-
-/* stage C with RC = m_j + m_{j+1} rows: pivot [H~_{j+1}; G_{j+1}] */
-template <int N, int BP, int RC>
-__device__ __forceinline__ void ss_stage_c(const PairSlice<N, BP>& S, const Eq<float>& Nx, int64_t sn, int mj)
-{
-  using L = PairSlice<N, BP>;
-  float P[N][RC], v[RC], tau[N];
-  cp_async_wait<1>();
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < RC; ++i) P[q][i] = i < mj ? S[L::Ht + q * N + i] : S[L::G1 + q * N + (i - mj)];
-#pragma unroll
-  for (int i = 0; i < RC; ++i) v[i] = i < mj ? S[L::ot + i] : S[L::o1 + (i - mj)];
-  hh_reg<RC, N>(P, tau);
-  apply_reg<RC, N>(P, tau, v);
-  constexpr int G = RC < N ? RC : N;
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < G; ++i) Nx.G.at(q * N + i, sn) = (i <= q) ? P[q][i] : 0.0f;
-#pragma unroll
-  for (int i = 0; i < G; ++i) Nx.o.at(i, sn) = v[i];
-  Nx.m[sn] = G;
-}
-
-/* stage B: pivot [H_j; R~_j] (2N rows) */
-template <int N, int BP>
-__device__ __forceinline__ void ss_stage_b(const PairSlice<N, BP>& S, const Eq<float>& Nx, const Rec<float>& Rr,
-                                           int64_t sn, int64_t se)
-{
-  using L = PairSlice<N, BP>;
-  constexpr int R2 = 2 * N;
-  float P[N][R2], v[R2], tau[N];
-  cp_async_wait<0>();
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      P[q][i] = S[L::Hj + q * N + i];
-      P[q][N + i] = S[L::Rt + q * N + i];
-    }
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    v[i] = S[L::cj + i];
-    v[N + i] = S[L::rt + i];
-  }
-  hh_reg<R2, N>(P, tau);
-  apply_reg<R2, N>(P, tau, v);
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < N; ++i) Rr.R.at(q * N + i, se) = (i <= q) ? P[q][i] : 0.0f;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    Rr.rhs.at(i, se) = v[i];
-    Nx.c.at(i, sn) = v[N + i];
-  }
-#pragma unroll 1
-  for (int q = 0; q < N; ++q) {
-    float col[R2];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      col[i] = S[L::Fj + q * N + i];
-      col[N + i] = 0.0f;
-    }
-    apply_reg<R2, N>(P, tau, col);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      Rr.Ft.at(q * N + i, se) = col[i];
-      Nx.F.at(q * N + i, sn) = col[N + i];
-    }
-  }
-#pragma unroll 1
-  for (int q = 0; q < N; ++q) {
-    float col[R2];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      col[i] = 0.0f;
-      col[N + i] = S[L::Yt + q * N + i];
-    }
-    apply_reg<R2, N>(P, tau, col);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      Rr.Y.at(q * N + i, se) = col[i];
-      Nx.H.at(q * N + i, sn) = col[N + i];
-    }
-  }
-}
-
-template <int N, int BP, int RA = N>
-__device__ __forceinline__ void ss_dispatch_a(int ra, const PairSlice<N, BP>& S)
-{
-  if constexpr (RA <= 2 * N) {
-    if (ra == RA) ss_stage_a<N, BP, RA>(S);
-    else ss_dispatch_a<N, BP, RA + 1>(ra, S);
-  }
-}
-
-template <int N, int BP, int RC = 1>
-__device__ __forceinline__ void ss_dispatch_c(int rc, const PairSlice<N, BP>& S, const Eq<float>& Nx, int64_t sn,
-                                              int mj)
-{
-  if constexpr (RC <= 2 * N) {
-    if (rc == RC) ss_stage_c<N, BP, RC>(S, Nx, sn, mj);
-    else ss_dispatch_c<N, BP, RC + 1>(rc, S, Nx, sn, mj);
-  }
-}
-
-constexpr int kPairSsBP = 64; /* default block size; 32 and 128 are tuning choices */
-
-template <int N, int BP = kPairSsBP>
-__global__ void __launch_bounds__(BP) pair_ss_kernel(Args<float, float> a, int)
-{
-  using L = PairSlice<N, BP>;
-  extern __shared__ __align__(16) float ss_smem[];
-  const int64_t item = (int64_t)blockIdx.x * BP + threadIdx.x;
-  if (item >= a.ct.npairs) return;
-  const int t = find_track(a.ct.pair, a.ntracks, item);
-  const int64_t p = item - a.ct.pair[t];
-  const int64_t sj = a.ct.slot[t] + 2 * p, sj1 = sj + 1;
-  const int64_t sn = a.nt.slot[t] + p, se = a.ct.solve[t] + p;
-  const Eq<float>& C = a.ce;
-  const int mj = C.m[sj], mj1 = C.m[sj1];
-  const L S{ss_smem + threadIdx.x};
-  auto cp = [&](int e, const Soa<float>& src, int es, int64_t s) { cp_async4(&S[e], &src.at(es, s)); };
-  /* group 0: stage A's pivot and right-hand side */
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      if (i < mj) cp(L::Gj + q * N + i, C.G, q * N + i, sj);
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    if (i < mj) cp(L::oj + i, C.o, i, sj);
-#pragma unroll
-  for (int e = 0; e < N * N; ++e) cp(L::F1 + e, C.F, e, sj1);
-#pragma unroll
-  for (int i = 0; i < N; ++i) cp(L::c1 + i, C.c, i, sj1);
-  cp_async_commit();
-  /* group 1: the H_{j+1} columns */
-#pragma unroll
-  for (int e = 0; e < N * N; ++e) cp(L::H1 + e, C.H, e, sj1);
-  cp_async_commit();
-  /* group 2: stage C's observation rows of step j+1 */
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      if (i < mj1) cp(L::G1 + q * N + i, C.G, q * N + i, sj1);
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    if (i < mj1) cp(L::o1 + i, C.o, i, sj1);
-  cp_async_commit();
-  /* group 3: stage B's blocks of step j (none for a track's first pair) */
-  if (p > 0) {
-#pragma unroll
-    for (int e = 0; e < N * N; ++e) {
-      cp(L::Hj + e, C.H, e, sj);
-      cp(L::Fj + e, C.F, e, sj);
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) cp(L::cj + i, C.c, i, sj);
-  }
-  cp_async_commit();
-
-  ss_dispatch_a<N, BP>(mj + N, S);
-  if (mj + mj1 == 0) a.ne.m[sn] = 0;
-  else ss_dispatch_c<N, BP>(mj + mj1, S, a.ne, sn, mj);
-  if (p == 0) { /* no stage B: the record is stage A's */
-    cp_async_wait<0>();
-#pragma unroll
-    for (int e = 0; e < N * N; ++e) {
-      a.cr.R.at(e, se) = S[L::Rt + e];
-      a.cr.Y.at(e, se) = S[L::Yt + e];
-      a.cr.Ft.at(e, se) = 0.0f;
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) a.cr.rhs.at(i, se) = S[L::rt + i];
-    return;
-  }
-  ss_stage_b<N, BP>(S, a.ne, a.cr, sn, se);
 }
 
 /* ---------------------------------------------------------------------------
@@ -1392,199 +1059,6 @@ __global__ void tail_kernel(Args<T, TI> a)
 }
 
 /* ---------------------------------------------------------------------------
- * FP32 tail work (states only) with register-resident blocks: the same
- * arithmetic as tail_kernel, each QR an instantiation with compile-time rows
- * (dispatched on the run-time row count).  Hand-offs between the stages (R~
- * and o' of the single step's observation, its leftover rows Z and o'') go
- * through a per-thread slice of shared memory, element e at [e*32 + lane].
- * ------------------------------------------------------------------------ */
-constexpr int kTailBS = 32;
-
-template <int N>
-struct TailSlice {
-  static constexpr int Rt = 0, op = N * N, Z = N * N + N, opp = 2 * N * N + N, width = 2 * N * N + 2 * N;
-  float* t0;
-  __device__ __forceinline__ float& operator[](int e) const { return t0[e * kTailBS]; }
-};
-
-/* observation QR of the single last step: [G_s | o_s], MS rows */
-template <int N, int MS>
-__device__ __forceinline__ void tail_obs(const Eq<float>& C, int64_t s, const TailSlice<N>& S)
-{
-  float P[N][MS], v[MS], tau[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < MS; ++i) P[q][i] = C.G.at(q * N + i, s);
-#pragma unroll
-  for (int i = 0; i < MS; ++i) v[i] = C.o.at(i, s);
-  hh_reg<MS, N>(P, tau);
-  apply_reg<MS, N>(P, tau, v);
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < MS; ++i) S[TailSlice<N>::Rt + q * N + i] = (i <= q) ? P[q][i] : 0.0f;
-#pragma unroll
-  for (int i = 0; i < MS; ++i) S[TailSlice<N>::op + i] = v[i];
-}
-
-/* evolution QR of the single last step: [H_s F_s c_s; R~ 0 o'], N+MT rows */
-template <int N, int MT>
-__device__ __forceinline__ void tail_evo(const Eq<float>& C, const Rec<float>& Rr, int64_t s, int64_t es,
-                                         const TailSlice<N>& S)
-{
-  using L = TailSlice<N>;
-  constexpr int R = N + MT;
-  float P[N][R], v[R], tau[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) P[q][i] = C.H.at(q * N + i, s);
-#pragma unroll
-    for (int i = 0; i < MT; ++i) P[q][N + i] = (i <= q) ? S[L::Rt + q * N + i] : 0.0f;
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = C.c.at(i, s);
-#pragma unroll
-  for (int i = 0; i < MT; ++i) v[N + i] = S[L::op + i];
-  hh_reg<R, N>(P, tau);
-  apply_reg<R, N>(P, tau, v);
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      Rr.R.at(q * N + i, es) = (i <= q) ? P[q][i] : 0.0f;
-      Rr.Y.at(q * N + i, es) = 0.0f;
-    }
-#pragma unroll
-  for (int i = 0; i < N; ++i) Rr.rhs.at(i, es) = v[i];
-#pragma unroll
-  for (int i = 0; i < MT; ++i) S[L::opp + i] = v[N + i];
-#pragma unroll 1
-  for (int q = 0; q < N; ++q) {
-    float col[R];
-#pragma unroll
-    for (int i = 0; i < N; ++i) col[i] = C.F.at(q * N + i, s);
-#pragma unroll
-    for (int i = 0; i < MT; ++i) col[N + i] = 0.0f;
-    apply_reg<R, N>(P, tau, col);
-#pragma unroll
-    for (int i = 0; i < N; ++i) Rr.Ft.at(q * N + i, es) = col[i];
-#pragma unroll
-    for (int i = 0; i < MT; ++i) S[L::Z + q * N + i] = col[N + i];
-  }
-}
-
-/* fix-up: QR of [G~ o (gp rows of the next level's slot); Z o''], RF rows */
-template <int N, int RF>
-__device__ __forceinline__ void tail_fix(const Eq<float>& Nx, int64_t sn, int gp, const TailSlice<N>& S)
-{
-  using L = TailSlice<N>;
-  float P[N][RF], v[RF], tau[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < RF; ++i) P[q][i] = i < gp ? Nx.G.at(q * N + i, sn) : S[L::Z + q * N + (i - gp)];
-#pragma unroll
-  for (int i = 0; i < RF; ++i) v[i] = i < gp ? Nx.o.at(i, sn) : S[L::opp + (i - gp)];
-  hh_reg<RF, N>(P, tau);
-  apply_reg<RF, N>(P, tau, v);
-  constexpr int G2 = RF < N ? RF : N;
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-#pragma unroll
-    for (int i = 0; i < G2; ++i) Nx.G.at(q * N + i, sn) = (i <= q) ? P[q][i] : 0.0f;
-#pragma unroll
-  for (int i = 0; i < G2; ++i) Nx.o.at(i, sn) = v[i];
-  Nx.m[sn] = G2;
-}
-
-template <int N, int K = 1>
-__device__ __forceinline__ void tail_obs_d(int ms, const Eq<float>& C, int64_t s, const TailSlice<N>& S)
-{
-  if constexpr (K <= N) {
-    if (ms == K) tail_obs<N, K>(C, s, S);
-    else tail_obs_d<N, K + 1>(ms, C, s, S);
-  }
-}
-template <int N, int K = 0>
-__device__ __forceinline__ void tail_evo_d(int mt, const Eq<float>& C, const Rec<float>& Rr, int64_t s, int64_t es,
-                                           const TailSlice<N>& S)
-{
-  if constexpr (K <= N) {
-    if (mt == K) tail_evo<N, K>(C, Rr, s, es, S);
-    else tail_evo_d<N, K + 1>(mt, C, Rr, s, es, S);
-  }
-}
-template <int N, int K = 1>
-__device__ __forceinline__ void tail_fix_d(int rf, const Eq<float>& Nx, int64_t sn, int gp, const TailSlice<N>& S)
-{
-  if constexpr (K <= 2 * N) {
-    if (rf == K) tail_fix<N, K>(Nx, sn, gp, S);
-    else tail_fix_d<N, K + 1>(rf, Nx, sn, gp, S);
-  }
-}
-
-template <int N>
-__global__ void __launch_bounds__(kTailBS) tail_reg_kernel(Args<float, float> a)
-{
-  __shared__ float tail_smem[TailSlice<N>::width * kTailBS];
-  const int64_t item = (int64_t)blockIdx.x * kTailBS + threadIdx.x;
-  if (item >= a.ct.ntail) return;
-  const Eq<float>& C = a.ce;
-  const int t = (int)a.ct.tail[item];
-  const int64_t L = a.ct.L[t];
-  const int64_t sb = a.ct.slot[t];
-  if (L == 1) { /* base case: x = R^{-1} Q^T o */
-    const int m0 = C.m[sb];
-    double* x = a.state + orig_step(a.track_start, a.level, t, 0) * N;
-    if (m0 < N) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) x[i] = NAN;
-      atomicOr(a.flag, 2);
-      return;
-    }
-    float P[N][N], v[N], tau[N];
-#pragma unroll
-    for (int q = 0; q < N; ++q)
-#pragma unroll
-      for (int i = 0; i < N; ++i) P[q][i] = C.G.at(q * N + i, sb);
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = C.o.at(i, sb);
-    hh_reg<N, N>(P, tau);
-    apply_reg<N, N>(P, tau, v);
-    bool bad = false;
-    if (a.baseR.p)
-#pragma unroll
-      for (int q = 0; q < N; ++q)
-#pragma unroll
-        for (int i = 0; i < N; ++i) a.baseR.at(q * N + i, t) = (i <= q) ? P[q][i] : 0.0f;
-#pragma unroll
-    for (int i = N - 1; i >= 0; --i) {
-      float sm = v[i];
-#pragma unroll
-      for (int k = i + 1; k < N; ++k) sm = fmaf(-P[k][i], v[k], sm);
-      bad |= P[i][i] == 0.0f;
-      v[i] = sm * (1.0f / P[i][i]);
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) x[i] = ukg_df::f32_to_f64(v[i]);
-    if (bad) atomicOr(a.flag, 2);
-    return;
-  }
-  const TailSlice<N> S{tail_smem + threadIdx.x};
-  const int64_t s = sb + L - 1;
-  const int64_t es = a.ct.solve[t] + (L - 1) / 2;
-  const int64_t sn = a.nt.slot[t] + L / 2 - 1;
-  const int ms = C.m[s], mt = ms < N ? ms : N;
-  if (ms > 0) tail_obs_d<N>(ms, C, s, S);
-  tail_evo_d<N>(mt, C, a.cr, s, es, S);
-  const int gp = a.ne.m[sn], rf = gp + mt;
-  if (rf > 0) tail_fix_d<N>(rf, a.ne, sn, gp, S);
-  else a.ne.m[sn] = 0;
-}
-
-/* ---------------------------------------------------------------------------
  * back-substitution and covariance recurrence for the even steps of a level
  *
  * With B = [Ft Y] and Sigma = [[Smm Smp]; [Smp^T Spp]] the joint covariance of
@@ -1597,14 +1071,14 @@ __global__ void __launch_bounds__(kTailBS) tail_reg_kernel(Args<float, float> a)
  * B Sigma, which are streamed one at a time).  In a refinement sweep the
  * right-hand side is y (yrhs) and `state` holds the correction d.
  * ------------------------------------------------------------------------ */
-template <typename T, int NT = 0, int BS = 0>
-__global__ void __launch_bounds__(BS ? BS : 1024) solve_kernel(Args<T, T> a, int want_cov)
+template <typename T>
+__global__ void solve_kernel(Args<T, T> a, int want_cov)
 {
   extern __shared__ unsigned char smem_raw[];
   T* smem = reinterpret_cast<T*>(smem_raw);
   const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= a.ct.nsolve) return;
-  const int n = NT ? NT : a.n;
+  const int n = a.n;
   const int64_t nn = (int64_t)n * n;
   const Rec<T>& Rr = a.cr;
   const int t = find_track(a.ct.solve, a.ntracks, item);
@@ -1616,9 +1090,8 @@ __global__ void __launch_bounds__(BS ? BS : 1024) solve_kernel(Args<T, T> a, int
   const int64_t om = hp ? orig_step(a.track_start, a.level, t, j - 1) : 0;
   const int64_t op = hn ? orig_step(a.track_start, a.level, t, j + 1) : 0;
 
-  using View = typename ViewOf<T, BS>::type;
-  View ws = ViewOf<T, BS>::make(smem);
-  View Rs = ws, Fs = ws + n * n, Ys = ws + 2 * n * n, M = ws + 3 * n * n, sg = ws + 4 * n * n, pv = sg + 2 * n,
+  PV<T> ws{smem + threadIdx.x, (int)blockDim.x};
+  PV<T> Rs = ws, Fs = ws + n * n, Ys = ws + 2 * n * n, M = ws + 3 * n * n, sg = ws + 4 * n * n, pv = sg + 2 * n,
        dv = pv + n;
   bool bad = false;
   for (int k = 0; k < n * n; ++k) {
@@ -1687,7 +1160,7 @@ __global__ void __launch_bounds__(BS ? BS : 1024) solve_kernel(Args<T, T> a, int
         for (int i = 0; i < n; ++i) pv[i] = fma(Ys[k * n + i], sk, pv[i]);
       }
     /* M += pv b_q^T, b_q = column q of B */
-    View bq = q < n ? Fs + q * n : Ys + (q - n) * n;
+    PV<T> bq = q < n ? Fs + q * n : Ys + (q - n) * n;
     for (int c = 0; c < n; ++c) {
       const T bc = bq[c];
       for (int i = 0; i < n; ++i) M[c * n + i] = fma(pv[i], bc, M[c * n + i]);
@@ -2061,129 +1534,114 @@ __global__ void __launch_bounds__(128) solve_state_reg_kernel(Args<float, float>
     bad |= R[i][i] == 0.0f;
     pv[i] = sm * (1.0f / R[i][i]);
   }
-  double* xo = a.state + orig_step(a.track_start, a.level, t, j) * N;
+  const int64_t so = orig_step(a.track_start, a.level, t, j) * N;
+  if (a.xadd)
 #pragma unroll
-  for (int i = 0; i < N; ++i) xo[i] = ukg_df::f32_to_f64(pv[i]);
+    for (int i = 0; i < N; ++i) a.xadd[so + i] += ukg_df::f32_to_f64(pv[i]);
+  if (!a.xadd || a.level > 0) /* nothing reads a correction of level 0 */
+#pragma unroll
+    for (int i = 0; i < N; ++i) a.state[so + i] = ukg_df::f32_to_f64(pv[i]);
   if (bad) atomicOr(a.flag, 2);
 }
 
+/* One level of R^T y = z for the refinement: thread e of the even steps takes
+ * y_{2e} = R^{-T} z_{2e} and, where step 2e + 1 exists, the next level's
+ * z' = z_{2e+1} - Y^T y_{2e} - Ft^T y_{2e+2} with its neighbour's y computed
+ * again (a triangular solve costs less than another launch and a round trip of
+ * y through memory: 43 launches of a 14-level smoothing became 15); the
+ * threads past the even steps take the tracks that have one step left, R^T y =
+ * z and R d = y with the base factor.                                        */
 template <int N>
-__global__ void __launch_bounds__(128) rt_even_reg_kernel(Args<float, float> a, Soa<float> zc, Soa<float> yc)
+__global__ void __launch_bounds__(128) rt_level_kernel(Args<float, float> a, Soa<float> zc, Soa<float> yc, Soa<float> zn)
 {
   const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= a.ct.nsolve) return;
-  const int t = find_track(a.ct.solve, a.ntracks, item);
-  const int64_t sz = a.ct.slot[t] + 2 * (item - a.ct.solve[t]);
-  float R[N][N], y[N];
+  float R[N][N], y[N]; /* R[j][i]: row i of column j, i <= j */
+  auto load = [&](const Soa<float>& Rm, int64_t e, int64_t sz) {
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    y[k] = zc.at(k, sz);
+    for (int k = 0; k < N; ++k) {
+      y[k] = zc.at(k, sz);
 #pragma unroll
-    for (int i = 0; i <= k; ++i) R[k][i] = a.cr.R.at(k * N + i, item);
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    float sm = y[i];
-#pragma unroll
-    for (int k = 0; k < i; ++k) sm = fmaf(-R[i][k], y[k], sm);
-    y[i] = sm * (1.0f / R[i][i]);
-    yc.at(i, item) = y[i];
-  }
-}
-
-template <int N>
-__global__ void __launch_bounds__(128) rt_odd_reg_kernel(Args<float, float> a, Soa<float> zc, Soa<float> yc,
-                                                         Soa<float> zn)
-{
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= a.ct.npairs) return;
-  const int t = find_track(a.ct.pair, a.ntracks, item);
-  const int64_t p = item - a.ct.pair[t], L = a.ct.L[t];
-  const int64_t so = a.ct.slot[t] + 2 * p + 1, sn = a.nt.slot[t] + p;
-  const int64_t e0 = a.ct.solve[t] + p, e1 = e0 + 1;
-  const bool right = 2 * p + 2 <= L - 1;
-  float Y[N][N], y0[N], z[N];
-#pragma unroll
-  for (int c = 0; c < N; ++c) {
-    z[c] = zc.at(c, so);
-    y0[c] = yc.at(c, e0);
-#pragma unroll
-    for (int r = 0; r < N; ++r) Y[c][r] = a.cr.Y.at(c * N + r, e0);
-  }
-  if (right) {
-    float F[N][N], y1[N];
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-      y1[c] = yc.at(c, e1);
-#pragma unroll
-      for (int r = 0; r < N; ++r) F[c][r] = a.cr.Ft.at(c * N + r, e1);
+      for (int i = 0; i <= k; ++i) R[k][i] = Rm.at(k * N + i, e);
     }
+  };
+  auto solve_t = [&]() {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float sm = y[i];
+#pragma unroll
+      for (int k = 0; k < i; ++k) sm = fmaf(-R[i][k], y[k], sm);
+      y[i] = sm * (1.0f / R[i][i]);
+    }
+  };
+  if (item >= a.ct.nsolve) { /* base cases */
+    const int64_t b = item - a.ct.nsolve;
+    if (b >= a.ct.ntail) return;
+    const int t = (int)a.ct.tail[b];
+    if (a.ct.L[t] != 1) return;
+    load(a.baseR, t, a.ct.slot[t]);
+    solve_t();
+#pragma unroll
+    for (int j = N - 1; j >= 0; --j) { /* R d = y */
+      y[j] = y[j] * (1.0f / R[j][j]);
+#pragma unroll
+      for (int i = 0; i < j; ++i) y[i] = fmaf(-y[j], R[j][i], y[i]);
+    }
+    const int64_t so = orig_step(a.track_start, a.level, t, 0) * N;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const double d = ukg_df::f32_to_f64(y[i]);
+      a.state[so + i] = d;
+      if (a.xadd) a.xadd[so + i] += d;
+    }
+    return;
+  }
+  const int t = find_track(a.ct.solve, a.ntracks, item);
+  const int64_t e = item - a.ct.solve[t], L = a.ct.L[t];
+  const int64_t se = a.ct.slot[t] + 2 * e;
+  load(a.cr.R, item, se);
+  solve_t();
+#pragma unroll
+  for (int i = 0; i < N; ++i) yc.at(i, item) = y[i];
+  if (2 * e + 1 >= L) return;
+  float z[N];
+#pragma unroll
+  for (int c = 0; c < N; ++c) z[c] = zc.at(c, se + 1);
+  float Y[N][N];
+#pragma unroll
+  for (int c = 0; c < N; ++c)
+#pragma unroll
+    for (int r = 0; r < N; ++r) Y[c][r] = a.cr.Y.at(c * N + r, item);
+  float u[N]; /* Y^T y_{2e} is subtracted after Ft^T y_{2e+2} */
+#pragma unroll
+  for (int r = 0; r < N; ++r) u[r] = y[r];
+  if (2 * e + 2 < L) {
+    load(a.cr.R, item + 1, se + 2);
+    solve_t();
 #pragma unroll
     for (int c = 0; c < N; ++c)
 #pragma unroll
-      for (int r = 0; r < N; ++r) z[c] = fmaf(-F[c][r], y1[r], z[c]);
+      for (int r = 0; r < N; ++r) z[c] = fmaf(-a.cr.Ft.at(c * N + r, item + 1), y[r], z[c]);
   }
+  const int64_t sn = a.nt.slot[t] + e;
 #pragma unroll
   for (int c = 0; c < N; ++c) {
-    float sm = z[c];
 #pragma unroll
-    for (int r = 0; r < N; ++r) sm = fmaf(-Y[c][r], y0[r], sm);
-    zn.at(c, sn) = sm;
+    for (int r = 0; r < N; ++r) z[c] = fmaf(-Y[c][r], u[r], z[c]);
+    zn.at(c, sn) = z[c];
   }
-}
-
-/* rt_base_kernel with the track's base-case R and right-hand side in
- * registers: the same two triangular solves in the same order (the results
- * are identical), without a round trip to memory per operation.            */
-template <int N>
-__global__ void __launch_bounds__(128) rt_base_reg_kernel(Args<float, float> a, Soa<float> zc)
-{
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= a.ct.ntail) return;
-  const int t = (int)a.ct.tail[item];
-  if (a.ct.L[t] != 1) return;
-  const int64_t sz = a.ct.slot[t];
-  float R[N][N], v[N]; /* R[j][i]: row i of column j, i <= j */
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    v[j] = zc.at(j, sz);
-#pragma unroll
-    for (int i = 0; i <= j; ++i) R[j][i] = a.baseR.at(j * N + i, t);
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) { /* R^T y = z */
-    float sm = v[i];
-#pragma unroll
-    for (int k = 0; k < i; ++k) sm = fmaf(-R[i][k], v[k], sm);
-    v[i] = sm * (1.0f / R[i][i]);
-  }
-#pragma unroll
-  for (int j = N - 1; j >= 0; --j) { /* R d = y */
-    const float xj = v[j] * (1.0f / R[j][j]);
-    v[j] = xj;
-#pragma unroll
-    for (int i = 0; i < j; ++i) v[i] = fmaf(-xj, R[j][i], v[i]);
-  }
-  double* d = a.state + orig_step(a.track_start, a.level, t, 0) * N;
-#pragma unroll
-  for (int i = 0; i < N; ++i) d[i] = ukg_df::f32_to_f64(v[i]);
 }
 
 struct RegSolves {
   void (*solve)(Args<float, float>) = nullptr;
-  void (*rt_even)(Args<float, float>, Soa<float>, Soa<float>) = nullptr;
-  void (*rt_odd)(Args<float, float>, Soa<float>, Soa<float>, Soa<float>) = nullptr;
-  void (*rt_base)(Args<float, float>, Soa<float>) = nullptr;
+  void (*rt_level)(Args<float, float>, Soa<float>, Soa<float>, Soa<float>) = nullptr;
 };
 RegSolves reg_solves(int n)
 {
   RegSolves r;
-  if (n == 6)
-    r.solve = solve_state_reg_kernel<6>, r.rt_even = rt_even_reg_kernel<6>, r.rt_odd = rt_odd_reg_kernel<6>,
-    r.rt_base = rt_base_reg_kernel<6>;
-  if (n == 4)
-    r.solve = solve_state_reg_kernel<4>, r.rt_even = rt_even_reg_kernel<4>, r.rt_odd = rt_odd_reg_kernel<4>,
-    r.rt_base = rt_base_reg_kernel<4>;
+#define UKG_RS(N_) \
+  case N_: r.solve = solve_state_reg_kernel<N_>, r.rt_level = rt_level_kernel<N_>; break;
+  switch (n) { UKG_RS(2) UKG_RS(3) UKG_RS(4) UKG_RS(5) UKG_RS(6) UKG_RS(7) UKG_RS(8) default: break; }
+#undef UKG_RS
   return r;
 }
 
@@ -2201,6 +1659,7 @@ __global__ void add_kernel(double* x, const double* d, int64_t count)
  * host side: plan, workspace, launches
  * ------------------------------------------------------------------------ */
 constexpr int kMaxLevels = 64;
+constexpr int kPairBP = 64; /* default block size of the FP32 thread-per-pair kernel; 32 and 128 are tuning choices */
 constexpr int kResidBS = 128;
 
 /* double-float weighing and residual kernels for (n, mx), or null (FP32
@@ -2233,7 +1692,7 @@ DfKernels df_kernels(int n, int mmax, int weigh_bs = kWeighBS)
  * start of every call.  Defaults: a thread per item below 9 states, a thread
  * block per item from 9 on; four CTAs per SM; the block sizes the FP32
  * kernels were written for.                                                  */
-kalman_gpu_tuning_t default_tuning() { return kalman_gpu_tuning_t{9, 4, kPairSsBP, kWeighBS}; }
+kalman_gpu_tuning_t default_tuning() { return kalman_gpu_tuning_t{9, 4, kPairBP, kWeighBS}; }
 std::mutex g_tune_mu;
 kalman_gpu_tuning_t g_tune = default_tuning();
 kalman_gpu_tuning_t tuning_now()
@@ -2392,49 +1851,8 @@ Eq<T> eq_at(char* B, size_t off, size_t off_m, int64_t stride, int n, int mx)
   return d;
 }
 
-/* The pair and solve kernels used for a state dimension: FP32 instantiations
- * with compile-time n, mx and block size for the common small shapes, the
- * runtime-dimension kernels otherwise (FP64 and double-float up to 8 states
- * have their own, SmallKernels below).                                       */
-template <typename T>
-struct Kernels {
-  void (*pair)(Args<T, T>, int) = nullptr;
-  void (*solve)(Args<T, T>, int) = nullptr;
-  int bp = 0, bs = 0;     /* fixed block sizes of the specialised kernels (0: pick) */
-  size_t pair_smem = 0;   /* dynamic shared memory of the pair kernel (0: per-thread workspace) */
-};
-
-template <typename T>
-Kernels<T> choose_kernels(int n, int mx, int pair_bp = kPairSsBP)
-{
-  Kernels<T> k;
-  if constexpr (sizeof(T) == sizeof(float)) {
-    if (n == mx && (n == 6 || n == 4)) {
-      if (n == 6)
-        k.pair = pair_bp == 32 ? pair_ss_kernel<6, 32> : pair_bp == 128 ? pair_ss_kernel<6, 128> : pair_ss_kernel<6, 64>;
-      else
-        k.pair = pair_bp == 32 ? pair_ss_kernel<4, 32> : pair_bp == 128 ? pair_ss_kernel<4, 128> : pair_ss_kernel<4, 64>;
-      k.solve = n == 6 ? solve_kernel<T, 6, 64> : solve_kernel<T, 4, 64>;
-      k.bp = pair_bp;
-      k.bs = 64;
-      k.pair_smem = (size_t)pair_bp * sizeof(float) * (n == 6 ? PairSlice<6, 64>::width : PairSlice<4, 64>::width);
-      return k;
-    }
-    if (n == mx && n == 8) {
-      k.pair = pair_kernel<T, T, 8, 8, 128>;
-      k.solve = solve_kernel<T, 8, 64>;
-      k.bp = 128;
-      k.bs = 64;
-      return k;
-    }
-  }
-  k.pair = pair_kernel<T, T>;
-  k.solve = solve_kernel<T>;
-  return k;
-}
-
-/* The FP64 and double-float kernels for n <= 8 and mx == n (oddeven_small.cuh):
- * lanes or threads per item, by the number of items of a level.             */
+/* The kernels for 2 to 8 states and mx == n (oddeven_small.cuh): lanes or
+ * threads per item, by the number of items of a level.                      */
 template <typename T>
 struct SmallKernels {
   void (*pair32)(Args<T, T>) = nullptr;
@@ -2444,6 +1862,7 @@ struct SmallKernels {
   void (*solve32)(Args<T, T>) = nullptr;
   void (*solve1)(Args<T, T>) = nullptr;
   void (*state)(Args<T, T>) = nullptr;
+  int pair_bs = 0; /* threads per block of pair1 */
 };
 constexpr int kPairThreadBS = 128, kSolveThreadBS = 64;
 
@@ -2462,10 +1881,17 @@ constexpr int kPairThreadBS = 128, kSolveThreadBS = 64;
  * 32 lanes 14 to 120 us from 608 to 7296, thread 64 throughout.  At n = 7 and
  * 8 a thread's pivot block does not fit its registers; in double-float eight
  * lanes stay the fastest at every size (3.8 million pairs: 16.7 ms, against
- * 19.7 by threads in registers and 21.9 in shared memory).                  */
+ * 19.7 by threads in registers and 21.9 in shared memory).  In FP32 (the
+ * precision form; a thread per pair in shared memory took 21 to 25 us a level):
+ *   32 lanes 11 13 14 21 - 36 -, 8 lanes 13 13 13 17 - 19 36 (40,000: 63),
+ *   thread 25 25 25 25 - 25 50 (40,000: 50).                                 */
 template <typename T>
 struct SmallLimits {
   static constexpr int64_t pair32 = 2432, pair8 = INT64_MAX, solve32 = 7296;
+};
+template <>
+struct SmallLimits<float> {
+  static constexpr int64_t pair32 = 2432, pair8 = 19456;
 };
 template <>
 struct SmallLimits<double> {
@@ -2473,30 +1899,38 @@ struct SmallLimits<double> {
 };
 
 template <typename T, int N>
-SmallKernels<T> small_kernels_n()
+SmallKernels<T> small_kernels_n(int pair_bs)
 {
   SmallKernels<T> k;
   k.pair32 = small::pair_lanes<T, N, 32>;
   k.pair8 = small::pair_lanes<T, N, 8>;
+  k.pair_bs = kPairThreadBS;
   if constexpr (std::is_same<T, double>::value && N <= 6) k.pair1 = small::pair_thread<T, N, kPairThreadBS, 2>;
   k.tail = small::tail_lanes<T, N>;
-  k.solve32 = small::solve_lanes<T, N>;
-  k.solve1 = small::solve_thread<T, N, kSolveThreadBS>;
-  k.state = small::solve_state<T, N>;
+  if constexpr (std::is_same<T, float>::value) {
+    k.pair_bs = pair_bs;
+    constexpr int per_sm = N <= 6 ? 512 : 256; /* threads per SM: 128 or 255 registers each */
+    k.pair1 = pair_bs == 32    ? small::pair_thread<T, N, 32, per_sm / 32>
+              : pair_bs == 128 ? small::pair_thread<T, N, 128, per_sm / 128> : small::pair_thread<T, N, 64, per_sm / 64>;
+  } else {
+    k.solve32 = small::solve_lanes<T, N>;
+    k.solve1 = small::solve_thread<T, N, kSolveThreadBS>;
+    k.state = small::solve_state<T, N>;
+  }
   return k;
 }
 template <typename T>
-SmallKernels<T> small_kernels(int n, int mx)
+SmallKernels<T> small_kernels(int n, int mx, int pair_bs)
 {
   if (n != mx) return SmallKernels<T>();
   switch (n) {
-    case 2: return small_kernels_n<T, 2>();
-    case 3: return small_kernels_n<T, 3>();
-    case 4: return small_kernels_n<T, 4>();
-    case 5: return small_kernels_n<T, 5>();
-    case 6: return small_kernels_n<T, 6>();
-    case 7: return small_kernels_n<T, 7>();
-    case 8: return small_kernels_n<T, 8>();
+    case 2: return small_kernels_n<T, 2>(pair_bs);
+    case 3: return small_kernels_n<T, 3>(pair_bs);
+    case 4: return small_kernels_n<T, 4>(pair_bs);
+    case 5: return small_kernels_n<T, 5>(pair_bs);
+    case 6: return small_kernels_n<T, 6>(pair_bs);
+    case 7: return small_kernels_n<T, 7>(pair_bs);
+    case 8: return small_kernels_n<T, 8>(pair_bs);
     default: return SmallKernels<T>();
   }
 }
@@ -2610,16 +2044,12 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     return ukg_set_error(KALMAN_GPU_EINVAL, "state dimension %d (observation rows %d) needs more shared memory per "
                          "thread than this build's odd-even kernels use", n, mx);
   const kalman_gpu_tuning_t tune = tuning_now();
-  const Kernels<T> K = choose_kernels<T>(n, mx, tune.pair_block);
-  if (K.bp) bp = K.bp;
-  if (K.bs) bs = K.bs;
   ukg_allow_dynamic_smem((const void*)weigh_kernel<T>);
   if (staged)
     ukg_allow_dynamic_smem((const void*)weigh_staged_kernel<T>);
-  const size_t pair_smem = K.pair_smem ? K.pair_smem : bp * pt_pair;
-  ukg_allow_dynamic_smem((const void*)K.pair);
+  ukg_allow_dynamic_smem((const void*)pair_kernel<T, T>);
   ukg_allow_dynamic_smem((const void*)tail_kernel<T, T>);
-  ukg_allow_dynamic_smem((const void*)K.solve);
+  ukg_allow_dynamic_smem((const void*)solve_kernel<T>);
   ukg_allow_dynamic_smem((const void*)residual_kernel);
 
   auto grid = [](int64_t items, int block) { return (unsigned)((items + block - 1) / block); };
@@ -2689,67 +2119,31 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     a.flag = dflag;
     a.baseR = baseR;
   };
-  /* ---- FP64 and double-float, n <= 8: lane and thread kernels ---- */
-  if constexpr (sizeof(T) != sizeof(float)) {
-    const SmallKernels<T> SK = small_kernels<T>(n, mx);
-    if (SK.pair32) {
-      const int lw = small::kLaneWarps, lt = 32 * lw;
-      for (int l = 0; l < nlev; ++l) {
-        Args<T, T> a;
-        memset(&a, 0, sizeof(a));
-        common(a, l);
-        a.ce = l == 0 ? eq0() : eqT(l);
-        if (l + 1 < nlev) a.ne = eqT(l + 1);
-        const int64_t np = lp[l].npairs;
-        if (np > 0) {
-          if (np <= SmallLimits<T>::pair32)
-            UKG_LAUNCH(kPair, st, (SK.pair32<<<grid(np, lw), lt, 0, st>>>(a)));
-          else if (np <= SmallLimits<T>::pair8 || !SK.pair1)
-            UKG_LAUNCH(kPair, st, (SK.pair8<<<grid(np, 4 * lw), lt, 0, st>>>(a)));
-          else
-            UKG_LAUNCH(kPair, st, (SK.pair1<<<grid(np, kPairThreadBS), kPairThreadBS, 0, st>>>(a)));
-        }
-        if (lp[l].ntail > 0) UKG_LAUNCH(kTail, st, (SK.tail<<<grid(lp[l].ntail, lw), lt, 0, st>>>(a)));
-      }
-      const size_t smem_cov = (size_t)kSolveThreadBS * 2 * nn * ts;
-      ukg_allow_dynamic_smem((const void*)SK.solve1);
-      for (int l = nlev - 2; l >= 0; --l) {
-        Args<T, T> a;
-        memset(&a, 0, sizeof(a));
-        common(a, l);
-        const int64_t ns = lp[l].nsolve;
-        if (ns == 0) continue;
-        if (!want_cov)
-          UKG_LAUNCH(kSolve, st, (SK.state<<<grid(ns, 64), 64, 0, st>>>(a)));
-        else if (ns <= SmallLimits<T>::solve32)
-          UKG_LAUNCH(kSolve, st, (SK.solve32<<<grid(ns, lw), lt, 0, st>>>(a)));
-        else
-          UKG_LAUNCH(kSolve, st, (SK.solve1<<<grid(ns, kSolveThreadBS), kSolveThreadBS, smem_cov, st>>>(a)));
-      }
-      return enqueue_only ? 0 : finish_plan(st, dflag);
-    }
-  }
   /* ---- forward elimination ---- */
+  const SmallKernels<T> SK = small_kernels<T>(n, mx, tune.pair_block);
+  const int lw = small::kLaneWarps, lt = 32 * lw;
   for (int l = 0; l < nlev; ++l) {
     Args<T, T> a;
     memset(&a, 0, sizeof(a));
     common(a, l);
     a.ce = l == 0 ? eq0() : eqT(l);
     if (l + 1 < nlev) a.ne = eqT(l + 1);
-    if (lp[l].npairs > 0)
-      UKG_LAUNCH(kPair, st, (K.pair<<<grid(lp[l].npairs, bp), bp, pair_smem, st>>>(a, rmax)));
-    if (lp[l].ntail > 0)
-    {
-      bool done = false;
-      if constexpr (sizeof(T) == sizeof(float)) {
-        if (!want_cov && n == mx && (n == 6 || n == 4)) {
-          auto tk = n == 6 ? tail_reg_kernel<6> : tail_reg_kernel<4>;
-          UKG_LAUNCH(UKG_K_TAIL, st, (tk<<<grid(lp[l].ntail, kTailBS), kTailBS, 0, st>>>(a)));
-          done = true;
-        }
+    const int64_t np = lp[l].npairs, nt = lp[l].ntail;
+    if (SK.pair32) { /* n <= 8: lanes or threads per item */
+      if (np > 0) {
+        if (np <= SmallLimits<T>::pair32)
+          UKG_LAUNCH(kPair, st, (SK.pair32<<<grid(np, lw), lt, 0, st>>>(a)));
+        else if (np <= SmallLimits<T>::pair8 || !SK.pair1)
+          UKG_LAUNCH(kPair, st, (SK.pair8<<<grid(np, 4 * lw), lt, 0, st>>>(a)));
+        else
+          UKG_LAUNCH(kPair, st, (SK.pair1<<<grid(np, SK.pair_bs), SK.pair_bs, 0, st>>>(a)));
       }
-      if (!done)
-        UKG_LAUNCH(kTail, st, (tail_kernel<T, T><<<grid(lp[l].ntail, bt), bt, bt * pt_tail, st>>>(a)));
+      if (nt > 0) UKG_LAUNCH(kTail, st, (SK.tail<<<grid(nt, lw), lt, 0, st>>>(a)));
+      continue;
+    }
+    if (np > 0) UKG_LAUNCH(kPair, st, (pair_kernel<T, T><<<grid(np, bp), bp, bp * pt_pair, st>>>(a, rmax)));
+    if (nt > 0) {
+      UKG_LAUNCH(kTail, st, (tail_kernel<T, T><<<grid(nt, bt), bt, bt * pt_tail, st>>>(a)));
     }
   }
   /* ---- back-substitution ---- */
@@ -2757,14 +2151,25 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     Args<T, T> a;
     memset(&a, 0, sizeof(a));
     common(a, l);
-    if (lp[l].nsolve == 0) continue;
+    const int64_t ns = lp[l].nsolve;
+    if (ns == 0) continue;
     if constexpr (sizeof(T) == sizeof(float)) {
       if (RS.solve && !want_cov) {
-        UKG_LAUNCH(kSolve, st, (RS.solve<<<grid(lp[l].nsolve, 128), 128, 0, st>>>(a)));
+        UKG_LAUNCH(kSolve, st, (RS.solve<<<grid(ns, 128), 128, 0, st>>>(a)));
         continue;
       }
+    } else if (SK.solve32) {
+      const size_t smem_cov = (size_t)kSolveThreadBS * 2 * nn * ts;
+      ukg_allow_dynamic_smem((const void*)SK.solve1);
+      if (!want_cov)
+        UKG_LAUNCH(kSolve, st, (SK.state<<<grid(ns, 64), 64, 0, st>>>(a)));
+      else if (ns <= SmallLimits<T>::solve32)
+        UKG_LAUNCH(kSolve, st, (SK.solve32<<<grid(ns, lw), lt, 0, st>>>(a)));
+      else
+        UKG_LAUNCH(kSolve, st, (SK.solve1<<<grid(ns, kSolveThreadBS), kSolveThreadBS, smem_cov, st>>>(a)));
+      continue;
     }
-    UKG_LAUNCH(kSolve, st, (K.solve<<<grid(lp[l].nsolve, bs), bs, bs * pt_solve, st>>>(a, want_cov ? 1 : 0)));
+    UKG_LAUNCH(kSolve, st, (solve_kernel<T><<<grid(ns, bs), bs, bs * pt_solve, st>>>(a, want_cov ? 1 : 0)));
   }
   /* ---- refinement sweeps (FP32 factors only) ---- */
   if constexpr (sizeof(T) == sizeof(float)) {
@@ -2797,25 +2202,21 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
         a.cov = nullptr;
         Soa<float> zc{(float*)(B + P.o_z[l]), std::max<int64_t>(lp[l].S, 1)};
         Soa<float> yc{(float*)(B + P.o_y[l]), std::max<int64_t>(lp[l].E, 1)};
-        if (lp[l].nsolve > 0) {
-          if (RS.rt_even)
-            UKG_LAUNCH(UKG_K_RT, st, (RS.rt_even<<<grid(lp[l].nsolve, 128), 128, 0, st>>>(a, zc, yc)));
-          else
-            UKG_LAUNCH(UKG_K_RT, st, (rt_even_kernel<<<grid(lp[l].nsolve, 128), 128, 0, st>>>(a, zc, yc)));
+        Soa<float> zn{nullptr, 1};
+        if (l + 1 < nlev) zn = Soa<float>{(float*)(B + P.o_z[l + 1]), std::max<int64_t>(lp[l + 1].S, 1)};
+        if (RS.rt_level) {
+          a.xadd = p->state;
+          const int64_t items = lp[l].nsolve + lp[l].ntail;
+          if (items > 0) UKG_LAUNCH(UKG_K_RT, st, (RS.rt_level<<<grid(items, 128), 128, 0, st>>>(a, zc, yc, zn)));
+          continue;
         }
-        if (lp[l].npairs > 0 && l + 1 < nlev) {
-          Soa<float> zn{(float*)(B + P.o_z[l + 1]), std::max<int64_t>(lp[l + 1].S, 1)};
-          if (RS.rt_odd)
-            UKG_LAUNCH(UKG_K_RT, st, (RS.rt_odd<<<grid(lp[l].npairs, 128), 128, 0, st>>>(a, zc, yc, zn)));
-          else
-            UKG_LAUNCH(UKG_K_RT, st, (rt_odd_kernel<<<grid(lp[l].npairs, 128), 128, 0, st>>>(a, zc, yc, zn)));
-        }
+        if (lp[l].nsolve > 0)
+          UKG_LAUNCH(UKG_K_RT, st, (rt_even_kernel<<<grid(lp[l].nsolve, 128), 128, 0, st>>>(a, zc, yc)));
+        if (lp[l].npairs > 0 && l + 1 < nlev)
+          UKG_LAUNCH(UKG_K_RT, st, (rt_odd_kernel<<<grid(lp[l].npairs, 128), 128, 0, st>>>(a, zc, yc, zn)));
         if (lp[l].ntail > 0) {
           Soa<float> tmp{(float*)(B + P.o_tmp), std::max(T_, 1)};
-          if (RS.rt_base)
-            UKG_LAUNCH(UKG_K_RT, st, (RS.rt_base<<<grid(lp[l].ntail, 128), 128, 0, st>>>(a, zc)));
-          else
-            UKG_LAUNCH(UKG_K_RT, st, (rt_base_kernel<<<grid(lp[l].ntail, 128), 128, 0, st>>>(a, zc, tmp)));
+          UKG_LAUNCH(UKG_K_RT, st, (rt_base_kernel<<<grid(lp[l].ntail, 128), 128, 0, st>>>(a, zc, tmp)));
         }
       }
       for (int l = nlev - 2; l >= 0; --l) {
@@ -2825,14 +2226,16 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
         a.state = dx;
         a.cov = nullptr;
         a.yrhs = Soa<float>{(float*)(B + P.o_y[l]), std::max<int64_t>(lp[l].E, 1)};
+        if (RS.solve) a.xadd = p->state; /* every step's correction is found once: added there */
         if (lp[l].nsolve == 0) continue;
         if (RS.solve)
           UKG_LAUNCH(UKG_K_RSOLVE, st, (RS.solve<<<grid(lp[l].nsolve, 128), 128, 0, st>>>(a)));
         else
-          UKG_LAUNCH(UKG_K_RSOLVE, st, (K.solve<<<grid(lp[l].nsolve, bs), bs, bs * pt_solve, st>>>(a, 0)));
+          UKG_LAUNCH(UKG_K_RSOLVE, st, (solve_kernel<T><<<grid(lp[l].nsolve, bs), bs, bs * pt_solve, st>>>(a, 0)));
       }
       const int64_t cnt = p->nsteps * n;
-      UKG_LAUNCH(UKG_K_REFINE, st, (add_kernel<<<grid(cnt, 256), 256, 0, st>>>(p->state, dx, cnt)));
+      if (!RS.solve)
+        UKG_LAUNCH(UKG_K_REFINE, st, (add_kernel<<<grid(cnt, 256), 256, 0, st>>>(p->state, dx, cnt)));
     }
   }
   return enqueue_only ? 0 : finish_plan(st, dflag);

@@ -471,11 +471,17 @@ __device__ __forceinline__ void thread_a_full(const Args<T, T>& a, const PairIdx
 #pragma unroll
   for (int i = 0; i < MB; ++i)
     if (i < I.mj) a.ne.o.at(i, I.sn) = v[N + i];
+  T hn[N]; /* the next column, on its way */
+#pragma unroll
+  for (int i = 0; i < N; ++i) hn[i] = C.H.at(i, I.sj1);
 #pragma unroll 1
   for (int q = 0; q < N; ++q) {
     T h[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i) h[i] = i < N ? C.H.at(q * N + i, I.sj1) : T(0);
+    for (int i = 0; i < R; ++i) h[i] = i < N ? hn[i] : T(0);
+    if (q + 1 < N)
+#pragma unroll
+      for (int i = 0; i < N; ++i) hn[i] = C.H.at((q + 1) * N + i, I.sj1);
     thread_apply_full<T, N, R>(p, am, iv, h);
 #pragma unroll
     for (int i = 0; i < N; ++i) a.cr.Y.at(q * N + i, I.se) = h[i];
@@ -554,11 +560,17 @@ __global__ void __launch_bounds__(BS, MINB) pair_thread(Args<T, T> a)
     thread_apply_tri<T, N>(x, am, iv, vt, vb);
 #pragma unroll
     for (int i = 0; i < N; ++i) Nx.o.at(i, I.sn) = vb[i];
+    T hn[N]; /* the next column, on its way */
+#pragma unroll
+    for (int i = 0; i < N; ++i) hn[i] = C.H.at(i, I.sj1);
 #pragma unroll 1
     for (int q = 0; q < N; ++q) {
       T ht[N], hb[N];
 #pragma unroll
-      for (int i = 0; i < N; ++i) ht[i] = T(0), hb[i] = C.H.at(q * N + i, I.sj1);
+      for (int i = 0; i < N; ++i) ht[i] = T(0), hb[i] = hn[i];
+      if (q + 1 < N)
+#pragma unroll
+        for (int i = 0; i < N; ++i) hn[i] = C.H.at((q + 1) * N + i, I.sj1);
       thread_apply_tri<T, N>(x, am, iv, ht, hb);
 #pragma unroll
       for (int i = 0; i < N; ++i) {
@@ -584,24 +596,32 @@ __global__ void __launch_bounds__(BS, MINB) pair_thread(Args<T, T> a)
     thread_apply_tri<T, N>(x, am, iv, vt, vb);
 #pragma unroll
     for (int i = 0; i < N; ++i) Nx.c.at(i, I.sn) = vb[i];
+    T nx[N]; /* the next column, on its way: F_j's, then Y~'s */
+#pragma unroll
+    for (int i = 0; i < N; ++i) nx[i] = C.F.at(i, I.sj);
 #pragma unroll 1
     for (int q = 0; q < 2 * N; ++q) {
+      const bool isF = q < N;
+      const int c = isF ? q : q - N;
       T ct[N], cb[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        ct[i] = q < N ? Rr.Y.at(q * N + i, I.se) : T(0);
-        cb[i] = q < N ? T(0) : C.F.at((q - N) * N + i, I.sj);
+        ct[i] = isF ? T(0) : nx[i];
+        cb[i] = isF ? nx[i] : T(0);
+      }
+      if (q + 1 < 2 * N) {
+        const T* src = q + 1 < N ? &C.F.at((q + 1) * N, I.sj) : &Rr.Y.at((q + 1 - N) * N, I.se);
+        const int64_t st = q + 1 < N ? C.F.stride : Rr.Y.stride;
+#pragma unroll
+        for (int i = 0; i < N; ++i) nx[i] = src[i * st];
       }
       thread_apply_tri<T, N>(x, am, iv, ct, cb);
+      const Soa<T> top{&(isF ? Rr.Ft : Rr.Y).at(c * N, I.se), Rr.R.stride};
+      const Soa<T> bot{&(isF ? Nx.F : Nx.H).at(c * N, I.sn), Nx.F.stride};
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        if (q < N) {
-          Rr.Y.at(q * N + i, I.se) = ct[i];
-          Nx.H.at(q * N + i, I.sn) = cb[i];
-        } else {
-          Rr.Ft.at((q - N) * N + i, I.se) = ct[i];
-          Nx.F.at((q - N) * N + i, I.sn) = cb[i];
-        }
+        top.at(i, 0) = ct[i];
+        bot.at(i, 0) = cb[i];
       }
     }
   } else {
