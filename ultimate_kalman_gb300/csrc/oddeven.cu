@@ -1481,28 +1481,24 @@ __global__ void rt_base_kernel(Args<float, float> a, Soa<float> zc, Soa<float> t
  * before its arithmetic, which keeps many loads in flight per SM.  Same
  * arithmetic as solve_kernel (want_cov = 0), rt_even_kernel and rt_odd_kernel.
  * ------------------------------------------------------------------------ */
-template <int N>
-__global__ void __launch_bounds__(128) solve_state_reg_kernel(Args<float, float> a)
+/* One even step: x <- x_j from its neighbours' entries xm(k), xp(k) (where hp
+ * and hn), or its correction from theirs; true on a zero pivot                */
+template <int N, class XM, class XP>
+__device__ __forceinline__ bool solve_state_step(const Rec<float>& Rr, const Soa<float>& rhs, int64_t rhs_at, int64_t item,
+                                                 bool hp, bool hn, XM xm, XP xp, float (&pv)[N])
 {
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= a.ct.nsolve) return;
-  const int t = find_track(a.ct.solve, a.ntracks, item);
-  const int64_t j = 2 * (item - a.ct.solve[t]), L = a.ct.L[t];
-  const bool hp = j > 0, hn = j + 1 < L;
-  const Rec<float>& Rr = a.cr;
-  float R[N][N], pv[N];
+  float R[N][N];
 #pragma unroll
   for (int k = 0; k < N; ++k)
 #pragma unroll
     for (int i = 0; i <= k; ++i) R[k][i] = Rr.R.at(k * N + i, item);
 #pragma unroll
-  for (int i = 0; i < N; ++i) pv[i] = a.yrhs.p ? a.yrhs.at(i, item) : Rr.rhs.at(i, item);
+  for (int i = 0; i < N; ++i) pv[i] = rhs.at(i, rhs_at);
   if (hp) {
-    const double* xm = a.state + orig_step(a.track_start, a.level, t, j - 1) * N;
     float F[N][N], x[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      x[k] = ukg_df::f64_to_f32(xm[k]);
+      x[k] = xm(k);
 #pragma unroll
       for (int i = 0; i < N; ++i) F[k][i] = Rr.Ft.at(k * N + i, item);
     }
@@ -1512,11 +1508,10 @@ __global__ void __launch_bounds__(128) solve_state_reg_kernel(Args<float, float>
       for (int i = 0; i < N; ++i) pv[i] = fmaf(-F[k][i], x[k], pv[i]);
   }
   if (hn) {
-    const double* xp = a.state + orig_step(a.track_start, a.level, t, j + 1) * N;
     float Y[N][N], x[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      x[k] = ukg_df::f64_to_f32(xp[k]);
+      x[k] = xp(k);
 #pragma unroll
       for (int i = 0; i < N; ++i) Y[k][i] = Rr.Y.at(k * N + i, item);
     }
@@ -1534,14 +1529,36 @@ __global__ void __launch_bounds__(128) solve_state_reg_kernel(Args<float, float>
     bad |= R[i][i] == 0.0f;
     pv[i] = sm * (1.0f / R[i][i]);
   }
-  const int64_t so = orig_step(a.track_start, a.level, t, j) * N;
-  if (a.xadd)
+  return bad;
+}
+/* the state or correction v of a step: to state, and added to xadd if given */
+template <int N>
+__device__ __forceinline__ void put_state(const float (&v)[N], double* state, double* xadd, bool keep)
+{
+  if (xadd)
 #pragma unroll
-    for (int i = 0; i < N; ++i) a.xadd[so + i] += ukg_df::f32_to_f64(pv[i]);
-  if (!a.xadd || a.level > 0) /* nothing reads a correction of level 0 */
+    for (int i = 0; i < N; ++i) xadd[i] += ukg_df::f32_to_f64(v[i]);
+  if (keep)
 #pragma unroll
-    for (int i = 0; i < N; ++i) a.state[so + i] = ukg_df::f32_to_f64(pv[i]);
-  if (bad) atomicOr(a.flag, 2);
+    for (int i = 0; i < N; ++i) state[i] = ukg_df::f32_to_f64(v[i]);
+}
+
+template <int N>
+__global__ void __launch_bounds__(128) solve_state_reg_kernel(Args<float, float> a)
+{
+  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (item >= a.ct.nsolve) return;
+  const int t = find_track(a.ct.solve, a.ntracks, item);
+  const int64_t j = 2 * (item - a.ct.solve[t]), L = a.ct.L[t];
+  const int64_t d = (int64_t)N << a.level;
+  double* x = a.state + orig_step(a.track_start, a.level, t, j) * N;
+  float v[N];
+  if (solve_state_step<N>(a.cr, a.yrhs.p ? a.yrhs : a.cr.rhs, item, item, j > 0, j + 1 < L,
+                          [&](int k) { return ukg_df::f64_to_f32(x[k - d]); },
+                          [&](int k) { return ukg_df::f64_to_f32(x[k + d]); }, v))
+    atomicOr(a.flag, 2);
+  /* nothing reads a correction of level 0 */
+  put_state<N>(v, x, a.xadd ? a.xadd + (x - a.state) : nullptr, !a.xadd || a.level > 0);
 }
 
 /* One level of R^T y = z for the refinement: thread e of the even steps takes
@@ -1552,19 +1569,19 @@ __global__ void __launch_bounds__(128) solve_state_reg_kernel(Args<float, float>
  * threads past the even steps take the tracks that have one step left, R^T y =
  * z and R d = y with the base factor.                                        */
 template <int N>
-__global__ void __launch_bounds__(128) rt_level_kernel(Args<float, float> a, Soa<float> zc, Soa<float> yc, Soa<float> zn)
-{
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+struct RtStep {
   float R[N][N], y[N]; /* R[j][i]: row i of column j, i <= j */
-  auto load = [&](const Soa<float>& Rm, int64_t e, int64_t sz) {
+  __device__ __forceinline__ void load(const Soa<float>& Rm, int64_t e, const Soa<float>& zc, int64_t sz)
+  {
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       y[k] = zc.at(k, sz);
 #pragma unroll
       for (int i = 0; i <= k; ++i) R[k][i] = Rm.at(k * N + i, e);
     }
-  };
-  auto solve_t = [&]() {
+  }
+  __device__ __forceinline__ void solve_t() /* y <- R^{-T} y */
+  {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       float sm = y[i];
@@ -1572,74 +1589,196 @@ __global__ void __launch_bounds__(128) rt_level_kernel(Args<float, float> a, Soa
       for (int k = 0; k < i; ++k) sm = fmaf(-R[i][k], y[k], sm);
       y[i] = sm * (1.0f / R[i][i]);
     }
-  };
+  }
+  /* the even step of record `item` in slot se (its y to entry ye), and the odd step after it (to
+   * the next level's slot sn) if there is one, with the even step after that */
+  __device__ __forceinline__ void even(const Rec<float>& cr, const Soa<float>& zc, const Soa<float>& yc,
+                                       const Soa<float>& zn, int64_t item, int64_t ye, int64_t se, int64_t sn, bool odd,
+                                       bool next)
+  {
+    load(cr.R, item, zc, se);
+    solve_t();
+#pragma unroll
+    for (int i = 0; i < N; ++i) yc.at(i, ye) = y[i];
+    if (!odd) return;
+    float z[N], u[N], Y[N][N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+      z[c] = zc.at(c, se + 1);
+      u[c] = y[c]; /* Y^T y_{2e} is subtracted after Ft^T y_{2e+2} */
+#pragma unroll
+      for (int r = 0; r < N; ++r) Y[c][r] = cr.Y.at(c * N + r, item);
+    }
+    if (next) {
+      load(cr.R, item + 1, zc, se + 2);
+      solve_t();
+#pragma unroll
+      for (int c = 0; c < N; ++c)
+#pragma unroll
+        for (int r = 0; r < N; ++r) z[c] = fmaf(-cr.Ft.at(c * N + r, item + 1), y[r], z[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+#pragma unroll
+      for (int r = 0; r < N; ++r) z[c] = fmaf(-Y[c][r], u[r], z[c]);
+      zn.at(c, sn) = z[c];
+    }
+  }
+  /* a track's last step, R^T y = z, R d = y: d in y */
+  __device__ __forceinline__ void base(const Soa<float>& baseR, int t, const Soa<float>& zc, int64_t sz)
+  {
+    load(baseR, t, zc, sz);
+    solve_t();
+#pragma unroll
+    for (int j = N - 1; j >= 0; --j) {
+      y[j] = y[j] * (1.0f / R[j][j]);
+#pragma unroll
+      for (int i = 0; i < j; ++i) y[i] = fmaf(-y[j], R[j][i], y[i]);
+    }
+  }
+};
+
+template <int N>
+__global__ void __launch_bounds__(128) rt_level_kernel(Args<float, float> a, Soa<float> zc, Soa<float> yc, Soa<float> zn)
+{
+  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  RtStep<N> S;
   if (item >= a.ct.nsolve) { /* base cases */
     const int64_t b = item - a.ct.nsolve;
     if (b >= a.ct.ntail) return;
     const int t = (int)a.ct.tail[b];
     if (a.ct.L[t] != 1) return;
-    load(a.baseR, t, a.ct.slot[t]);
-    solve_t();
-#pragma unroll
-    for (int j = N - 1; j >= 0; --j) { /* R d = y */
-      y[j] = y[j] * (1.0f / R[j][j]);
-#pragma unroll
-      for (int i = 0; i < j; ++i) y[i] = fmaf(-y[j], R[j][i], y[i]);
-    }
     const int64_t so = orig_step(a.track_start, a.level, t, 0) * N;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const double d = ukg_df::f32_to_f64(y[i]);
-      a.state[so + i] = d;
-      if (a.xadd) a.xadd[so + i] += d;
-    }
+    S.base(a.baseR, t, zc, a.ct.slot[t]);
+    put_state<N>(S.y, a.state + so, a.xadd + so, true);
     return;
   }
   const int t = find_track(a.ct.solve, a.ntracks, item);
   const int64_t e = item - a.ct.solve[t], L = a.ct.L[t];
-  const int64_t se = a.ct.slot[t] + 2 * e;
-  load(a.cr.R, item, se);
-  solve_t();
+  S.even(a.cr, zc, yc, zn, item, item, a.ct.slot[t] + 2 * e, a.nt.slot[t] + e, 2 * e + 1 < L, 2 * e + 2 < L);
+}
+
+/* The levels from l0 on of a track by one block: in a refinement sweep the
+ * transpose solves up to the base, then (always) the back-substitution down to
+ * l0.  For few tracks, whose upper levels are a launch of a block or two each.
+ * What one level leaves for the next (z, y, states or corrections) stays in
+ * shared memory, and a level's factors are brought into L1 while the one before
+ * runs, so a level is a barrier and a short chain instead of 5 to 7 us.       */
+constexpr int kTopThreads = 512;
+constexpr int kTopSteps = 1024; /* a track's steps at level l0 at most: an even step per thread */
+constexpr int kTopTracks = 304; /* two blocks on each of 152 SMs */
+struct TopLevel {
+  const int64_t *slot, *solve;
+  Rec<float> rec;
+};
+struct TopArgs {
+  int l0;
+  bool refine;
+  const int64_t* track_start;
+  double *state, *xadd;
+  Soa<float> baseR, z; /* z: level l0's */
+  int* flag;
+  TopLevel lev[32];
+};
+/* shared memory: N entries each of z at every level, y of every even step, and
+ * the states (or corrections) of level l0's steps                            */
+constexpr int kTopZ = 2 * kTopSteps + 32, kTopY = kTopSteps + 32;
+constexpr size_t top_smem(int n) { return (size_t)n * (kTopZ + kTopY + kTopSteps) * sizeof(float); }
+
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
+template <int N>
+__global__ void __launch_bounds__(kTopThreads) top_levels_kernel(const __grid_constant__ TopArgs a)
+{
+  extern __shared__ float top_buf[];
+  __shared__ int64_t rec0[32]; /* the track's first record at each level */
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const int64_t s0 = a.track_start[t], len = a.track_start[t + 1] - s0;
+  const int L0 = (int)(len >> a.l0);
+  if (L0 == 0) return; /* finished below */
+  int nl = 0; /* levels above l0 */
+  while ((L0 >> nl) > 1) ++nl;
+  if (tid < nl) rec0[tid] = a.lev[a.l0 + tid].solve[t];
+  float* zs = top_buf;
+  float* ys = zs + N * kTopZ;
+  float* xs = ys + N * kTopY; /* entry c of level l0's step q: xs[c * kTopSteps + q] */
+  __syncthreads();
+  auto fetch = [&](int u, bool next) { /* level u's factors for this thread's even step */
+    if (u >= nl || u < 0 || 2 * tid >= (L0 >> u)) return;
+    const Rec<float>& V = a.lev[a.l0 + u].rec;
+    const int64_t item = rec0[u] + tid;
+    if (tid & 7) return; /* a 32-byte sector holds eight records of an entry */
+    for (int e = 0; e < N * N; ++e) {
+      prefetch_l1(&V.R.at(e, item));
+      prefetch_l1(&V.Y.at(e, item));
+      prefetch_l1(&V.Ft.at(e, item));
+    }
+    if (next)
+      for (int e = 0; e < N; ++e) prefetch_l1(&V.rhs.at(e, item));
+  };
+  auto zoff = [&](int u) { int o = 0; for (int v = 0; v < u; ++v) o += (L0 >> v) + 1; return o; };
+  auto yoff = [&](int u) { int o = 0; for (int v = 0; v < u; ++v) o += ((L0 >> v) + 1) / 2; return o; };
+  const int qb = (1 << nl) - 1; /* the base's step */
+  bool bad = false;
+  if (a.refine) {
+    RtStep<N> S;
+    for (int q = tid; q < L0; q += kTopThreads)
 #pragma unroll
-  for (int i = 0; i < N; ++i) yc.at(i, item) = y[i];
-  if (2 * e + 1 >= L) return;
-  float z[N];
+      for (int c = 0; c < N; ++c) zs[c * kTopZ + q] = a.z.at(c, a.lev[a.l0].slot[t] + q);
+    __syncthreads();
+    for (int u = 0; u < nl; ++u) {
+      const int L = L0 >> u;
+      fetch(u + 1, false);
+      const Soa<float> zc{zs + zoff(u), kTopZ}, zn{zs + zoff(u + 1), kTopZ}, yc{ys + yoff(u), kTopY};
+      if (2 * tid < L)
+        S.even(a.lev[a.l0 + u].rec, zc, yc, zn, rec0[u] + tid, tid, 2 * tid, tid, 2 * tid + 1 < L, 2 * tid + 2 < L);
+      __syncthreads();
+    }
+    if (tid == 0) {
+      const Soa<float> zc{zs + zoff(nl), kTopZ};
+      S.base(a.baseR, t, zc, 0);
+      const int64_t so = (s0 + (((int64_t)qb + 1) << a.l0) - 1) * N;
+      put_state<N>(S.y, a.state + so, a.xadd + so, true);
 #pragma unroll
-  for (int c = 0; c < N; ++c) z[c] = zc.at(c, se + 1);
-  float Y[N][N];
-#pragma unroll
-  for (int c = 0; c < N; ++c)
-#pragma unroll
-    for (int r = 0; r < N; ++r) Y[c][r] = a.cr.Y.at(c * N + r, item);
-  float u[N]; /* Y^T y_{2e} is subtracted after Ft^T y_{2e+2} */
-#pragma unroll
-  for (int r = 0; r < N; ++r) u[r] = y[r];
-  if (2 * e + 2 < L) {
-    load(a.cr.R, item + 1, se + 2);
-    solve_t();
-#pragma unroll
-    for (int c = 0; c < N; ++c)
-#pragma unroll
-      for (int r = 0; r < N; ++r) z[c] = fmaf(-a.cr.Ft.at(c * N + r, item + 1), y[r], z[c]);
+      for (int c = 0; c < N; ++c) xs[c * kTopSteps + qb] = S.y[c];
+    }
+  } else if (tid < N) {
+    const int64_t so = (s0 + (((int64_t)qb + 1) << a.l0) - 1) * N;
+    xs[tid * kTopSteps + qb] = ukg_df::f64_to_f32(a.state[so + tid]);
   }
-  const int64_t sn = a.nt.slot[t] + e;
+  __syncthreads();
+  for (int u = nl - 1; u >= 0; --u) {
+    const int L = L0 >> u, d = 1 << u;
+    if (!a.refine) fetch(u - 1, true);
+    if (2 * tid < L) {
+      const TopLevel& V = a.lev[a.l0 + u];
+      const int j = 2 * tid, q = ((j + 1) << u) - 1; /* level l0's step */
+      const int64_t item = rec0[u] + tid;
+      const Soa<float> yc{ys + yoff(u), kTopY};
+      float v[N];
+      bad |= solve_state_step<N>(V.rec, a.refine ? yc : V.rec.rhs, a.refine ? tid : item, item, j > 0, j + 1 < L,
+                                 [&](int k) { return xs[k * kTopSteps + q - d]; },
+                                 [&](int k) { return xs[k * kTopSteps + q + d]; }, v);
 #pragma unroll
-  for (int c = 0; c < N; ++c) {
-#pragma unroll
-    for (int r = 0; r < N; ++r) z[c] = fmaf(-Y[c][r], u[r], z[c]);
-    zn.at(c, sn) = z[c];
+      for (int c = 0; c < N; ++c) xs[c * kTopSteps + q] = v[c];
+      const int64_t so = (s0 + (((int64_t)q + 1) << a.l0) - 1) * N;
+      put_state<N>(v, a.state + so, a.refine ? a.xadd + so : nullptr, !a.refine || a.l0 + u > 0);
+    }
+    __syncthreads();
   }
+  if (bad) atomicOr(a.flag, 2);
 }
 
 struct RegSolves {
   void (*solve)(Args<float, float>) = nullptr;
   void (*rt_level)(Args<float, float>, Soa<float>, Soa<float>, Soa<float>) = nullptr;
+  void (*top)(TopArgs) = nullptr;
 };
 RegSolves reg_solves(int n)
 {
   RegSolves r;
 #define UKG_RS(N_) \
-  case N_: r.solve = solve_state_reg_kernel<N_>, r.rt_level = rt_level_kernel<N_>; break;
+  case N_: r.solve = solve_state_reg_kernel<N_>, r.rt_level = rt_level_kernel<N_>, r.top = top_levels_kernel<N_>; break;
   switch (n) { UKG_RS(2) UKG_RS(3) UKG_RS(4) UKG_RS(5) UKG_RS(6) UKG_RS(7) UKG_RS(8) default: break; }
 #undef UKG_RS
   return r;
@@ -2130,14 +2269,15 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     if (l + 1 < nlev) a.ne = eqT(l + 1);
     const int64_t np = lp[l].npairs, nt = lp[l].ntail;
     if (SK.pair32) { /* n <= 8: lanes or threads per item */
-      if (np > 0) {
-        if (np <= SmallLimits<T>::pair32)
-          UKG_LAUNCH(kPair, st, (SK.pair32<<<grid(np, lw), lt, 0, st>>>(a)));
-        else if (np <= SmallLimits<T>::pair8 || !SK.pair1)
-          UKG_LAUNCH(kPair, st, (SK.pair8<<<grid(np, 4 * lw), lt, 0, st>>>(a)));
-        else
-          UKG_LAUNCH(kPair, st, (SK.pair1<<<grid(np, SK.pair_bs), SK.pair_bs, 0, st>>>(a)));
+      if (np <= SmallLimits<T>::pair32) { /* with the tails */
+        if (np + nt > 0)
+          UKG_LAUNCH(kPair, st, (SK.pair32<<<grid(np + nt, lw), lt, 0, st>>>(a)));
+        continue;
       }
+      if (np <= SmallLimits<T>::pair8 || !SK.pair1)
+        UKG_LAUNCH(kPair, st, (SK.pair8<<<grid(np, 4 * lw), lt, 0, st>>>(a)));
+      else
+        UKG_LAUNCH(kPair, st, (SK.pair1<<<grid(np, SK.pair_bs), SK.pair_bs, 0, st>>>(a)));
       if (nt > 0) UKG_LAUNCH(kTail, st, (SK.tail<<<grid(nt, lw), lt, 0, st>>>(a)));
       continue;
     }
@@ -2146,8 +2286,33 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
       UKG_LAUNCH(kTail, st, (tail_kernel<T, T><<<grid(nt, bt), bt, bt * pt_tail, st>>>(a)));
     }
   }
+  /* Few tracks: the levels from `top` on, of at most kTopSteps steps a track,
+     are one launch (1,000 steps of 6 states: 20 launches of 5 to 8 us become one
+     of 15); many tracks fill the chip level by level.                       */
+  int top = nlev;
+  TopArgs ta;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (RS.top && !want_cov && T_ <= kTopTracks && nlev <= 32) {
+      int64_t kmax = 0;
+      for (int t = 0; t < T_; ++t) kmax = std::max<int64_t>(kmax, p->track_start[t + 1] - p->track_start[t]);
+      for (top = 0; (kmax >> top) > kTopSteps;) ++top;
+      memset(&ta, 0, sizeof(ta));
+      ta.l0 = top;
+      ta.track_start = dtab + P.off_ts;
+      ta.baseR = baseR;
+      ta.flag = dflag;
+      for (int l = top; l < nlev; ++l) {
+        const Tables tb = tables(l);
+        ta.lev[l] = TopLevel{tb.slot, tb.solve, rec(l)};
+      }
+      if (P.refine) ta.z = Soa<float>{(float*)(B + P.o_z[top]), std::max<int64_t>(lp[top].S, 1)};
+      ukg_allow_dynamic_smem((const void*)RS.top);
+      ta.state = p->state;
+      if (top + 1 < nlev) UKG_LAUNCH(kSolve, st, (RS.top<<<(unsigned)T_, kTopThreads, top_smem(n), st>>>(ta)));
+    }
+  }
   /* ---- back-substitution ---- */
-  for (int l = nlev - 2; l >= 0; --l) {
+  for (int l = std::min(nlev - 1, top) - 1; l >= 0; --l) {
     Args<T, T> a;
     memset(&a, 0, sizeof(a));
     common(a, l);
@@ -2194,7 +2359,7 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
                      (atr_kernel<<<grid(p->nsteps, 128), 128, 0, st>>>(r, raw, wE, zp, z0, p->nsteps)));
         }
       }
-      for (int l = 0; l < nlev; ++l) {
+      for (int l = 0; l < std::min(nlev, top); ++l) {
         Args<float, float> a;
         memset(&a, 0, sizeof(a));
         common(a, l);
@@ -2219,7 +2384,13 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
           UKG_LAUNCH(UKG_K_RT, st, (rt_base_kernel<<<grid(lp[l].ntail, 128), 128, 0, st>>>(a, zc, tmp)));
         }
       }
-      for (int l = nlev - 2; l >= 0; --l) {
+      if (top < nlev) {
+        ta.refine = true;
+        ta.state = dx;
+        ta.xadd = p->state;
+        UKG_LAUNCH(UKG_K_RT, st, (RS.top<<<(unsigned)T_, kTopThreads, top_smem(n), st>>>(ta)));
+      }
+      for (int l = std::min(nlev - 1, top) - 1; l >= 0; --l) {
         Args<float, float> a;
         memset(&a, 0, sizeof(a));
         common(a, l);

@@ -66,11 +66,150 @@ __device__ __forceinline__ void store_col(const Soa<T>& first, int e, int64_t s,
 }
 
 /* ---------------------------------------------------------------------------
+ * odd-length tracks, one warp each: the single last step s (observation QR,
+ * then [H_s F_s c_s; R~ 0 o']) and the fix-up of the next level's last
+ * observation, or the one-step base case.
+ * ------------------------------------------------------------------------ */
+template <typename T, int N>
+__device__ __forceinline__ void tail_item(const Args<T, T>& a, int tr, T* hb, int lane)
+{
+  using K = Col<N>;
+  const unsigned gm = 0xffffffffu;
+  const Soa<T>&C = a.ce.F, &Nx = a.ne.F, &Rr = a.cr.R;
+  const int64_t L = a.ct.L[tr], sb = a.ct.slot[tr];
+  const int64_t s = sb + L - 1; /* the last step (the only one if L == 1) */
+  const int ms = a.ce.m[s], mt = ms; /* m <= mx == N */
+  T t[1][N], b[1][N];
+  /* [G_s | o_s] on lanes 0..N; from level 1 on it is triangular already */
+  load_col<T, N>(C, lane < N ? K::G + lane * N : K::o, s, lane <= N, t[0]);
+  T q[N];
+  load_col<T, N>(C, lane < N ? K::H + lane * N : lane == N ? K::c : K::F + (lane - N - 1) * N, s,
+                 L > 1 && lane <= 2 * N, q);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    b[0][i] = T(0);
+    if (i >= ms) t[0][i] = T(0);
+  }
+  if (a.level == 0) lanes_qr_full<T, N, 32, 1, N>(t, b, gm, lane, 0, mt);
+
+  if (L == 1) { /* base case: x = R^{-1} Q^T o, S = R^{-1} R^{-T} */
+    const int64_t os = orig_step(a.track_start, a.level, tr, 0);
+    double* x = a.state + os * N;
+    double* Sg = a.cov ? a.cov + os * (int64_t)N * N : nullptr;
+    if (ms < N) {
+      if (lane < N) x[lane] = NAN;
+      if (Sg)
+        for (int e = lane; e < N * N; e += 32) Sg[e] = NAN;
+      if (lane == 0) atomicOr(a.flag, 2);
+      return;
+    }
+    if (lane < N) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) hb[lane * N + i] = i <= lane ? t[0][i] : T(0);
+    }
+    if (lane < N && a.baseR.p)
+#pragma unroll
+      for (int i = 0; i < N; ++i) a.baseR.at(lane * N + i, tr) = i <= lane ? t[0][i] : T(0);
+    __syncwarp();
+    T dg = T(1);
+    if (lane < N) dg = hb[lane * N + lane];
+    if (lane < N && dg == T(0)) atomicOr(a.flag, 2);
+    const T dv = recip(dg);
+    /* R x = y on lane N, R r = e_q on lanes q < N */
+    T v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = lane == N ? t[0][i] : i == lane ? T(1) : T(0);
+#pragma unroll
+    for (int j = N - 1; j >= 0; --j) {
+      v[j] = v[j] * shfl(gm, dv, j, 32);
+#pragma unroll
+      for (int i = 0; i < j; ++i) v[i] = fma(-v[j], hb[j * N + i], v[i]);
+    }
+    if (lane == N)
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] = ukg_df::widen(v[i]);
+    if (Sg) {
+      __syncwarp();
+      if (lane < N)
+#pragma unroll
+        for (int i = 0; i < N; ++i) hb[lane * N + i] = v[i];
+      __syncwarp();
+      for (int e = lane; e < N * N; e += 32) {
+        const int j = e / N, i = e - j * N;
+        T sm = T(0);
+        for (int k = i > j ? i : j; k < N; ++k) sm = fma(hb[k * N + i], hb[k * N + j], sm);
+        Sg[e] = ukg_df::widen(sm);
+      }
+    }
+    return;
+  }
+
+  const int64_t es = a.ct.solve[tr] + (L - 1) / 2;
+  const int64_t sn = a.nt.slot[tr] + L / 2 - 1;
+  const bool tri = mt == N; /* R~ is triangular after its QR at every level */
+  /* [H_s | c_s | F_s; R~ | o' | 0]: pivots on lanes 0..N-1, the right-hand
+     side on N, F_s on N+1..2N; R~ on top when it has all n rows */
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const T r = lane <= N && i <= lane && i < mt ? t[0][i] : T(0);
+    t[0][i] = tri ? r : q[i];
+    b[0][i] = tri ? q[i] : r;
+  }
+  if (tri) lanes_qr_tri<T, N, 32, 1>(t, b, gm, lane, 0, N);
+  else lanes_qr_full<T, N, 32, 1, N>(t, b, gm, lane, 0, N);
+  T zero[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    zero[i] = T(0);
+    if (lane < N && i > lane) t[0][i] = T(0);
+    if (lane >= N && lane <= 2 * N) hb[(lane == N ? N : lane - N - 1) * N + i] = b[0][i];
+  }
+  store_col<T, N>(Rr, lane < N ? K::R + lane * N : lane == N ? K::rhs : K::Ft + (lane - N - 1) * N, es,
+                  lane <= 2 * N ? N : 0, t[0]);
+  store_col<T, N>(Rr, K::Y + lane * N, es, lane < N ? N : 0, zero);
+  __syncwarp();
+  /* fix-up: [G~ | o; Z | o''], mt rows of Z; stacked without a gap unless both are full */
+  const int gp = a.ne.m[sn], rF = gp + mt, nF = rF < N ? rF : N;
+  const bool triF = tri && gp == N;
+  const int eg = lane < N ? K::G + lane * N : K::o;
+  const T* g = Nx.p + (int64_t)eg * Nx.stride + sn;
+#pragma unroll
+  for (int r = 0; r < 2 * N; ++r) {
+    T v = T(0);
+    if (lane <= N && r < gp) v = g[r * Nx.stride];
+    else if (lane <= N && r < rF) v = hb[lane * N + r - gp];
+    (r < N ? t[0][r] : b[0][r - N]) = v;
+  }
+  __syncwarp();
+  if (triF) lanes_qr_tri<T, N, 32, 1>(t, b, gm, lane, 0, N);
+  else lanes_qr_full<T, N, 32, 1, N>(t, b, gm, lane, 0, nF);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (lane < N && i > lane) t[0][i] = T(0);
+  store_col<T, N>(Nx, eg, sn, lane <= N ? nF : 0, t[0]);
+  if (lane == 0) a.ne.m[sn] = nF;
+}
+
+__host__ __device__ constexpr int tail_entries(int n) { return (2 * n + 1) * n; } /* tail_item's shared memory */
+
+template <typename T, int N>
+__global__ void __launch_bounds__(32 * kLaneWarps) tail_lanes(Args<T, T> a)
+{
+  __shared__ T buf[kLaneWarps][tail_entries(N)];
+  const int w = threadIdx.x >> 5;
+  const int64_t item = (int64_t)blockIdx.x * kLaneWarps + w;
+  if (item < a.ct.ntail) tail_item<T, N>(a, (int)a.ct.tail[item], buf[w], threadIdx.x & 31); /* the whole warp */
+}
+
+/* ---------------------------------------------------------------------------
  * forward elimination of a pair (j, j+1) by a group of LPI lanes.
  * Stage A's columns: 0..N-1 pivots, N right-hand side, N+1..2N H_{j+1};
  * stage B's: the same with Y~ in place of H, then 2N+1..3N F_j; stage C's:
  * 0..N-1 pivots, N right-hand side -- with LPI = 32 and N <= 7 on the lanes
  * 3N+1..4N+1 at the same time as stage B.
+ * With 32 lanes the level's tails are part of the launch: the warp of an odd
+ * track's last pair goes on to the fix-up, and the warps past the pairs take
+ * the tracks that have one step left.
  * ------------------------------------------------------------------------ */
 template <typename T, int N, int LPI>
 __global__ void __launch_bounds__(32 * kLaneWarps) pair_lanes(Args<T, T> a)
@@ -79,11 +218,19 @@ __global__ void __launch_bounds__(32 * kLaneWarps) pair_lanes(Args<T, T> a)
   constexpr int S = (3 * N + 1 + LPI - 1) / LPI, SC = (N + 1 + LPI - 1) / LPI;
   constexpr bool kMerge = LPI == 32 && 4 * N + 2 <= 32;
   constexpr int GPB = 32 * kLaneWarps / LPI; /* groups per block */
-  __shared__ T hbuf[GPB][(N + 1) * N];       /* H~ and o~ of the group's item: column q's rows at q * N */
+  /* H~ and o~ of the group's item: column q's rows at q * N */
+  __shared__ T hbuf[GPB][LPI == 32 ? tail_entries(N) : (N + 1) * N];
   const int grp = threadIdx.x / LPI, lane = threadIdx.x % LPI;
   const unsigned gm = LPI == 32 ? 0xffffffffu : ((1u << (LPI & 31)) - 1u) << ((threadIdx.x & 31) / LPI * LPI);
   const int64_t item = (int64_t)blockIdx.x * GPB + grp;
-  if (item >= a.ct.npairs) return; /* the whole group */
+  T* hb = hbuf[grp];
+  if (item >= a.ct.npairs) { /* the whole group */
+    if (LPI == 32 && item - a.ct.npairs < a.ct.ntail) {
+      const int tr = (int)a.ct.tail[item - a.ct.npairs];
+      if (a.ct.L[tr] == 1) tail_item<T, N>(a, tr, hb, lane);
+    }
+    return;
+  }
   const Soa<T>&C = a.ce.F, &Nx = a.ne.F, &Rr = a.cr.R;
   const int tr = find_track(a.ct.pair, a.ntracks, item);
   const int64_t p = item - a.ct.pair[tr];
@@ -91,7 +238,6 @@ __global__ void __launch_bounds__(32 * kLaneWarps) pair_lanes(Args<T, T> a)
   const int64_t sn = a.nt.slot[tr] + p;
   const int64_t se = a.ct.solve[tr] + p;
   const int mj = a.ce.m[sj], mj1 = a.ce.m[sj1];
-  T* hb = hbuf[grp];
 
   /* everything the pair reads is on its way before the first reflector: the
      rows of G_j, those of F_{j+1} with H_{j+1}, stage B's lower rows
@@ -218,137 +364,13 @@ __global__ void __launch_bounds__(32 * kLaneWarps) pair_lanes(Args<T, T> a)
     store_col<T, N>(Rr, er, se, c <= 3 * N ? N : 0, t[s]);
     store_col<T, N>(Nx, en, sn, p > 0 && c >= N && c <= 3 * N ? N : 0, b[s]);
   }
-}
-
-/* ---------------------------------------------------------------------------
- * odd-length tracks, one warp each: the single last step s (observation QR,
- * then [H_s F_s c_s; R~ 0 o']) and the fix-up of the next level's last
- * observation, or the one-step base case.
- * ------------------------------------------------------------------------ */
-template <typename T, int N>
-__global__ void __launch_bounds__(32 * kLaneWarps) tail_lanes(Args<T, T> a)
-{
-  __shared__ T buf[kLaneWarps][(2 * N + 1) * N];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t item = (int64_t)blockIdx.x * kLaneWarps + w;
-  if (item >= a.ct.ntail) return; /* the whole warp */
-  using K = Col<N>;
-  const unsigned gm = 0xffffffffu;
-  const Soa<T>&C = a.ce.F, &Nx = a.ne.F, &Rr = a.cr.R;
-  T* hb = buf[w];
-  const int tr = (int)a.ct.tail[item];
-  const int64_t L = a.ct.L[tr], sb = a.ct.slot[tr];
-  const int64_t s = sb + L - 1; /* the last step (the only one if L == 1) */
-  const int ms = a.ce.m[s], mt = ms; /* m <= mx == N */
-  T t[1][N], b[1][N];
-  /* [G_s | o_s] on lanes 0..N; from level 1 on it is triangular already */
-  load_col<T, N>(C, lane < N ? K::G + lane * N : K::o, s, lane <= N, t[0]);
-  T q[N];
-  load_col<T, N>(C, lane < N ? K::H + lane * N : lane == N ? K::c : K::F + (lane - N - 1) * N, s,
-                 L > 1 && lane <= 2 * N, q);
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    b[0][i] = T(0);
-    if (i >= ms) t[0][i] = T(0);
-  }
-  if (a.level == 0) lanes_qr_full<T, N, 32, 1, N>(t, b, gm, lane, 0, mt);
-
-  if (L == 1) { /* base case: x = R^{-1} Q^T o, S = R^{-1} R^{-T} */
-    const int64_t os = orig_step(a.track_start, a.level, tr, 0);
-    double* x = a.state + os * N;
-    double* Sg = a.cov ? a.cov + os * (int64_t)N * N : nullptr;
-    if (ms < N) {
-      if (lane < N) x[lane] = NAN;
-      if (Sg)
-        for (int e = lane; e < N * N; e += 32) Sg[e] = NAN;
-      if (lane == 0) atomicOr(a.flag, 2);
-      return;
+  if constexpr (LPI == 32) {
+    const int64_t L = a.ct.L[tr];
+    if ((L & 1) && 2 * p + 3 == L) {
+      __syncwarp(); /* the next level's slot is this warp's own */
+      tail_item<T, N>(a, tr, hb, lane);
     }
-    if (lane < N) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) hb[lane * N + i] = i <= lane ? t[0][i] : T(0);
-    }
-    if (lane < N && a.baseR.p)
-#pragma unroll
-      for (int i = 0; i < N; ++i) a.baseR.at(lane * N + i, tr) = i <= lane ? t[0][i] : T(0);
-    __syncwarp();
-    T dg = T(1);
-    if (lane < N) dg = hb[lane * N + lane];
-    if (lane < N && dg == T(0)) atomicOr(a.flag, 2);
-    const T dv = recip(dg);
-    /* R x = y on lane N, R r = e_q on lanes q < N */
-    T v[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = lane == N ? t[0][i] : i == lane ? T(1) : T(0);
-#pragma unroll
-    for (int j = N - 1; j >= 0; --j) {
-      v[j] = v[j] * shfl(gm, dv, j, 32);
-#pragma unroll
-      for (int i = 0; i < j; ++i) v[i] = fma(-v[j], hb[j * N + i], v[i]);
-    }
-    if (lane == N)
-#pragma unroll
-      for (int i = 0; i < N; ++i) x[i] = ukg_df::widen(v[i]);
-    if (Sg) {
-      __syncwarp();
-      if (lane < N)
-#pragma unroll
-        for (int i = 0; i < N; ++i) hb[lane * N + i] = v[i];
-      __syncwarp();
-      for (int e = lane; e < N * N; e += 32) {
-        const int j = e / N, i = e - j * N;
-        T sm = T(0);
-        for (int k = i > j ? i : j; k < N; ++k) sm = fma(hb[k * N + i], hb[k * N + j], sm);
-        Sg[e] = ukg_df::widen(sm);
-      }
-    }
-    return;
   }
-
-  const int64_t es = a.ct.solve[tr] + (L - 1) / 2;
-  const int64_t sn = a.nt.slot[tr] + L / 2 - 1;
-  const bool tri = mt == N; /* R~ is triangular after its QR at every level */
-  /* [H_s | c_s | F_s; R~ | o' | 0]: pivots on lanes 0..N-1, the right-hand
-     side on N, F_s on N+1..2N; R~ on top when it has all n rows */
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const T r = lane <= N && i <= lane && i < mt ? t[0][i] : T(0);
-    t[0][i] = tri ? r : q[i];
-    b[0][i] = tri ? q[i] : r;
-  }
-  if (tri) lanes_qr_tri<T, N, 32, 1>(t, b, gm, lane, 0, N);
-  else lanes_qr_full<T, N, 32, 1, N>(t, b, gm, lane, 0, N);
-  T zero[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    zero[i] = T(0);
-    if (lane < N && i > lane) t[0][i] = T(0);
-    if (lane >= N && lane <= 2 * N) hb[(lane == N ? N : lane - N - 1) * N + i] = b[0][i];
-  }
-  store_col<T, N>(Rr, lane < N ? K::R + lane * N : lane == N ? K::rhs : K::Ft + (lane - N - 1) * N, es,
-                  lane <= 2 * N ? N : 0, t[0]);
-  store_col<T, N>(Rr, K::Y + lane * N, es, lane < N ? N : 0, zero);
-  __syncwarp();
-  /* fix-up: [G~ | o; Z | o''], mt rows of Z; stacked without a gap unless both are full */
-  const int gp = a.ne.m[sn], rF = gp + mt, nF = rF < N ? rF : N;
-  const bool triF = tri && gp == N;
-  const int eg = lane < N ? K::G + lane * N : K::o;
-  const T* g = Nx.p + (int64_t)eg * Nx.stride + sn;
-#pragma unroll
-  for (int r = 0; r < 2 * N; ++r) {
-    T v = T(0);
-    if (lane <= N && r < gp) v = g[r * Nx.stride];
-    else if (lane <= N && r < rF) v = hb[lane * N + r - gp];
-    (r < N ? t[0][r] : b[0][r - N]) = v;
-  }
-  __syncwarp();
-  if (triF) lanes_qr_tri<T, N, 32, 1>(t, b, gm, lane, 0, N);
-  else lanes_qr_full<T, N, 32, 1, N>(t, b, gm, lane, 0, nF);
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    if (lane < N && i > lane) t[0][i] = T(0);
-  store_col<T, N>(Nx, eg, sn, lane <= N ? nF : 0, t[0]);
-  if (lane == 0) a.ne.m[sn] = nF;
 }
 
 /* ---------------------------------------------------------------------------
