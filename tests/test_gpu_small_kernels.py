@@ -54,3 +54,20 @@ def test_unobservable_is_reported(k):
         with pytest.raises(native.KalmanError) as e:
             native.smooth(P, "oddeven", fp32_refine=df)
         assert e.value.status == native.KALMAN_GPU_ESINGULAR
+
+
+@pytest.mark.parametrize("n,k", [(2, 1023), (3, 1), (4, 1025), (6, 2047), (6, 2), (7, 1024), (8, 2500)])
+@pytest.mark.parametrize("sweeps", [1, 2])
+def test_upper_levels_in_one_launch(n, k, sweeps):
+    """The precision form takes the levels of at most 1,024 steps a track in
+    one launch for up to 304 tracks, and level by level above: the same bits."""
+    P = pb.random_dynamics([k], n, n, seed=n + k, K_type="C", C_type="C")
+    st, Xo, _ = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, _ = native.smooth(P, "oddeven", covariance=False, fp32_refine=True, sweeps=sweeps)
+    if sweeps == 2:
+        assert oracle.rel_err_states(X, Xo) < 1e-9
+    for T in (304, 305):
+        Xb, _ = native.smooth(P.select_tracks([0] * T), "oddeven", covariance=False, fp32_refine=True, sweeps=sweeps)
+        for t in (0, T - 1):
+            np.testing.assert_array_equal(Xb[k * t:k * t + k], X, err_msg=f"{T} tracks")

@@ -1662,11 +1662,12 @@ __global__ void __launch_bounds__(128) rt_level_kernel(Args<float, float> a, Soa
  * transpose solves up to the base, then (always) the back-substitution down to
  * l0.  For few tracks, whose upper levels are a launch of a block or two each.
  * What one level leaves for the next (z, y, states or corrections) stays in
- * shared memory, and a level's factors are brought into L1 while the one before
- * runs, so a level is a barrier and a short chain instead of 5 to 7 us.       */
+ * shared memory.  A chain of loads and of 2 n dependent steps a level bounds it:
+ * 2 to 2.5 us each, instead of 5 to 8 for a launch.  (Prefetching the next
+ * level's factors into L1 made a window of 1,000 steps 20 us slower.)         */
 constexpr int kTopThreads = 512;
 constexpr int kTopSteps = 1024; /* a track's steps at level l0 at most: an even step per thread */
-constexpr int kTopTracks = 304; /* two blocks on each of 152 SMs */
+constexpr int kTopTracks = 304; /* two blocks on each of 152 SMs, by threads; one from n = 7 on, by shared memory */
 struct TopLevel {
   const int64_t *slot, *solve;
   Rec<float> rec;
@@ -1685,8 +1686,6 @@ struct TopArgs {
 constexpr int kTopZ = 2 * kTopSteps + 32, kTopY = kTopSteps + 32;
 constexpr size_t top_smem(int n) { return (size_t)n * (kTopZ + kTopY + kTopSteps) * sizeof(float); }
 
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-
 template <int N>
 __global__ void __launch_bounds__(kTopThreads) top_levels_kernel(const __grid_constant__ TopArgs a)
 {
@@ -1703,19 +1702,6 @@ __global__ void __launch_bounds__(kTopThreads) top_levels_kernel(const __grid_co
   float* ys = zs + N * kTopZ;
   float* xs = ys + N * kTopY; /* entry c of level l0's step q: xs[c * kTopSteps + q] */
   __syncthreads();
-  auto fetch = [&](int u, bool next) { /* level u's factors for this thread's even step */
-    if (u >= nl || u < 0 || 2 * tid >= (L0 >> u)) return;
-    const Rec<float>& V = a.lev[a.l0 + u].rec;
-    const int64_t item = rec0[u] + tid;
-    if (tid & 7) return; /* a 32-byte sector holds eight records of an entry */
-    for (int e = 0; e < N * N; ++e) {
-      prefetch_l1(&V.R.at(e, item));
-      prefetch_l1(&V.Y.at(e, item));
-      prefetch_l1(&V.Ft.at(e, item));
-    }
-    if (next)
-      for (int e = 0; e < N; ++e) prefetch_l1(&V.rhs.at(e, item));
-  };
   auto zoff = [&](int u) { int o = 0; for (int v = 0; v < u; ++v) o += (L0 >> v) + 1; return o; };
   auto yoff = [&](int u) { int o = 0; for (int v = 0; v < u; ++v) o += ((L0 >> v) + 1) / 2; return o; };
   const int qb = (1 << nl) - 1; /* the base's step */
@@ -1728,7 +1714,6 @@ __global__ void __launch_bounds__(kTopThreads) top_levels_kernel(const __grid_co
     __syncthreads();
     for (int u = 0; u < nl; ++u) {
       const int L = L0 >> u;
-      fetch(u + 1, false);
       const Soa<float> zc{zs + zoff(u), kTopZ}, zn{zs + zoff(u + 1), kTopZ}, yc{ys + yoff(u), kTopY};
       if (2 * tid < L)
         S.even(a.lev[a.l0 + u].rec, zc, yc, zn, rec0[u] + tid, tid, 2 * tid, tid, 2 * tid + 1 < L, 2 * tid + 2 < L);
@@ -1749,7 +1734,6 @@ __global__ void __launch_bounds__(kTopThreads) top_levels_kernel(const __grid_co
   __syncthreads();
   for (int u = nl - 1; u >= 0; --u) {
     const int L = L0 >> u, d = 1 << u;
-    if (!a.refine) fetch(u - 1, true);
     if (2 * tid < L) {
       const TopLevel& V = a.lev[a.l0 + u];
       const int j = 2 * tid, q = ((j + 1) << u) - 1; /* level l0's step */
@@ -2287,8 +2271,11 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     }
   }
   /* Few tracks: the levels from `top` on, of at most kTopSteps steps a track,
-     are one launch (1,000 steps of 6 states: 20 launches of 5 to 8 us become one
-     of 15); many tracks fill the chip level by level.                       */
+     are one launch; many tracks fill the chip level by level.  6 states, 1,000
+     steps, the solves and one or two sweeps: one track 314 us level by level, 260
+     so (all of a call by plan); about 300 tracks (304 in one launch, 310 level
+     by level), back-substitution 0.12 ms level by level, 0.07 so, two sweeps
+     0.51 and 0.27.                                                          */
   int top = nlev;
   TopArgs ta;
   if constexpr (sizeof(T) == sizeof(float)) {
