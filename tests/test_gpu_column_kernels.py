@@ -56,3 +56,18 @@ def test_associative_register_sizes(n, m, cov):
     assert st == 0
     X, S = native.smooth(P, "associative")
     assert oracle.rel_err_states(X, Xo) < 1e-11 and oracle.rel_err_covs(S, So) < 1e-11
+
+
+@pytest.mark.parametrize("n,m,cov", [(97, 97, "C"), (99, 1, "w"), (100, 40, "W"), (113, 112, "C"), (127, 20, "F"),
+                                     (128, 128, "C"), (128, 64, "W"), (120, 128, "C")])
+def test_two_pass_sizes(n, m, cov):
+    """97 to 128 states in the precision form: pivots first, the other columns after."""
+    P = pb.random_dynamics([1, 2, 7, 12, 13], n, m, seed=n + m, K_type=cov, C_type=cov, missing=0.3, per_step=True)
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, S = native.smooth(P, "oddeven", fp32_refine=True)
+    assert oracle.rel_err_states(X, Xo) < 1e-9 and oracle.rel_err_covs(S, So) < 1e-9
+    X, _ = native.smooth(P, "oddeven", covariance=False, fp32_refine=True, sweeps=3)
+    assert oracle.rel_err_states(X, Xo) < 1e-9
+    X, _ = native.smooth(P, "oddeven", covariance=False)
+    assert oracle.rel_err_states(X, Xo) < 1e-11

@@ -1777,6 +1777,7 @@ __global__ void add_kernel(double* x, const double* d, int64_t count)
 #include "oddeven_cta.cuh"
 #include "oddeven_small.cuh"
 #include "oddeven_cols.cuh"
+#include "oddeven_wide.cuh"
 
 /* ---------------------------------------------------------------------------
  * host side: plan, workspace, launches
@@ -2608,6 +2609,12 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     ukg_allow_dynamic_smem((const void*)CK.tail);
     if (CK.solve) ukg_allow_dynamic_smem((const void*)CK.solve);
   }
+  const wide::Kernels WK = sizeof(T) == sizeof(float) ? wide::kernels(n, mx) : wide::Kernels();
+  if (WK.pair) {
+    ukg_allow_dynamic_smem((const void*)WK.triangularize);
+    ukg_allow_dynamic_smem((const void*)WK.pair);
+    ukg_allow_dynamic_smem((const void*)WK.tail);
+  }
   const ctak::RawA raw{p->H, p->F, p->c, p->K, p->G, p->o, p->C, p->K_type, p->C_type, p->obs_rows, p->mmax};
   {
     ctak::CArgs<T> a;
@@ -2626,6 +2633,9 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     } else {
       UKG_LAUNCH(kWeigh, st, (ctak::weigh_cta<T><<<grid(p->nsteps), cta::NT, 0, st>>>(a, raw, p->nsteps)));
     }
+    if constexpr (sizeof(T) == sizeof(float))
+      if (WK.pair)
+        UKG_LAUNCH(kWeigh, st, (WK.triangularize<<<(unsigned)((p->nsteps + 1) / 2), wide::NT, WK.smem, st>>>(a, p->nsteps)));
   }
   const int kPair = P.fp32 ? UKG_K_PAIR32 : kDD ? UKG_K_DF_PAIR : UKG_K_PAIR;
   const int kSolve = P.fp32 ? UKG_K_SOLVE32 : kDD ? UKG_K_DF_SOLVE : UKG_K_SOLVE;
@@ -2634,6 +2644,14 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     common(a, l);
     a.ce = eq_level(l);
     if (l + 1 < nlev) a.ne = eq_level(l + 1);
+    if constexpr (sizeof(T) == sizeof(float))
+      if (WK.pair) {
+        if (lp[l].npairs > 0)
+          UKG_LAUNCH(kPair, st, (WK.pair<<<(unsigned)lp[l].npairs, wide::NT, WK.smem, st>>>(a)));
+        if (lp[l].ntail > 0)
+          UKG_LAUNCH(kTail, st, (WK.tail<<<(unsigned)lp[l].ntail, wide::NT, WK.smem, st>>>(a)));
+        continue;
+      }
     if (CK.pair) {
       if (lp[l].npairs > 0)
         UKG_LAUNCH(kPair, st, (CK.pair<<<(unsigned)lp[l].npairs, CK.threads, ck_pair, st>>>(a)));

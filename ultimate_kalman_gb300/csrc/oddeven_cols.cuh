@@ -1,8 +1,7 @@
 /*
- * oddeven_cols.cuh -- the odd-even smoother for 9 to 64 states (to 96 in
- * FP32), no more observation rows than states: one thread block per work item,
- * one thread per matrix column, the column's rows in registers.  Included by
- * oddeven.cu.
+ * oddeven_cols.cuh -- the odd-even smoother for 9 to 64 states, no more
+ * observation rows than states: one thread block per work item, one thread per
+ * matrix column, the column's rows in registers.  Included by oddeven.cu.
  *
  * The block-per-item kernels of oddeven_cta.cuh keep their panels in global
  * scratch: every reflector reads each column twice and writes it once through
@@ -15,7 +14,7 @@
  *   16 tracks of 64 to 4,000 steps, n = 12  FP64   7.2 2.0 1.5    2.2 1.1 0.7
  *   2,000 steps, n = 48                     FP64   22.7 8.4 1.6   12.0 6.3 2.2
  *                                           df     16.6 9.9 1.0   5.7 6.6 1.8
- *   4,000 steps, n = 64, states             FP32   8.9 1.0 1.5    5.7 0.5 3.4
+ *   4,000 steps, n = 64, states             FP32   8.9 1.0 1.5    4.2 0.5 3.2
  * (the weighing now includes the triangularization).
  *
  * Structure.  Every observation block is upper trapezoidal: the weighing
@@ -64,6 +63,11 @@ __host__ __device__ constexpr int blocks3()
                         : (NP <= 12 ? 12 : NP <= 16 ? 12 : NP <= 24 ? 6 : NP <= 32 ? 4 : NP <= 64 ? 2 : 1);
 }
 
+/* the fewest states an instantiation is used for; rows below it need no test
+ * (a test every few rows keeps the reads of x from running ahead)             */
+template <int NP>
+__host__ __device__ constexpr int least() { return NP <= 16 ? NP - 3 : NP <= 24 ? 17 : NP <= 32 ? 25 : NP <= 48 ? 33 : 49; }
+
 template <typename T, int NP>
 struct QrShared {
   T x[2][2][NP];       /* [step parity][panel]: the pivot column's rows below */
@@ -86,7 +90,7 @@ __device__ __forceinline__ T step(QrShared<T, NP>& sm, int k, int panel, bool on
   T d0 = T(0), d1 = T(0);
 #pragma unroll
   for (int i = 0; i < NP; i += 4)
-    if (i < n) { /* rows past n are zero; the same in every thread */
+    if (i < least<NP>() || i < n) { /* rows past n are zero; the same in every thread */
       d0 = fma(x[i], b[i], d0);
       d1 = fma(x[i + 1], b[i + 1], d1);
       d0 = fma(x[i + 2], b[i + 2], d0);
@@ -110,7 +114,7 @@ __device__ __forceinline__ T step(QrShared<T, NP>& sm, int k, int panel, bool on
   const T d = fma(amb, tk, dot) * inv;
 #pragma unroll
   for (int i = 0; i < NP; i += 4)
-    if (i < n) {
+    if (i < least<NP>() || i < n) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) b[i + u] = fma(-d, x[i + u], b[i + u]);
     }
@@ -775,9 +779,9 @@ Kernels<T> kernels(int n, int mx)
   if (n <= 32) return kernels_np<T, 32>();
   if (n <= 48) return kernels_np<T, 48>();
   if (n <= 64) return kernels_np<T, 64>();
-  if constexpr (sizeof(T) == sizeof(float))
-    if (n <= 96) return kernels_np<T, 96>();
-  return Kernels<T>();
+  Kernels<T> k; /* above, the states' back-substitution alone */
+  k.state = state_cols<T, 128>;
+  return k;
 }
 
 }  // namespace cols
