@@ -9,6 +9,8 @@
 #pragma once
 #include <cstdint>
 
+#include "lanes.cuh"
+
 namespace cta {
 
 constexpr int NT = 128; /* threads per CTA; rows of a panel beyond NT are looped */
@@ -370,27 +372,34 @@ static __device__ bool cholesky_cm(T* L, int rows)
 {
   __shared__ T Ps[kChNB][kMaxCov];
   __shared__ int bad_c;
+  __shared__ T inv_c;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) bad_c = 0;
   for (int j0 = 0; j0 < rows; j0 += kChNB) {
     const int nb = rows - j0 < kChNB ? rows - j0 : kChNB;
     for (int jj = warp; jj < kChNB; jj += NT / 32)
       for (int i = j0 + lane; i < rows; i += 32) Ps[jj][i] = jj < nb ? L[(int64_t)(j0 + jj) * rows + i] : T(0);
+    /* column jj's root, by the thread that updates its diagonal entry last:
+       two barriers a column, and no division by the root                     */
+    auto root = [&](int jj) {
+      const T d = Ps[jj][j0 + jj];
+      const bool ok = d > T(0);
+      if (!ok) bad_c = 1;
+      inv_c = ok ? lanes::inv_root(d) : T(1);
+      Ps[jj][j0 + jj] = !ok ? T(1) : inv_c == T(0) ? sqrt(d) : d * inv_c; /* an infinite variance stays one */
+    };
+    __syncthreads();
+    if (tid == 0) root(0);
     __syncthreads();
     for (int jj = 0; jj < nb; ++jj) {
       const int j = j0 + jj;
-      if (tid == 0) {
-        const T d = Ps[jj][j];
-        if (!(d > T(0))) bad_c = 1;
-        Ps[jj][j] = d > T(0) ? sqrt(d) : T(1);
-      }
-      __syncthreads();
-      const T ljj = Ps[jj][j];
-      for (int i = j + 1 + tid; i < rows; i += NT) Ps[jj][i] /= ljj;
+      const T inv = inv_c;
+      for (int i = j + 1 + tid; i < rows; i += NT) Ps[jj][i] = Ps[jj][i] * inv;
       __syncthreads();
       for (int kk = jj + 1 + warp; kk < nb; kk += NT / 32) {
         const T mk = Ps[jj][j0 + kk];
         for (int i = j0 + kk + lane; i < rows; i += 32) Ps[kk][i] = fma(-Ps[jj][i], mk, Ps[kk][i]);
+        if (tid == 0 && kk == jj + 1) root(kk);
       }
       __syncthreads();
     }
@@ -479,36 +488,6 @@ static __device__ void forward_subst_cm(const T* L, int rows, T* B, int ldb, int
   int c = threadIdx.x;
   for (; c + NT < cols; c += 2 * NT) fsub_cols<2>(L, rows, B, ldb, c, NT);
   for (; c < cols; c += NT) fsub_cols<1>(L, rows, B, ldb, c, 0);
-  __syncthreads();
-}
-
-/* w <- L^{-1} w (lower = true) or L^{-T} w for the column-major lower
- * triangular L (ld rows) and the CTA-shared vector w; run by warp 0, columns of
- * L read along their length, and followed by a CTA barrier.                 */
-template <typename T>
-static __device__ void tri_solve_vec_cm(const T* L, int rows, T* w, bool lower)
-{
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    if (lower)
-      for (int j = 0; j < rows; ++j) {
-        const T wj = w[j] / L[(int64_t)j * rows + j];
-        __syncwarp();
-        if (lane == 0) w[j] = wj;
-        for (int i = j + 1 + lane; i < rows; i += 32) w[i] = fma(-L[(int64_t)j * rows + i], wj, w[i]);
-        __syncwarp();
-      }
-    else
-      for (int j = rows - 1; j >= 0; --j) {
-        T d = T(0);
-        for (int i = j + 1 + lane; i < rows; i += 32) d = fma(L[(int64_t)j * rows + i], w[i], d);
-        for (int off = 16; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-        const T wj = (w[j] - d) / L[(int64_t)j * rows + j];
-        __syncwarp();
-        if (lane == 0) w[j] = wj;
-        __syncwarp();
-      }
-  }
   __syncthreads();
 }
 

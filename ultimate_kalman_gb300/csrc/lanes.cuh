@@ -43,6 +43,15 @@ __device__ __forceinline__ ukg_df::dd recip(ukg_df::dd d) { return ukg_df::dd(1)
 
 __device__ __forceinline__ float recip(float d) { return 1.0f / d; }
 
+/* 1 / sqrt(s), s > 0 */
+template <typename T>
+__device__ __forceinline__ T inv_root(T s) { return T(1) / sqrt(s); }
+template <>
+__device__ __forceinline__ double inv_root<double>(double s)
+{
+  return series_range(s) ? rsqrt_series(s) : 1.0 / sqrt(s);
+}
+
 /* The reflector that maps (alpha, x) to (beta, 0), tail = x^T x != 0, as
  * H = I - inv u u^T with u = (amb, x): a column (a_k, a) takes
  * d = inv (x^T a + amb a_k), a_k -= d amb, a -= d x.  x stays unscaled.      */

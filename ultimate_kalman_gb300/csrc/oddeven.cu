@@ -18,9 +18,10 @@
  *   solve_kernel     one thread per even step: back-substitution and the
  *                    covariance recurrence (Solve_Estimates 614-975)
  *
- * These are the FP32 kernels and, in FP64 and double-float, those of shapes
- * with more observation rows than states; up to 8 states FP64 and double-float
- * run oddeven_small.cuh, from 9 on every form runs oddeven_cta.cuh.
+ * Except for the weighing these are the kernels of one state, and of up to 8
+ * with more observation rows than states; other shapes of 2 to 8 states run
+ * oddeven_small.cuh, of 9 to 64 oddeven_cols.cuh, of 65 to 128 in FP32
+ * oddeven_wide.cuh, and the rest oddeven_cta.cuh.
  *
  * Every "QR, then apply Q^T" of the reference is a Householder triangularization
  * of the pivot block whose reflectors are then streamed over the other columns
@@ -43,7 +44,8 @@
  * residual run in double-float arithmetic on the FP32 pipe (weigh_df_kernel
  * stores the weighed equations as FP32 high + low parts, residual_df_kernel
  * reads them; df64.cuh); other shapes weigh in FP32 and form the residual in
- * FP64 from the raw equations (residual_kernel, atr_kernel).
+ * FP64 from the raw equations (residual_kernel and atr_kernel, or
+ * ctak::residual_cta).
  *
  * Layout in HBM ("slot" = a step of a level, every track's slots start at an
  * even slot so pairs never straddle tracks):
@@ -2687,45 +2689,30 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     const int requested = (int)((options >> 21) & 3u);
     const int sweeps = P.refine ? (requested ? requested : 2) : 0;
     double* dx = P.refine ? (double*)(B + P.o_dx) : nullptr;
-    auto pargs = [&](int l) { /* for rt_base_kernel and atr_kernel (no level arrays) */
-      Args<float, float> a;
-      memset(&a, 0, sizeof(a));
-      a.ct = tables(l);
-      a.nt = tables(l + 1);
-      a.n = n;
-      a.mx = mx;
-      a.level = l;
-      a.ntracks = T_;
-      a.track_start = dtab + P.off_ts;
-      a.state = dx;
-      a.flag = dflag;
-      a.baseR = baseR;
-      return a;
-    };
-    const RawDev rawd{p->H, p->F, p->c, p->K, p->G, p->o, p->C, p->K_type, p->C_type, p->obs_rows, p->mmax};
-    /* the residual's scratch (a factor and four vectors, FP64) is small: two
-       of its CTAs per slot where they fit */
-    const int64_t rr = std::max(n, p->mmax), rneed = rr * rr + 4 * rr;
+    /* the residual's scratch (a factor, FP64) is small: two of its CTAs per
+       slot where they fit */
+    const int64_t rr = std::max(n, p->mmax), rneed = rr * rr;
+    /* level 0's region holds C's factors if they are no larger than G in FP32
+       (a float more for their alignment)                                   */
+    const int keep = sweeps > 1 ? (2 * (int64_t)p->mmax * p->mmax + 1 <= (int64_t)mx * n ? 3 : 1) : 0;
     const bool r2 = 2 * rneed <= per_cta;
     const int64_t rper = r2 ? per_cta / 2 : per_cta;
     const unsigned rgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(p->nsteps, (r2 ? 2 : 1) * (int64_t)ncta));
     for (int sw = 0; sw < sweeps; ++sw) {
-      Soa<double> wE{(double*)(B + P.o_rE), P.S0}, zp{(double*)(B + P.o_rO), P.S0};
+      Soa<double> zf{(double*)(B + P.o_rE), P.S0}, zp{(double*)(B + P.o_rO), P.S0};
       Soa<float> z0{(float*)(B + P.o_z[0]), std::max<int64_t>(lp[0].S, 1)};
       {
         ctak::CArgs<float> a;
         common(a, 0);
         a.ce = eq_level(0);
         UKG_LAUNCH(UKG_K_RESID, st,
-                   (ctak::residual_cta<<<rgrid, cta::NT, 0, st>>>(a, raw, wE, zp, (double*)scratch, rper,
-                                                                           p->nsteps)));
-        Args<float, float> r = pargs(0);
-        r.state = p->state;
+                   (ctak::residual_cta<<<rgrid, cta::NT, 0, st>>>(a, raw, zf, zp, (double*)scratch, rper,
+                                                                  p->nsteps, keep | (sw > 0 ? 4 : 0))));
         UKG_LAUNCH(UKG_K_RESID, st,
-                   (atr_kernel<<<(unsigned)((p->nsteps + 127) / 128), 128, 0, st>>>(r, rawd, wE, zp, z0, p->nsteps)));
+                   (ctak::next_step_kernel<<<dim3((unsigned)((p->nsteps + 127) / 128), (unsigned)std::min(n, 32)), 128, 0,
+                                             st>>>(a, zf, zp, z0, p->nsteps)));
       }
       for (int l = 0; l < nlev; ++l) {
-        Args<float, float> a = pargs(l);
         ctak::CArgs<float> ca;
         common(ca, l);
         Soa<float> zc{(float*)(B + P.o_z[l]), std::max<int64_t>(lp[l].S, 1)};
@@ -2739,8 +2726,8 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
                      (ctak::rt_odd_aos<<<(unsigned)((lp[l].npairs * 32 + 127) / 128), 128, 0, st>>>(ca, zc, yc, zn)));
         }
         if (lp[l].ntail > 0) {
-          Soa<float> tmp{(float*)(B + P.o_tmp), std::max(T_, 1)};
-          UKG_LAUNCH(UKG_K_RT, st, (rt_base_kernel<<<(unsigned)((lp[l].ntail + 127) / 128), 128, 0, st>>>(a, zc, tmp)));
+          ca.state = dx;
+          UKG_LAUNCH(UKG_K_RT, st, (ctak::rt_base_aos<<<(unsigned)((lp[l].ntail * 32 + 127) / 128), 128, 0, st>>>(ca, zc)));
         }
       }
       for (int l = nlev - 2; l >= 0; --l) {

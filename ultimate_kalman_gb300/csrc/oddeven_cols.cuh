@@ -34,6 +34,7 @@ using ctak::RawA;
 using columns::back_subst;
 using columns::load_end;
 using columns::load_rows;
+using lanes::inv_root;
 using lanes::recip;
 using lanes::Refl;
 using lanes::reflector;
@@ -157,14 +158,6 @@ __device__ __forceinline__ void reduce(QrShared<T, NP>& sm, int panel, bool act,
  * level 0: weighing, and the triangularization of [W G | W o].
  * Threads 0..2n: columns of [H | -F | c]; threads 2n+1..3n+1: columns of [G | o].
  * ------------------------------------------------------------------------ */
-template <typename T>
-__device__ __forceinline__ T inv_root(T s) { return T(1) / sqrt(s); }
-template <>
-__device__ __forceinline__ double inv_root<double>(double s)
-{
-  return lanes::series_range(s) ? lanes::rsqrt_series(s) : 1.0 / sqrt(s);
-}
-
 /* Lower Cholesky factors of the n x n matrices in L[0] and L[1] (column-major,
  * ld NP + 1; n[f] = 0: none) side by side, reciprocals of the diagonals in d.
  * Column j, scaled, waits in row j of the upper half, which nothing else

@@ -501,13 +501,57 @@ __global__ void __launch_bounds__(NT) solve_cta(CArgs<T> a, int want_cov)
 /* ---------------------------------------------------------------------------
  * refinement right-hand side, first part, one step per CTA (FP64, from the
  * raw equations; as residual_kernel): with r = c + F x_{i-1} - H x_i and
- * s = o - G x_i,  wE = K^{-1} r,  zp = H^T wE + G^T C^{-1} s.  Scratch: a
- * factor (rmax^2) and four vectors of rmax.
+ * s = o - G x_i and w = K^{-1} r:  zp = H^T w + G^T C^{-1} s,  zf = F^T w, which
+ * is the step before's (next_step_kernel).  Scratch: a factor (rmax^2).
  * ------------------------------------------------------------------------ */
+/* w <- L^{-T} L^{-1} w by the first warp, w in its registers (rows <= 128), L
+ * lower, column-major; dv: the reciprocals of its diagonal (shared memory).
+ * Both directions subtract a column at a time: a dot product per row would add
+ * five exchanges and additions to each of the second direction's steps.      */
+static __device__ void precision_solve(const double* L, const double* dv, int rows, double* w)
+{
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  double v[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) v[u] = lane + 32 * u < rows ? w[lane + 32 * u] : 0.0;
+#pragma unroll
+  for (int u0 = 0; u0 < 4; ++u0)
+#pragma unroll 4
+    for (int jj = 0; jj < 32; ++jj) {
+      const int j = 32 * u0 + jj;
+      if (j < rows) {
+        const double x = __shfl_sync(0xffffffffu, v[u0], jj) * dv[j];
+        if (lane == jj) v[u0] = x;
+#pragma unroll
+        for (int u = u0; u < 4; ++u)
+          if (lane + 32 * u > j && lane + 32 * u < rows) v[u] = fma(-L[j * rows + lane + 32 * u], x, v[u]);
+      }
+    }
+#pragma unroll
+  for (int u0 = 3; u0 >= 0; --u0)
+#pragma unroll 4
+    for (int jj = 31; jj >= 0; --jj) {
+      const int j = 32 * u0 + jj;
+      if (j < rows) {
+        const double x = __shfl_sync(0xffffffffu, v[u0], jj) * dv[j];
+        if (lane == jj) v[u0] = x;
+#pragma unroll
+        for (int u = 0; u <= u0; ++u)
+          if (lane + 32 * u < j) v[u] = fma(-L[(lane + 32 * u) * rows + j], x, v[u]);
+      }
+    }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (lane + 32 * u < rows) w[lane + 32 * u] = v[u];
+}
+
 /* w <- Cov^{-1} w for the covariance factor (cov column-major, ld ldc, rows
  * x rows): 'C' L^{-T} L^{-1} (L = chol), 'U'/'F' the same with L = tril(cov),
- * 'W' W^T W, 'w' diag(cov)^2.  w and tmp are vectors shared by the CTA. */
-__device__ void apply_precision_cta(char type, const double* cov, int ldc, int rows, double* L, double* w, double* tmp)
+ * 'W' W^T W, 'w' diag(cov)^2.  w, tmp and dv are shared memory; ready: L holds
+ * the factor already. */
+__device__ void apply_precision_cta(char type, const double* cov, int ldc, int rows, double* L, bool ready, double* w,
+                                    double* tmp, double* dv)
 {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (type == 'w') {
@@ -532,24 +576,33 @@ __device__ void apply_precision_cta(char type, const double* cov, int ldc, int r
     return;
   }
   if (type != 'C' && type != 'U' && type != 'F') return;
-  for (int j = warp; j < rows; j += NT / 32)
-    for (int i = lane; i < rows; i += 32) L[(int64_t)j * rows + i] = i >= j ? cov[(int64_t)j * ldc + i] : 0.0;
+  if (!ready) {
+    for (int j = warp; j < rows; j += NT / 32)
+      for (int i = lane; i < rows; i += 32) L[(int64_t)j * rows + i] = i >= j ? cov[(int64_t)j * ldc + i] : 0.0;
+    __syncthreads();
+    if (type == 'C') cholesky_cm(L, rows); /* the weighing reports a bad factor */
+  }
+  for (int i = tid; i < rows; i += NT) dv[i] = 1.0 / L[(int64_t)i * rows + i];
   __syncthreads();
-  if (type == 'C') cholesky_cm(L, rows); /* the weighing reports a bad factor */
-  tri_solve_vec_cm(L, rows, w, true);
-  tri_solve_vec_cm(L, rows, w, false);
+  precision_solve(L, dv, rows, w);
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(NT) residual_cta(CArgs<float> a, RawA raw, Soa<double> wE, Soa<double> zp,
-                                                   double* scratch, int64_t per_cta, int64_t nsteps)
+/* keep: what a sweep leaves for the next, in level 0's equations, which nothing
+ * reads after the elimination: 1 the factors of K, where F and H were (their
+ * 2 n^2 floats a step), 2 those of C, where G was; 4: they are there.  The
+ * factorization is most of a sweep: 4,000 steps of 64 states, 32 observations,
+ * two sweeps 6.3 ms without, 2.7 with it and the solves in registers.  One
+ * sweep, 5,000 steps of 128 states, 64 observations: 10.7 ms before, 8.6 now, of
+ * which 4.1 are the FP64 pipe's time for the factors alone.                   */
+__global__ void __launch_bounds__(NT) residual_cta(CArgs<float> a, RawA raw, Soa<double> zf, Soa<double> zp,
+                                                   double* scratch, int64_t per_cta, int64_t nsteps, int keep)
 {
+  __shared__ double w[kMaxCov], tmp[kMaxCov], dv[kMaxCov], z[kMaxCov];
   const int n = a.n, mm = raw.mmax, tid = threadIdx.x;
-  const int rmax = n > mm ? n : mm;
   const int64_t nn = (int64_t)n * n;
-  double* L = scratch + (int64_t)blockIdx.x * per_cta;
-  double* w = L + (int64_t)rmax * rmax;
-  double* tmp = w + rmax;
-  double* z = tmp + rmax;
+  double* const L = scratch + (int64_t)blockIdx.x * per_cta;
+  const bool ready = keep & 4;
   for (int64_t g = blockIdx.x; g < nsteps; g += gridDim.x) {
     const int t = find_track(a.track_start, a.ntracks, g);
     const int64_t i = g - a.track_start[t], q = a.ct.slot[t] + i;
@@ -565,13 +618,22 @@ __global__ void __launch_bounds__(NT) residual_cta(CArgs<float> a, RawA raw, Soa
         w[r] = sm;
       }
       __syncthreads();
-      apply_precision_cta(raw.K_type[g], raw.K + g * nn, n, n, L, w, tmp);
-      for (int r = tid; r < n; r += NT) wE.at(r, q) = w[r];
-      for (int c = tid >> 5; c < n; c += NT / 32) { /* z = H^T w, column c of H along the lanes */
-        double sm = 0.0;
-        for (int r = tid & 31; r < n; r += 32) sm = fma(H[(int64_t)c * n + r], w[r], sm);
-        for (int off = 16; off > 0; off >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, off);
-        if ((tid & 31) == 0) z[c] = sm;
+      double* Lk = keep & 1 ? (double*)a.ce.F.p + q * nn : L;
+      apply_precision_cta(raw.K_type[g], raw.K + g * nn, n, n, Lk, ready && (keep & 1), w, tmp, dv);
+      for (int c = tid >> 5; c < n; c += NT / 32) { /* H^T w and F^T w, column c along the lanes */
+        double sm = 0.0, sf = 0.0;
+        for (int r = tid & 31; r < n; r += 32) {
+          sm = fma(H[(int64_t)c * n + r], w[r], sm);
+          sf = fma(F[(int64_t)c * n + r], w[r], sf);
+        }
+        for (int off = 16; off > 0; off >>= 1) {
+          sm += __shfl_xor_sync(0xffffffffu, sm, off);
+          sf += __shfl_xor_sync(0xffffffffu, sf, off);
+        }
+        if ((tid & 31) == 0) {
+          z[c] = sm;
+          zf.at(c, q) = sf;
+        }
       }
       __syncthreads();
     }
@@ -584,7 +646,8 @@ __global__ void __launch_bounds__(NT) residual_cta(CArgs<float> a, RawA raw, Soa
         w[r] = sm;
       }
       __syncthreads();
-      apply_precision_cta(raw.C_type[g], raw.C + g * (int64_t)mm * mm, mm, m, L, w, tmp);
+      double* Lc = keep & 2 ? (double*)(((uintptr_t)&a.ce.G.at(0, q) + 7) & ~(uintptr_t)7) : L;
+      apply_precision_cta(raw.C_type[g], raw.C + g * (int64_t)mm * mm, mm, m, Lc, ready && (keep & 2), w, tmp, dv);
       for (int c = tid >> 5; c < n; c += NT / 32) {
         double sm = 0.0;
         for (int r = tid & 31; r < m; r += 32) sm = fma(G[(int64_t)c * mm + r], w[r], sm);
@@ -598,17 +661,57 @@ __global__ void __launch_bounds__(NT) residual_cta(CArgs<float> a, RawA raw, Soa
   }
 }
 
-/* refinement transpose solves over slot-major FP32 records, one warp per
- * item (as rt_even_kernel / rt_odd_kernel), state entries k = lane + 32 q
- * (q < 4: n <= 128) held in registers, record columns read along the lanes:
+/* z_i = zp_i - F_{i+1}^T w_{i+1}, rounded to FP32; an entry per thread.  (The
+ * product formed here, a thread per step over F's columns, took 3.8 ms for
+ * 5,000 steps of 128 states, where the whole of F is 0.1 ms of memory.)       */
+__global__ void next_step_kernel(CArgs<float> a, Soa<double> zf, Soa<double> zp, Soa<float> z0, int64_t nsteps)
+{
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= nsteps) return;
+  const int t = find_track(a.track_start, a.ntracks, g);
+  const int64_t q = a.ct.slot[t] + (g - a.track_start[t]);
+  const bool next = g + 1 < a.track_start[t + 1];
+  for (int c = blockIdx.y; c < a.n; c += gridDim.y)
+    z0.at(c, q) = ukg_df::f64_to_f32(zp.at(c, q) - (next ? zf.at(c, q + 1) : 0.0));
+}
+
+/* refinement transpose solves over slot-major FP32 records, one warp per item
+ * (as rt_even_kernel / rt_odd_kernel), state entry k = lane + 32 q (q < 4: n <=
+ * 128) in lane k's registers, record columns read along the lanes:
  *   even steps  y_j = R_j^{-T} z_j
- *   odd steps   z' = z_{2p+1} - Y_{2p}^T y_{2p} - Ft_{2p+2}^T y_{2p+2}      */
+ *   odd steps   z' = z_{2p+1} - Y_{2p}^T y_{2p} - Ft_{2p+2}^T y_{2p+2}
+ *   one step    d = R^{-1} R^{-T} z (the base)
+ * What bounds a level is the latency of its n columns one after another, so
+ * nothing is stored until the end: reads of several columns are then under way
+ * at once.  n = 128, a level of any size: even 133 us before, 66 now, base
+ * (by one thread before) 640 and 77.                                          */
 constexpr int kRtQ = 4;
 
 static __device__ __forceinline__ float warp_sum(float v)
 {
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
+}
+/* y <- R^{-T} z; rc(r, i): row r of column i; dv: the diagonal's reciprocals */
+template <class RC>
+__device__ __forceinline__ void solve_t(RC rc, const float (&dv)[kRtQ], const float (&z)[kRtQ], int n, int lane, float (&y)[kRtQ])
+{
+#pragma unroll
+  for (int q = 0; q < kRtQ; ++q) y[q] = 0.f;
+#pragma unroll
+  for (int u = 0; u < kRtQ; ++u)
+#pragma unroll 8
+    for (int jj = 0; jj < 32; ++jj) {
+      const int i = 32 * u + jj;
+      if (i < n) {
+        float d = 0.f;
+#pragma unroll
+        for (int q = 0; q <= u; ++q)
+          if (lane + 32 * q < i) d = fmaf(rc(lane + 32 * q, i), y[q], d);
+        d = warp_sum(d);
+        if (lane == jj) y[u] = (z[u] - d) * dv[u];
+      }
+    }
 }
 
 __global__ void rt_even_aos(CArgs<float> a, Soa<float> zc, Soa<float> yc)
@@ -618,26 +721,18 @@ __global__ void rt_even_aos(CArgs<float> a, Soa<float> zc, Soa<float> yc)
   const int lane = threadIdx.x & 31, n = a.n;
   const int t = find_track(a.ct.solve, a.ntracks, item);
   const int64_t sz = a.ct.slot[t] + 2 * (item - a.ct.solve[t]);
-  const float* Rp = &a.cr.R.at(0, item); /* column i of R (entries k < i) at Rp[i * n + k] */
-  float yr[kRtQ];
+  const float* Rp = &a.cr.R.at(0, item);
+  float z[kRtQ], dv[kRtQ], y[kRtQ];
 #pragma unroll
-  for (int q = 0; q < kRtQ; ++q) yr[q] = 0.f;
-  for (int i = 0; i < n; ++i) {
-    float d = 0.f;
-#pragma unroll
-    for (int q = 0; q < kRtQ; ++q) {
-      const int k = lane + 32 * q;
-      if (k < i) d = fmaf(Rp[(int64_t)i * n + k], yr[q], d);
-    }
-    d = warp_sum(d);
-    const float yi = (zc.at(i, sz) - d) / Rp[(int64_t)i * n + i];
-#pragma unroll
-    for (int q = 0; q < kRtQ; ++q)
-      if (i == lane + 32 * q) yr[q] = yi;
+  for (int q = 0; q < kRtQ; ++q) {
+    const int k = lane + 32 * q;
+    z[q] = k < n ? zc.at(k, sz) : 0.f;
+    dv[q] = k < n ? 1.f / Rp[k * n + k] : 0.f;
   }
+  solve_t([&](int r, int i) { return Rp[i * n + r]; }, dv, z, n, lane, y);
 #pragma unroll
   for (int q = 0; q < kRtQ; ++q)
-    if (lane + 32 * q < n) yc.at(lane + 32 * q, item) = yr[q];
+    if (lane + 32 * q < n) yc.at(lane + 32 * q, item) = y[q];
 }
 
 __global__ void rt_odd_aos(CArgs<float> a, Soa<float> zc, Soa<float> yc, Soa<float> zn)
@@ -652,26 +747,72 @@ __global__ void rt_odd_aos(CArgs<float> a, Soa<float> zc, Soa<float> yc, Soa<flo
   const bool right = 2 * p + 2 <= L - 1;
   const float* Yp = &a.cr.Y.at(0, e0);
   const float* Fp = &a.cr.Ft.at(0, right ? e1 : e0);
-  float y0[kRtQ], y1[kRtQ];
+  float y0[kRtQ], y1[kRtQ], z[kRtQ];
 #pragma unroll
   for (int q = 0; q < kRtQ; ++q) {
     const int r = lane + 32 * q;
     y0[q] = r < n ? yc.at(r, e0) : 0.f;
     y1[q] = r < n && right ? yc.at(r, e1) : 0.f;
+    z[q] = r < n ? zc.at(r, so) : 0.f;
   }
-  for (int c = 0; c < n; ++c) {
-    float d = 0.f;
 #pragma unroll
-    for (int q = 0; q < kRtQ; ++q) {
-      const int r = lane + 32 * q;
-      if (r < n) {
-        d = fmaf(Yp[(int64_t)c * n + r], y0[q], d);
-        if (right) d = fmaf(Fp[(int64_t)c * n + r], y1[q], d);
+  for (int u = 0; u < kRtQ; ++u)
+#pragma unroll 4
+    for (int jj = 0; jj < 32; ++jj) {
+      const int c = 32 * u + jj;
+      if (c < n) {
+        float d = 0.f;
+#pragma unroll
+        for (int q = 0; q < kRtQ; ++q) {
+          const int r = lane + 32 * q;
+          if (r < n) {
+            d = fmaf(Yp[c * n + r], y0[q], d);
+            if (right) d = fmaf(Fp[c * n + r], y1[q], d);
+          }
+        }
+        d = warp_sum(d);
+        if (lane == jj) z[u] -= d;
       }
     }
-    d = warp_sum(d);
-    if (lane == 0) zn.at(c, sn) = zc.at(c, so) - d;
+#pragma unroll
+  for (int q = 0; q < kRtQ; ++q)
+    if (lane + 32 * q < n) zn.at(lane + 32 * q, sn) = z[q];
+}
+
+__global__ void rt_base_aos(CArgs<float> a, Soa<float> zc)
+{
+  const int64_t item = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (item >= a.ct.ntail) return;
+  const int lane = threadIdx.x & 31, n = a.n;
+  const int t = (int)a.ct.tail[item];
+  if (a.ct.L[t] != 1) return;
+  const int64_t sz = a.ct.slot[t];
+  auto rc = [&](int r, int i) { return a.baseR.at(i * n + r, t); };
+  float z[kRtQ], dv[kRtQ], y[kRtQ];
+#pragma unroll
+  for (int q = 0; q < kRtQ; ++q) {
+    const int k = lane + 32 * q;
+    z[q] = k < n ? zc.at(k, sz) : 0.f;
+    dv[q] = k < n ? 1.f / rc(k, k) : 0.f;
   }
+  solve_t(rc, dv, z, n, lane, y);
+#pragma unroll
+  for (int u = kRtQ - 1; u >= 0; --u)
+#pragma unroll 8
+    for (int jj = 31; jj >= 0; --jj) {
+      const int i = 32 * u + jj;
+      if (i < n) {
+        const float x = __shfl_sync(0xffffffffu, y[u] * dv[u], jj);
+        if (lane == jj) y[u] = x;
+#pragma unroll
+        for (int q = 0; q <= u; ++q)
+          if (lane + 32 * q < i) y[q] = fmaf(-rc(lane + 32 * q, i), x, y[q]);
+      }
+    }
+  double* d = a.state + orig_step(a.track_start, a.level, t, 0) * n;
+#pragma unroll
+  for (int q = 0; q < kRtQ; ++q)
+    if (lane + 32 * q < n) d[lane + 32 * q] = ukg_df::widen(y[q]);
 }
 
 }  // namespace ctak
