@@ -2722,8 +2722,9 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
                      (ctak::rt_even_aos<<<(unsigned)((lp[l].nsolve * 32 + 127) / 128), 128, 0, st>>>(ca, zc, yc)));
         if (lp[l].npairs > 0 && l + 1 < nlev) {
           Soa<float> zn{(float*)(B + P.o_z[l + 1]), std::max<int64_t>(lp[l + 1].S, 1)};
-          UKG_LAUNCH(UKG_K_RT, st,
-                     (ctak::rt_odd_aos<<<(unsigned)((lp[l].npairs * 32 + 127) / 128), 128, 0, st>>>(ca, zc, yc, zn)));
+          const int Q = (n + 31) / 32;
+          auto* odd = Q <= 1 ? ctak::rt_odd_aos<1> : Q == 2 ? ctak::rt_odd_aos<2> : Q == 3 ? ctak::rt_odd_aos<3> : ctak::rt_odd_aos<4>;
+          UKG_LAUNCH(UKG_K_RT, st, (odd<<<(unsigned)((lp[l].npairs * Q + 3) / 4), 128, 0, st>>>(ca, zc, yc, zn)));
         }
         if (lp[l].ntail > 0) {
           ca.state = dx;

@@ -699,13 +699,29 @@ __global__ void __launch_bounds__(128) state_cols(CArgs<T> a)
     const int r = lane + 32 * u;
     x[u] = r < n ? (a.yrhs.p ? a.yrhs.at(r, item) : Rr.rhs.at(r, item)) : T(0);
   }
-  auto sub = [&](const T* B, const double* s) {
-#pragma unroll 4
-    for (int k = 0; k < n; ++k) {
-      const T sk = -ukg_df::narrow<T>(s[k]);
+  /* eight columns' reads before their use, without branches (rows and columns
+     past n are the last one's, times zero or not used): left to the compiler,
+     each column waited for its own (12 levels of 128 states 1.86 ms, now
+     0.84)                                                                   */
+  constexpr int KB = sizeof(T) * RU > 16 ? 4 : 8;
+  int row[RU];
 #pragma unroll
-      for (int u = 0; u < RU; ++u)
-        if (lane + 32 * u < n) x[u] = fma(B[k * n + lane + 32 * u], sk, x[u]);
+  for (int u = 0; u < RU; ++u) row[u] = lane + 32 * u < n ? lane + 32 * u : n - 1;
+  auto sub = [&](const T* B, const double* s) {
+#pragma unroll 1
+    for (int k0 = 0; k0 < n; k0 += KB) {
+      T v[KB][RU], sk[KB];
+#pragma unroll
+      for (int i = 0; i < KB; ++i) {
+        const int k = k0 + i < n ? k0 + i : n - 1;
+        sk[i] = k0 + i < n ? -ukg_df::narrow<T>(s[k]) : T(0);
+#pragma unroll
+        for (int u = 0; u < RU; ++u) v[i][u] = B[k * n + row[u]];
+      }
+#pragma unroll
+      for (int i = 0; i < KB; ++i)
+#pragma unroll
+        for (int u = 0; u < RU; ++u) x[u] = fma(v[i][u], sk[i], x[u]);
     }
   };
   if (hp) sub(&Rr.Ft.at(0, item), a.state + orig_step(a.track_start, a.level, t, j - 1) * n);
@@ -721,14 +737,26 @@ __global__ void __launch_bounds__(128) state_cols(CArgs<T> a)
     dv[u] = recip(d);
   }
 #pragma unroll
-  for (int v = RU - 1; v >= 0; --v)
-#pragma unroll 4
-    for (int c = (n - 1 < 32 * v + 31 ? n - 1 : 32 * v + 31); c >= 32 * v; --c) {
-      const T xc = bcast(x[v] * dv[v], c - 32 * v);
-      if (lane == c - 32 * v) x[v] = xc;
+  for (int w = RU - 1; w >= 0; --w)
+#pragma unroll 1
+    for (int c0 = 32 * w + 32 - KB; c0 >= 32 * w; c0 -= KB) {
+      if (c0 >= n) continue;
+      T v[KB][RU];
 #pragma unroll
-      for (int u = 0; u <= v; ++u)
-        if (lane + 32 * u < c) x[u] = fma(-xc, R[c * n + lane + 32 * u], x[u]);
+      for (int i = 0; i < KB; ++i)
+#pragma unroll
+        for (int u = 0; u <= w; ++u) v[i][u] = R[(c0 + i < n ? c0 + i : n - 1) * n + row[u]];
+#pragma unroll
+      for (int i = KB - 1; i >= 0; --i) {
+        const int c = c0 + i;
+        if (c < n) { /* the same in every lane */
+          const T xc = bcast(x[w] * dv[w], c - 32 * w);
+          if (lane == c - 32 * w) x[w] = xc;
+#pragma unroll
+          for (int u = 0; u <= w; ++u)
+            if (lane + 32 * u < c) x[u] = fma(-xc, v[i][u], x[u]);
+        }
+      }
     }
   double* xo = a.state + orig_step(a.track_start, a.level, t, j) * n;
 #pragma unroll
