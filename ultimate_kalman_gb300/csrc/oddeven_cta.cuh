@@ -738,7 +738,7 @@ __global__ void rt_even_aos(CArgs<float> a, Soa<float> zc, Soa<float> yc)
 /* 32 columns a warp, Q >= n / 32 warps a pair.  Without branches (entries past n
  * are the last one's, times zero): the reads of eight columns run ahead, which
  * they did not past the tests of rows and columns.  n = 128: 12 levels 3.5 ms
- * before, 0.5 now.                                                           */
+ * before, 0.6 now.                                                           */
 template <int Q>
 __global__ void rt_odd_aos(CArgs<float> a, Soa<float> zc, Soa<float> yc, Soa<float> zn)
 {
