@@ -120,3 +120,86 @@ def test_small_states_in_rounds(n, m, mmax, kt, ct):
     D.filter()
     Xb, Sb = D.results()
     assert (Xb.reshape(T, 41, n) == X).all() and (Sb.reshape(T, 41, n, n) == S).all()
+
+
+def _no_prior(n, rows, F, K=None, seed=0):
+    """One track without a prior: step s observes the rows `rows[s]` (a list of
+    vectors of n entries, maybe none); covariances drawn per step."""
+    rng = np.random.default_rng(seed)
+    k, m = len(rows), max(len(r) for r in rows)
+    P = pb.empty_problem(n, max(n, m), [k])
+    x = rng.standard_normal(n)
+    for s in range(k):
+        P.H[s] = np.eye(n)
+        P.F[s] = F.T
+        P.c[s] = 0.1 * rng.standard_normal(n)
+        P.K[s] = pb.random_spd(rng, n) if K is None else K
+        x = F @ x + rng.standard_normal(n)
+        r = len(rows[s])
+        P.obs_rows[s] = r
+        if r:
+            G = np.array(rows[s])
+            P.G[s, :, :r] = G.T
+            P.o[s, :r] = G @ x + rng.standard_normal(r)
+            P.C[s, :r, :r] = pb.random_spd(rng, r)
+    return P
+
+
+def _pv(n, order):
+    """Positions that move by 0.1 times their velocities: [p.. v..], [v.. p..] or [p v p v ..]."""
+    h = n // 2
+    p = {"pv": np.arange(h), "vp": h + np.arange(h), "mixed": 2 * np.arange(h)}[order]
+    v = {"pv": h + np.arange(h), "vp": np.arange(h), "mixed": 2 * np.arange(h) + 1}[order]
+    F = np.eye(n)
+    F[p, v] = 0.1
+    return F, p
+
+
+def _undetermined_starts():
+    out = {}
+    for n, order in ((2, "vp"), (4, "mixed"), (4, "vp"), (6, "pv"), (6, "vp"), (8, "mixed"), (8, "vp"), (10, "vp")):
+        F, p = _pv(n, order)
+        out[f"{order}{n}"] = (n, [np.eye(n)[p]] * 6, F)
+    F, p = _pv(4, "mixed")
+    e = np.eye(4)
+    out["alternating"] = (4, [[e[2 * (s % 2)]] for s in range(8)], F)
+    out["late"] = (4, [[], []] + [e[p]] * 5, F)
+    out["between"] = (4, [e[p], [], e[p], [], [], e[p]], F)
+    F3 = np.array([[1, 0.1, 0.005], [0, 1, 0.1], [0, 0, 1.0]])
+    e = np.eye(3)
+    out["position_acceleration"] = (3, [e[[0, 2]]] * 6, F3)
+    out["one_position"] = (3, [e[[0]]] * 6, F3)
+    out["last_first"] = (3, [e[[2]], e[[0]], e[[0, 2]], e[[0]], e[[0]]], F3)
+    for n in (3, 6, 8, 9):  # the leading columns depend on each other
+        rng = np.random.default_rng(n)
+        G = rng.standard_normal((2, n))
+        G[:, 1] = 2.0 * G[:, 0]
+        out[f"dependent{n}"] = (n, [G] * (n // 2 + 4), pb.random_orthogonal(rng, n))
+    return out
+
+
+@pytest.mark.parametrize("cov", [True, False], ids=["cov", "states"])
+@pytest.mark.parametrize("name", list(_undetermined_starts()))
+def test_tracks_without_a_prior(name, cov):
+    """A track's first observations may leave columns of the factor empty: none
+    of them may be lost.  Every step that its prefix determines equals the
+    dense least-squares solution of that prefix, every other is NaN."""
+    _cuda()
+    n, rows, F = _undetermined_starts()[name]
+    P = _no_prior(n, rows, F, seed=n)
+    D = native.DeviceProblem(P, covariance=cov)
+    assert D.filter(covariance=cov, check=False) == native.KALMAN_GPU_ESINGULAR
+    X, S = D.results()
+    seen = 0
+    for s in range(P.nsteps):
+        Q = P.step_range(0, s + 1)
+        enough = P.obs_rows[:s + 1].sum() >= n
+        if not enough or np.linalg.matrix_rank(oracle.dense_system(Q, 0)[0]) < (s + 1) * n:
+            assert np.isnan(X[s]).all() and (not cov or np.isnan(S[s]).all()), f"step {s}"
+            continue
+        seen += 1
+        Xd, Sd = oracle.dense_smooth(Q)
+        assert oracle.rel_err_states(X[s:s + 1], Xd[-1:]) < TOL, f"step {s}"
+        if cov:
+            assert oracle.rel_err_covs(S[s:s + 1], Sd[-1:]) < TOL, f"step {s}"
+    assert seen > 0

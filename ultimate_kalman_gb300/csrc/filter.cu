@@ -398,6 +398,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a
 #pragma unroll
       for (int r = 0; r < N; ++r) tp[0][r] = 0.0;
     }
+    /* with fewer than N rows the observation's follow them without a gap: a
+       column of zeros takes no reflector, so a row past a gap might never be
+       brought up                                                           */
+#pragma unroll 1
+    for (int d = z; d < N; ++d) {
+#pragma unroll
+      for (int r = 0; r + 1 < N + M; ++r)
+        if (r >= z) (r < N ? tp[0][r] : bo[0][r - N]) = r + 1 < N ? tp[0][r + 1] : bo[0][r + 1 - N];
+      bo[0][M - 1] = 0.0;
+    }
     z = z + mq < N ? z + mq : N;
     lanes::lanes_qr_full<double, N, 32, 1, M>(tp, bo, all, lane, 0, z);
     double* Ro = a.cov ? a.cov + (s0 + q) * nn : w.factor + ((int64_t)t * w.kc + q) * nn;
