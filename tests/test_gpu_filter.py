@@ -165,6 +165,9 @@ def _undetermined_starts():
     out["alternating"] = (4, [[e[2 * (s % 2)]] for s in range(8)], F)
     out["late"] = (4, [[], []] + [e[p]] * 5, F)
     out["between"] = (4, [e[p], [], e[p], [], [], e[p]], F)
+    F, _ = _pv(2, "pv")
+    e = np.eye(2)
+    out["repeated_row"] = (2, [e[[0, 0]], [], e[[0]], e[[0]]], F)
     F3 = np.array([[1, 0.1, 0.005], [0, 1, 0.1], [0, 0, 1.0]])
     e = np.eye(3)
     out["position_acceleration"] = (3, [e[[0, 2]]] * 6, F3)
@@ -203,3 +206,47 @@ def test_tracks_without_a_prior(name, cov):
         if cov:
             assert oracle.rel_err_covs(S[s:s + 1], Sd[-1:]) < TOL, f"step {s}"
     assert seen > 0
+
+
+def _kalman(F, K, G, C, x, Pm, c, o):
+    """The covariance form of the filter in extended precision, K and C
+    diagonal: estimates and covariances after every step but the first."""
+    t = np.longdouble
+    F, G, x, Pm, c, o = (np.asarray(a).astype(t) for a in (F, G, x, Pm, c, o))
+    X, S = [], []
+    for s in range(len(o)):
+        x = F @ x + c[s]
+        Pm = F @ Pm @ F.T + np.diag(np.asarray(K).astype(t))
+        for r in range(len(G)):  # one observation at a time
+            h = Pm @ G[r]
+            g = h / (G[r] @ h + t(C[r]))
+            x = x + g * (o[s, r] - G[r] @ x)
+            Pm = Pm - np.outer(g, h)
+        X.append(x.astype(float))
+        S.append(Pm.astype(float))
+    return np.array(X), np.array(S)
+
+
+@pytest.mark.parametrize("n", [2, 4, 6, 8])
+@pytest.mark.parametrize("k,c", [(1e-14, 0.1), (1e-10, 1e4), (1.0, 0.1)])
+def test_small_process_noise(n, k, c):
+    """The weighed evolution's rows are up to 1e9 times as large as the factor's:
+    the information on the next state must not come from their differences."""
+    _cuda()
+    F, p = _pv(n, "pv")
+    rng = np.random.default_rng(n)
+    G = np.eye(n)[p]
+    N, m = 60, len(p)
+    P = pb.empty_problem(n, n, [N])
+    P.H[:], P.F[:], P.K[:] = np.eye(n), F.T, k * np.eye(n)
+    P.c[:] = 0.1 * rng.standard_normal((N, n))
+    P.G[:, :, :m], P.C[:, :m, :m] = G.T, c * np.eye(m)
+    P.o[:, :m] = rng.standard_normal((N, m))
+    P.obs_rows[:] = m
+    P.G[0], P.C[0], P.o[0], P.obs_rows[0] = np.eye(n), np.eye(n), rng.standard_normal(n), n
+    X, S = _kalman(F, [k] * n, G, [c] * m, P.o[0], np.eye(n), P.c[1:], P.o[1:, :m])
+    D = native.DeviceProblem(P, covariance=True)
+    D.filter()
+    Xg, Sg = D.results()
+    assert oracle.rel_err_states(Xg[1:], X) < TOL
+    assert oracle.rel_err_covs(Sg[1:], S) < TOL

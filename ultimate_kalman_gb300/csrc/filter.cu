@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(NT) filter_cta(FilterArgs a)
  *                    evolve  [R 0 y; -VF VH Vc] -> the information on x_i
  *                    observe [that; WG Wo] -> R, y
  *   filter_estimate  x = R^{-1} y, P = R^{-1} R^{-T}, in place of the factor
- * A chain step is n reflectors of 27 FP64 instructions and n of 32 at n = 6,
+ * A chain step is n reflectors of 32 FP64 instructions each at n = 6,
  * at 64 to 76 cycles each: 11 to 13 us, and 16 us with the shuffles between
  * them; with the weighing and the estimate inside the chain it was 42 us.  512
  * tracks of 50 to 500 steps: 21.2 ms before, 8.2 ms now.
@@ -326,10 +326,12 @@ __global__ void __launch_bounds__(64) filter_weigh(FilterArgs a, SmallArgs w)
 }
 
 /* The factor's z rows (all n in the usual case) are carried on lanes 0..N
- * ([R | y], zero rows past z).  With z = n the triangle R is on top of the
- * weighed evolution; before that the evolution is on top and R's rows below,
- * whose zero rows stay exactly zero.  Either way the lower rows of the columns
- * N..2N become the information on x_i.                                       */
+ * ([R | y], zero rows past z).  The weighed evolution goes on top of them: where
+ * the process noise is small its rows are the large ones, and with the factor on
+ * top the information on x_i, what is left in the lower rows of the columns
+ * N..2N, would be small differences of large numbers (a covariance error of
+ * 1.7e-8 instead of 1.4e-15 with noise of variance 1e-14).  Zero rows of the
+ * factor stay exactly zero.                                                  */
 template <int N, int M>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a, SmallArgs w)
 {
@@ -375,20 +377,17 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a
   for (int64_t q = 0; q < cnt; ++q) {
     double tp[1][N], bt[1][N], bo[1][M];
     const int mq = m;
-    const bool tri = z == N;
 #pragma unroll
     for (int r = 0; r < N; ++r) {
       const double y = __shfl_sync(all, R[r], N);
-      const double c = lane < N ? R[r] : lane == 2 * N ? y : 0.0;
-      tp[0][r] = tri ? c : e[r];
-      bt[0][r] = tri ? e[r] : c;
+      tp[0][r] = e[r];
+      bt[0][r] = lane < N ? R[r] : lane == 2 * N ? y : 0.0;
     }
 #pragma unroll
     for (int r = 0; r < M; ++r) bo[0][r] = g[r];
     if (q + 1 < cnt) load(q + 1);
     if (w.first + q > 0) {
-      if (tri) lanes::lanes_qr_tri<double, N, 32, 1>(tp, bt, all, lane, 0, N);
-      else lanes::lanes_qr_full<double, N, 32, 1, N>(tp, bt, all, lane, 0, N);
+      lanes::lanes_qr_full<double, N, 32, 1, N>(tp, bt, all, lane, 0, N);
 #pragma unroll
       for (int r = 0; r < N; ++r) {
         const double v = __shfl_sync(all, bt[0][r], (lane + N) & 31);
