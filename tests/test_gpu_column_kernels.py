@@ -3,6 +3,7 @@ the edges of their register sizes (12, 16, 24, 32, 48, 64, 96 rows) against
 the oracle: every covariance type, unobserved steps (the trapezoids then run
 out of rows), odd and even lengths.  Bars as elsewhere: 1e-11 in FP64, 1e-9
 in the precision form and in double-float."""
+import numpy as np
 import pytest
 
 import oracle
@@ -71,3 +72,18 @@ def test_two_pass_sizes(n, m, cov):
     assert oracle.rel_err_states(X, Xo) < 1e-9
     X, _ = native.smooth(P, "oddeven", covariance=False)
     assert oracle.rel_err_states(X, Xo) < 1e-11
+
+
+@pytest.mark.parametrize("n,m", [(9, 3), (12, 5), (24, 8), (48, 24)])
+def test_associative_variances_up_and_down(n, m):
+    """Process noise whose variance goes from 1e-6 over 1 to 1e6 and back, in
+    the associative smoother: a filtered variance is up to 1e6 times the
+    smoothed one, so a covariance is right to about 1e6 n k eps (1e-7 at most
+    here), unless an unsymmetric rounding error of the filtered one survives."""
+    k = 10 if n < 24 else 7
+    P = pb.random_dynamics([k], n, m, seed=n, per_step=True)
+    P.K[1:] *= np.array([1.0, 1e6, 1e-6])[np.arange(1, k) % 3][:, None, None]
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, S = native.smooth(P, "associative")
+    assert oracle.rel_err_states(X, Xo) < 1e-7 and oracle.rel_err_covs(S, So) < 1e-7

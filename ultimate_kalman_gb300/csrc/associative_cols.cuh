@@ -11,7 +11,7 @@
  * warp instructions at n = 48 (a third of them the reductions); at 19 cycles an
  * SM each that bounds the large levels, and the chain of n reflectors and four
  * half products the small ones.  5,000 steps, n = 48, m = 24: scans 74.5 ms
- * before, 50.7 now, smoothing elements 9.9 and 6.4.
+ * before, 50.4 now, smoothing elements 9.9 and 7.5.
  */
 #pragma once
 #include "columns.cuh"
@@ -463,9 +463,18 @@ __global__ void __launch_bounds__(threads2<NP>(), NP <= 32 ? blocks2<NP>() : NP 
   /* column q of E^T is row q of E */
   if (g == 1) back_subst<double, NP>(R, dv, n, b, [&](int p, double u) { E[p * n + q] = u; });
   __syncthreads();
-  /* L = P - E (F P), F P = (P F^T)^T: P is symmetric */
+  /* L = P - (E F) P.  Not P - E (P F^T)^T, a product less: P is symmetric only up
+     to its rounding errors, which I - E F damps and I + E F would double (a
+     covariance error of 0.8 instead of 3e-4 where the variances of 12 states
+     go up and down by 16 decades)                                          */
+#pragma unroll
+  for (int p = 0; p < NP; ++p) b[p] = 0.0;
+  if (act) matvec_half<NP>(E, n, g, b, [&](int l) { return F[(int64_t)q * n + l]; });
+  join<NP>(R + (act ? q : 0) * n, n, act, g, b);
+  if (g == 0) put_rows<NP>(S + q * n, n, b);
+  __syncthreads();
   load_rows<double, NP>(P + (int64_t)(act ? q : 0) * n, n, g == 0, b);
-  if (act) matvec_half<NP>(E, n, g, b, [&](int l) { return -S[l + q * n]; });
+  if (act) matvec_half<NP>(S, n, g, b, [&](int l) { return -P[(int64_t)q * n + l]; });
   join<NP>(R + (act ? q : 0) * n, n, act, g, b);
   if (g == 0) {
     put_rows<NP>(&out.L.at((int64_t)q * n, r), n, b);
