@@ -250,3 +250,30 @@ def test_small_process_noise(n, k, c):
     Xg, Sg = D.results()
     assert oracle.rel_err_states(Xg[1:], X) < TOL
     assert oracle.rel_err_covs(Sg[1:], S) < TOL
+
+
+def test_many_uneven_tracks_in_bounded_memory():
+    """Up to 8 states the workspace is a round's (128 MiB) and the tracks' tables,
+    whatever their number; every track is a prefix of one and gives its bits."""
+    _cuda()
+    P = pb.random_dynamics([900], 8, 4, seed=3, missing=0.2)
+    D = native.DeviceProblem(P, covariance=True)
+    D.filter()
+    X, S = D.results()
+    rng = np.random.default_rng(0)
+    for lens in (np.r_[rng.integers(0, 4, 100000), 900, 1, 700], np.r_[rng.integers(1, 40, 4000), np.full(5, 900)],
+                 np.full(260, 900)):
+        ts = np.zeros(len(lens) + 1, dtype=np.int64)
+        ts[1:] = np.cumsum(lens)
+        idx = np.arange(ts[-1]) - np.repeat(ts[:-1], lens)
+        B = pb.PackedProblem(8, 8, ts, *[np.ascontiguousarray(getattr(P, f)[idx]) for f in (
+            "H", "F", "c", "K", "K_type", "G", "o", "C", "C_type", "obs_rows")])
+        for cov in (True, False):
+            native.release()
+            D = native.DeviceProblem(B, covariance=cov)
+            D.filter(covariance=cov)
+            assert native.workspace_held() <= (130 << 20) + 24 * len(lens)
+            Xb, Sb = D.results()
+            np.testing.assert_array_equal(Xb, X[idx])
+            if cov:
+                np.testing.assert_array_equal(Sb, S[idx])

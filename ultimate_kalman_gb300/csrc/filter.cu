@@ -20,10 +20,13 @@
  * The QR reductions, weighing and triangular solves are the CTA routines of
  * the smoothers (cta_linalg.cuh).  FP64.
  */
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <new>
+#include <numeric>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -173,28 +176,39 @@ __global__ void __launch_bounds__(NT) filter_cta(FilterArgs a)
  *                    evolve  [R 0 y; -VF VH Vc] -> the information on x_i
  *                    observe [that; WG Wo] -> R, y
  *   filter_estimate  x = R^{-1} y, P = R^{-1} R^{-T}, in place of the factor
- * A chain step is n reflectors of 32 FP64 instructions each at n = 6,
- * at 64 to 76 cycles each: 11 to 13 us, and 16 us with the shuffles between
- * them; with the weighing and the estimate inside the chain it was 42 us.  512
- * tracks of 50 to 500 steps: 21.2 ms before, 8.2 ms now.
+ * A chain step is 2 n reflectors of about 32 FP64 instructions at n = 6, at 64
+ * to 76 cycles each: 12 to 14 us, and 16 us with the shuffles between them; with
+ * the weighing and the estimate inside the chain it was 42 us.  512 tracks of 50
+ * to 500 steps: 21.2 ms before, 8.3 ms now.
  *
- * Tracks are taken kc steps at a time (the weighed equations of a round must
- * fit the workspace); the factor is carried over between rounds.
+ * A round takes kc steps of nt tracks, whose weighed equations must fit the
+ * workspace; the factor is carried over between rounds.  Where one round does
+ * not hold all, the tracks go by length, the longest first and at most
+ * 1/kMinRound of the round's steps at a time, so that the tracks still running
+ * are the first of them and their rounds get longer as the others end.  (With
+ * kc steps of all tracks in every round, 150,000 tracks of 2 steps and 10 of
+ * 1,500 took 1,500 rounds of one step, 117 ms; all in one launch, before the
+ * filter was split, 75 ms.)
  * ------------------------------------------------------------------------ */
 constexpr int kWarpsPerBlock = 4;
 constexpr int kSmallN = 8;
 constexpr int64_t kRoundBytes = (int64_t)128 << 20; /* 140,000 steps of 6 states: about what L2 holds */
+constexpr int64_t kMinRound = 4; /* steps of a round at least: 33,000 tracks of 6 states, 50 warps a scheduler */
 
 /* entries of a step's weighed equations: columns of [-F | H | c], n rows each,
  * then columns of [G | o], mmax rows each (zero past the step's rows) */
 __host__ __device__ constexpr int step_entries(int n, int mmax) { return (2 * n + 1) * n + (n + 1) * mmax; }
 
 struct SmallArgs {
-  double* weighed;  /* [ntracks][kc][step_entries] */
-  double* factor;   /* [ntracks][kc][n * n] where no covariances are asked for, else null: in place of P */
-  double* carry;    /* [ntracks][(n + 1) * n] */
-  int* carry_rows;  /* [ntracks] */
-  int64_t first, kc; /* steps first .. first + kc - 1 of every track */
+  double* weighed;  /* [nt][kc][step_entries] */
+  double* factor;   /* [nt][kc][n * n] where no covariances are asked for, else null: in place of P */
+  double* carry;    /* [nt][(n + 1) * n] */
+  int* carry_rows;  /* [nt] */
+  const int32_t* order; /* the tracks by length, or null: as they are */
+  int t0, nt;           /* tracks t0 .. t0 + nt - 1 of them */
+  int64_t first, kc;    /* steps first .. first + kc - 1 of each */
+  bool more;            /* their next steps follow */
+  __device__ __forceinline__ int track(int u) const { return order ? order[t0 + u] : t0 + u; }
 };
 
 /* Weighing of one covariance factor by one thread: the lower factor L and the
@@ -273,9 +287,10 @@ template <int N, int M>
 __global__ void __launch_bounds__(64) filter_weigh(FilterArgs a, SmallArgs w)
 {
   const int64_t e = (int64_t)blockIdx.x * 64 + threadIdx.x;
-  const int t = (int)(e / w.kc);
-  if (t >= a.ntracks) return;
-  const int64_t s0 = a.track_start[t], s = s0 + w.first + (e - t * w.kc);
+  const int u = (int)(e / w.kc);
+  if (u >= w.nt) return;
+  const int t = w.track(u);
+  const int64_t s0 = a.track_start[t], s = s0 + w.first + (e - u * w.kc);
   if (s >= a.track_start[t + 1]) return;
   const int mm = a.mmax;
   const int64_t nn = (int64_t)N * N;
@@ -336,10 +351,12 @@ template <int N, int M>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a, SmallArgs w)
 {
   const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (t >= a.ntracks) return; /* the whole warp */
+  /* tracks by length: a long one with shorter ones on an SM, whose four
+     schedulers share the FP64 pipe                                         */
+  const int u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  if (u >= w.nt) return; /* the whole warp */
   const unsigned all = 0xffffffffu;
-  const int mm = a.mmax, per = step_entries(N, mm);
+  const int t = w.track(u), mm = a.mmax, per = step_entries(N, mm);
   const int64_t s0 = a.track_start[t] + w.first;
   const int64_t cnt = a.track_start[t + 1] - s0 < w.kc ? a.track_start[t + 1] - s0 : w.kc;
   if (cnt <= 0) return;
@@ -348,12 +365,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a
 #pragma unroll
   for (int r = 0; r < N; ++r) R[r] = 0.0;
   if (w.first > 0) {
-    z = w.carry_rows[t];
+    z = w.carry_rows[u];
     if (lane <= N)
 #pragma unroll
-      for (int r = 0; r < N; ++r) R[r] = w.carry[((int64_t)t * (N + 1) + lane) * N + r];
+      for (int r = 0; r < N; ++r) R[r] = w.carry[((int64_t)u * (N + 1) + lane) * N + r];
   }
-  const double* in = w.weighed + (int64_t)t * w.kc * per;
+  const double* in = w.weighed + (int64_t)u * w.kc * per;
   const int64_t nn = (int64_t)N * N;
   double e[N], g[M]; /* the step's columns, loaded a step ahead */
   int m = 0;
@@ -409,7 +426,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a
     }
     z = z + mq < N ? z + mq : N;
     lanes::lanes_qr_full<double, N, 32, 1, M>(tp, bo, all, lane, 0, z);
-    double* Ro = a.cov ? a.cov + (s0 + q) * nn : w.factor + ((int64_t)t * w.kc + q) * nn;
+    double* Ro = a.cov ? a.cov + (s0 + q) * nn : w.factor + ((int64_t)u * w.kc + q) * nn;
 #pragma unroll
     for (int r = 0; r < N; ++r) R[r] = lane <= N && r <= lane && r < z ? tp[0][r] : 0.0;
     double* out = lane < N ? Ro + lane * N : a.state + (s0 + q) * N;
@@ -417,10 +434,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) filter_chain(FilterArgs a
 #pragma unroll
       for (int r = 0; r < N; ++r) out[r] = R[r];
   }
+  if (!w.more) return;
   if (lane <= N)
 #pragma unroll
-    for (int r = 0; r < N; ++r) w.carry[((int64_t)t * (N + 1) + lane) * N + r] = R[r];
-  if (lane == 0) w.carry_rows[t] = z;
+    for (int r = 0; r < N; ++r) w.carry[((int64_t)u * (N + 1) + lane) * N + r] = R[r];
+  if (lane == 0) w.carry_rows[u] = z;
 }
 
 /* x = R^{-1} y and P = R^{-1} R^{-T} of a step, over the factor that the chain
@@ -430,9 +448,10 @@ template <int N>
 __global__ void __launch_bounds__(64) filter_estimate(FilterArgs a, SmallArgs w)
 {
   const int64_t e = (int64_t)blockIdx.x * 64 + threadIdx.x;
-  const int t = (int)(e / w.kc);
-  if (t >= a.ntracks) return;
-  const int64_t s = a.track_start[t] + w.first + (e - t * w.kc);
+  const int u = (int)(e / w.kc);
+  if (u >= w.nt) return;
+  const int t = w.track(u);
+  const int64_t s = a.track_start[t] + w.first + (e - u * w.kc);
   if (s >= a.track_start[t + 1]) return;
   const int64_t nn = (int64_t)N * N;
   double* P = a.cov ? a.cov + s * nn : nullptr;
@@ -493,24 +512,73 @@ __global__ void __launch_bounds__(64) filter_estimate(FilterArgs a, SmallArgs w)
     }
 }
 
-template <int N, int M>
-void filter_small_nm(const FilterArgs& a, SmallArgs w, int64_t longest, cudaStream_t st)
+/* the tracks, the longest first: by counting, and by comparison past 65,535 steps */
+bool by_length(const int64_t* start, int ntracks, int64_t longest, std::vector<int32_t>& order)
 {
-  const unsigned chain = (unsigned)((a.ntracks + kWarpsPerBlock - 1) / kWarpsPerBlock);
-  const unsigned steps = (unsigned)((a.ntracks * w.kc + 63) / 64);
-  for (w.first = 0; w.first < longest; w.first += w.kc) {
-    UKG_LAUNCH(UKG_K_FILTER, st, (filter_weigh<N, M><<<steps, 64, 0, st>>>(a, w)));
-    UKG_LAUNCH(UKG_K_FILTER, st, (filter_chain<N, M><<<chain, 32 * kWarpsPerBlock, 0, st>>>(a, w)));
-    UKG_LAUNCH(UKG_K_FILTER, st, (filter_estimate<N><<<steps, 64, 0, st>>>(a, w)));
+  try {
+    const int64_t top = std::min<int64_t>(longest, 65535);
+    auto len = [&](int t) { return start[t + 1] - start[t]; };
+    auto bucket = [&](int t) { return top - std::min(len(t), top); };
+    std::vector<int32_t> at(top + 2, 0);
+    for (int t = 0; t < ntracks; ++t) ++at[bucket(t) + 1];
+    std::partial_sum(at.begin(), at.end(), at.begin());
+    const int32_t longer = at[1];
+    order.resize(ntracks);
+    for (int t = 0; t < ntracks; ++t) order[at[bucket(t)]++] = t;
+    if (longest > top) std::sort(order.begin(), order.begin() + longer, [&](int32_t x, int32_t y) { return len(x) > len(y); });
+    return true;
+  } catch (const std::bad_alloc&) {
+    return false;
   }
+}
+
+/* The rounds of a call that one round does not hold: len(i) is the length of the
+ * i-th track, the longest first, steps what a round holds; round(t0, nt, first,
+ * kc, more), more: the same tracks' next steps follow.                       */
+template <class LEN, class F>
+void rounds(int ntracks, int64_t steps, LEN len, F round)
+{
+  for (int t0 = 0, nt; t0 < ntracks && len(t0) > 0; t0 += nt) {
+    const int64_t longest = len(t0);
+    nt = (int)std::min<int64_t>(ntracks - t0, std::max<int64_t>(1, steps / std::min(longest, kMinRound)));
+    int on = nt; /* still running */
+    for (int64_t first = 0, kc; first < longest; first += kc) {
+      while (len(t0 + on - 1) <= first) --on;
+      kc = std::min(longest - first, std::max<int64_t>(1, steps / on));
+      round(t0, on, first, kc, first + kc < longest);
+    }
+  }
+}
+
+template <int N, int M>
+void filter_small_nm(const FilterArgs& a, const SmallArgs& w, cudaStream_t st)
+{
+  const unsigned chain = (unsigned)((w.nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  const unsigned steps = (unsigned)((w.nt * w.kc + 63) / 64);
+  UKG_LAUNCH(UKG_K_FILTER, st, (filter_weigh<N, M><<<steps, 64, 0, st>>>(a, w)));
+  UKG_LAUNCH(UKG_K_FILTER, st, (filter_chain<N, M><<<chain, 32 * kWarpsPerBlock, 0, st>>>(a, w)));
+  UKG_LAUNCH(UKG_K_FILTER, st, (filter_estimate<N><<<steps, 64, 0, st>>>(a, w)));
 }
 /* observation rows in registers: half of n, n or 8 */
 template <int N>
-void filter_small_n(const FilterArgs& a, const SmallArgs& w, int64_t longest, cudaStream_t st)
+void filter_small_n(const FilterArgs& a, const SmallArgs& w, cudaStream_t st)
 {
-  if (a.mmax <= (N + 1) / 2) filter_small_nm<N, (N + 1) / 2>(a, w, longest, st);
-  else if (a.mmax <= N) filter_small_nm<N, N>(a, w, longest, st);
-  else filter_small_nm<N, kSmallN>(a, w, longest, st);
+  if (a.mmax <= (N + 1) / 2) filter_small_nm<N, (N + 1) / 2>(a, w, st);
+  else if (a.mmax <= N) filter_small_nm<N, N>(a, w, st);
+  else filter_small_nm<N, kSmallN>(a, w, st);
+}
+void filter_small(const FilterArgs& a, const SmallArgs& w, cudaStream_t st)
+{
+  switch (a.n) {
+    case 1: filter_small_n<1>(a, w, st); break;
+    case 2: filter_small_n<2>(a, w, st); break;
+    case 3: filter_small_n<3>(a, w, st); break;
+    case 4: filter_small_n<4>(a, w, st); break;
+    case 5: filter_small_n<5>(a, w, st); break;
+    case 6: filter_small_n<6>(a, w, st); break;
+    case 7: filter_small_n<7>(a, w, st); break;
+    default: filter_small_n<8>(a, w, st); break;
+  }
 }
 
 struct Workspace {
@@ -564,17 +632,36 @@ extern "C" int kalman_gpu_filter_packed(uint32_t options, const kalman_gpu_probl
   const bool small = p->n <= kSmallN && p->mmax <= kSmallN;
   SmallArgs w;
   memset(&w, 0, sizeof(w));
-  int64_t longest = 0;
   size_t scratch = (size_t)ncta * per;
-  if (small) { /* steps of every track at a time: at most kRoundBytes of weighed equations */
+  /* the rounds: of one, or of the tracks by length */
+  std::vector<int32_t> order;
+  auto len = [&](int i) {
+    const int t = order.empty() ? i : order[i];
+    return p->track_start[t + 1] - p->track_start[t];
+  };
+  int64_t round_steps = 0, whole = 0, carried = 0;
+  const int64_t step = step_entries(p->n, p->mmax) + (want_cov ? 0 : p->n * p->n);
+  const int64_t carry = (p->n + 1) * (int64_t)p->n + 1; /* and the number of rows */
+  if (small) {
+    const int64_t hold = kRoundBytes / ((int64_t)sizeof(double) * (step + (carry + kMinRound - 1) / kMinRound));
+    int64_t longest = 0;
+    bool sorted = true;
     for (int t = 0; t < p->ntracks; ++t) {
-      const int64_t k = p->track_start[t + 1] - p->track_start[t];
-      longest = k > longest ? k : longest;
+      sorted = sorted && (t == 0 || len(t) <= len(t - 1));
+      longest = std::max<int64_t>(longest, len(t));
     }
-    const int64_t step = step_entries(p->n, p->mmax) + (want_cov ? 0 : p->n * p->n);
-    w.kc = kRoundBytes / ((int64_t)sizeof(double) * step * p->ntracks);
-    w.kc = w.kc < 1 ? 1 : w.kc < longest ? w.kc : longest;
-    scratch = (size_t)p->ntracks * (w.kc * step + (p->n + 1) * p->n + 1);
+    if (longest <= hold / p->ntracks) {
+      whole = longest;
+      round_steps = p->ntracks * longest;
+    } else {
+      if (!sorted && !by_length(p->track_start, p->ntracks, longest, order))
+        return ukg_set_error(KALMAN_GPU_ENOMEM, "filter: the order of %d tracks", p->ntracks);
+      round_steps = hold;
+      rounds(p->ntracks, hold, len, [&](int, int nt, int64_t, int64_t, bool more) {
+        if (more) carried = std::max<int64_t>(carried, nt);
+      });
+    }
+    scratch = (size_t)(round_steps * step + carried * carry) + (order.size() + 1) / 2;
   }
   if (int e = ensure(tab + 256 + scratch * sizeof(double))) return e;
   char* base = (char*)tl_ws.p;
@@ -603,21 +690,21 @@ extern "C" int kalman_gpu_filter_packed(uint32_t options, const kalman_gpu_probl
   a.per_cta = per;
   a.flag = dflag;
   if (small) {
-    const int64_t T = p->ntracks;
     w.weighed = a.scratch;
-    w.carry = w.weighed + T * w.kc * step_entries(p->n, p->mmax);
-    w.factor = w.carry + T * (p->n + 1) * p->n;
-    w.carry_rows = (int*)(w.factor + (want_cov ? 0 : T * w.kc * p->n * p->n));
-    switch (p->n) {
-      case 1: filter_small_n<1>(a, w, longest, st); break;
-      case 2: filter_small_n<2>(a, w, longest, st); break;
-      case 3: filter_small_n<3>(a, w, longest, st); break;
-      case 4: filter_small_n<4>(a, w, longest, st); break;
-      case 5: filter_small_n<5>(a, w, longest, st); break;
-      case 6: filter_small_n<6>(a, w, longest, st); break;
-      case 7: filter_small_n<7>(a, w, longest, st); break;
-      default: filter_small_n<8>(a, w, longest, st); break;
+    w.carry = w.weighed + round_steps * step;
+    w.carry_rows = (int*)(w.carry + carried * (carry - 1));
+    if (!order.empty()) {
+      int32_t* dorder = (int32_t*)(w.carry + carried * carry);
+      cudaMemcpyAsync(dorder, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+      w.order = dorder;
     }
+    auto round = [&](int t0, int nt, int64_t first, int64_t kc, bool more) {
+      w.t0 = t0, w.nt = nt, w.first = first, w.kc = kc, w.more = more;
+      w.factor = w.weighed + nt * kc * step_entries(p->n, p->mmax); /* used without covariances only */
+      filter_small(a, w, st);
+    };
+    if (whole) round(0, p->ntracks, 0, whole, false);
+    else rounds(p->ntracks, round_steps, len, round);
   } else {
     UKG_LAUNCH(UKG_K_FILTER, st, (filter_cta<<<ncta, NT, 0, st>>>(a)));
   }
