@@ -137,3 +137,19 @@ def test_small_states_all_lengths(n, m, k):
     Xb, Sb = native.smooth(P.select_tracks([0] * 37), "associative")
     np.testing.assert_array_equal(Xb[36 * k:], X)
     np.testing.assert_array_equal(Sb[36 * k:], S)
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (2, 2), (3, 1), (4, 2), (5, 3), (6, 2)])
+def test_many_items_same_bits(n, m):
+    """Up to 5 states a scan level of more than 4,864 combines takes a thread
+    for each, below a warp: 400 copies of 33 steps have levels of 6,400, 3,200
+    and fewer, and give the bits of one."""
+    P = pb.random_dynamics([33], n, m, seed=5 * n, per_step=True, missing=0.2)
+    X, S = native.smooth(P, "associative")
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    assert oracle.rel_err_states(X, Xo) < 1e-11 and oracle.rel_err_covs(S, So) < 1e-11
+    Xb, Sb = native.smooth(P.select_tracks([0] * 400), "associative")
+    for t in (0, 199, 399):
+        np.testing.assert_array_equal(Xb[33 * t:33 * t + 33], X)
+        np.testing.assert_array_equal(Sb[33 * t:33 * t + 33], S)

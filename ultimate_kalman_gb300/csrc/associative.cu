@@ -937,38 +937,34 @@ extern "C" int ukg_associative_device(uint32_t options, const kalman_gpu_problem
   ukg_allow_dynamic_smem((const void*)smooth_element_kernel);
   auto grid = [](int64_t items, int block) { return (unsigned)((items + block - 1) / block); };
   const int ew = 128;
-  const asmall::Scans sc = asmall::scans(n); /* n <= 8 here */
-  const int bc = 32 * asmall::kWarps;
 
   /* filtering elements and the forward scan */
   const int64_t* fstart0 = dtab + fp.off_start[0];
   UKG_LAUNCH(UKG_K_AS_ELEMENT, st,
              (element_kernel<<<grid(N, be), be, be * pt_elem, st>>>(a, raw, felems(0), fstart0, N, mx)));
-  for (int l = 0; l + 1 < fp.nlev; ++l)
-    if (fp.nup[l] > 0)
-      UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (sc.up_f<<<grid(fp.nup[l], asmall::kWarps), bc, 0, st>>>(T, level(fp, l), level(fp, l + 1), felems(l),
-                                                                          felems(l + 1), dflag)));
-  for (int l = fp.nlev - 2; l >= 0; --l)
-    if (fp.ndown[l] > 0)
-      UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (sc.down_f<<<grid(fp.ndown[l], asmall::kWarps), bc, 0, st>>>(T, level(fp, l), level(fp, l + 1),
-                                                                              felems(l), felems(l + 1), dflag)));
+  auto filter_level = [&](bool up, int l, int64_t items) { /* n <= 8 here */
+    if (items == 0) return;
+    const asmall::Scans sc = asmall::scans(n, items);
+    UKG_LAUNCH(UKG_K_AS_SCAN, st,
+               ((up ? sc.up_f : sc.down_f)<<<grid(items, sc.filter_per_block), sc.block, 0, st>>>(
+                   T, level(fp, l), level(fp, l + 1), felems(l), felems(l + 1), dflag)));
+  };
+  auto smooth_level = [&](bool up, int l, int64_t items) {
+    if (items == 0) return;
+    const asmall::Scans sc = asmall::scans(n, items);
+    UKG_LAUNCH(UKG_K_AS_SCAN, st,
+               ((up ? sc.up_s : sc.down_s)<<<grid(items, sc.smooth_per_block), sc.block, 0, st>>>(
+                   T, level(sp, l), level(sp, l + 1), selems(l), selems(l + 1))));
+  };
+  for (int l = 0; l + 1 < fp.nlev; ++l) filter_level(true, l, fp.nup[l]);
+  for (int l = fp.nlev - 2; l >= 0; --l) filter_level(false, l, fp.ndown[l]);
   UKG_LAUNCH(UKG_K_AS_ELEMENT, st, (filtered_out_kernel<<<grid(N, ew), ew, 0, st>>>(a, felems(0), fstart0, N)));
   /* smoothing elements and the reverse scan */
   const int64_t* sstart0 = dtab + sp.off_start[0];
   UKG_LAUNCH(UKG_K_AS_SMOOTH, st,
              (smooth_element_kernel<<<grid(N, bsm), bsm, bsm * pt_selem, st>>>(a, raw, selems(0), sstart0, N)));
-  for (int l = 0; l + 1 < sp.nlev; ++l)
-    if (sp.nup[l] > 0)
-      UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (sc.up_s<<<grid(sp.nup[l], sc.smooth_per_block), bc, 0, st>>>(T, level(sp, l), level(sp, l + 1),
-                                                                               selems(l), selems(l + 1))));
-  for (int l = sp.nlev - 2; l >= 0; --l)
-    if (sp.ndown[l] > 0)
-      UKG_LAUNCH(UKG_K_AS_SCAN, st,
-                 (sc.down_s<<<grid(sp.ndown[l], sc.smooth_per_block), bc, 0, st>>>(T, level(sp, l), level(sp, l + 1),
-                                                                                   selems(l), selems(l + 1))));
+  for (int l = 0; l + 1 < sp.nlev; ++l) smooth_level(true, l, sp.nup[l]);
+  for (int l = sp.nlev - 2; l >= 0; --l) smooth_level(false, l, sp.ndown[l]);
   UKG_LAUNCH(UKG_K_AS_SMOOTH, st, (smoothed_out_kernel<<<grid(N, ew), ew, 0, st>>>(a, selems(0), sstart0, N)));
 
   return finish(st, dflag);

@@ -1,6 +1,7 @@
 /*
  * associative_small.cuh -- the scans of the associative smoother for up to 8
- * states, a warp (or half of one) per combine.  Included by associative.cu (it
+ * states, a warp (or half of one) per combine, up to 5 states a thread where
+ * there are many.  Included by associative.cu (it
  * uses that file's FElems, SElems, ScanLevel and find_track).
  *
  * A thread that combines two elements alone is a chain of some 2,700 FP64
@@ -296,18 +297,268 @@ __global__ void __launch_bounds__(32 * kWarps) down_smooth(int T, ScanLevel lv, 
   if (p > 0) combine_smooth_lanes<N>(bufs[grp], lane, gm, nxt, b0 - 1, cur, s0, cur, s0);
 }
 
-/* the scan kernels of a state dimension */
+/* ---------------------------------------------------------------------------
+ * The same combines by a thread each, its operations on every entry those of the
+ * lanes, so that the number of items changes no bit: for levels of many items up
+ * to 5 states.  A warp's instruction costs the same whether 4 N or 32 of its
+ * lanes have work: 1,000 tracks of 1,000 steps, n = 1 to 5, by lanes alone 2.4,
+ * 7.4, 14.7, 24.3 and 38.4 ms, now 0.9, 2.2, 5.3, 10.5 and 20.6 (a thread per
+ * combine with its matrices in shared memory 1.1, 2.9, 7.9, 16.8 and 37.2).
+ * From 6 states on the matrices do not fit a thread's registers.
+ * ------------------------------------------------------------------------ */
+constexpr int kThreads = 64;
+
+template <int N>
+__device__ __forceinline__ double at(const Soa& first, int c, int r, int64_t s)
+{
+  return first.p[(int64_t)(c * N + r) * first.stride + s];
+}
+template <int N>
+__device__ __forceinline__ void load_mat(const Soa& first, int c, int64_t s, double (&M)[N][N])
+{
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int r = 0; r < N; ++r) M[k][r] = at<N>(first, c + k, r, s);
+}
+/* out <- out + M v */
+template <int N>
+__device__ __forceinline__ void matvec(const double (&M)[N][N], const double (&v)[N], double (&out)[N])
+{
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int p = 0; p < N; ++p) out[p] = fma(M[k][p], v[k], out[p]);
+}
+
+/* X <- B^T (I + L R)^{-1}, B in the columns X on entry; false: a zero pivot */
+template <int N>
+__device__ __forceinline__ bool solve_thread(const double (&L)[N][N], const double (&R)[N][N], double (&X)[N][N])
+{
+  double t[2 * N][N], dv[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+      t[q][p] = p == q ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < N; ++k) t[q][p] = fma(L[k][q], R[p][k], t[q][p]);
+      t[N + q][p] = X[q][p];
+    }
+#pragma unroll
+  for (int k = 0; k + 1 < N; ++k) {
+    double tail = 0.0;
+#pragma unroll
+    for (int i = k + 1; i < N; ++i) tail = fma(t[k][i], t[k][i], tail);
+    if (tail == 0.0) continue;
+    const lanes::Refl<double> r = lanes::reflector(t[k][k], tail);
+    t[k][k] = r.beta;
+#pragma unroll
+    for (int c = k + 1; c < 2 * N; ++c) {
+      double d = 0.0;
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) d = fma(t[k][i], t[c][i], d);
+      d = fma(r.amb, t[c][k], d) * r.inv;
+      t[c][k] = fma(-d, r.amb, t[c][k]);
+#pragma unroll
+      for (int i = k + 1; i < N; ++i) t[c][i] = fma(-d, t[k][i], t[c][i]);
+    }
+  }
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    ok = ok && t[k][k] != 0.0;
+    dv[k] = lanes::recip(t[k][k]);
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+#pragma unroll
+    for (int k = N - 1; k >= 0; --k) {
+      t[N + q][k] *= dv[k];
+      X[k][q] = t[N + q][k];
+#pragma unroll
+      for (int p = 0; p < k; ++p) t[N + q][p] = fma(-t[N + q][k], t[k][p], t[N + q][p]);
+    }
+  return ok;
+}
+
+/* combine_lanes' formulas; all of Xj is read before the entries it shares with
+ * O are written                                                              */
+template <int N>
+__device__ __forceinline__ bool combine_thread(const FElems& Xi, int64_t i, const FElems& Xj, int64_t j, const FElems& O,
+                                               int64_t o)
+{
+  double Zi[N][N], Jj[N][N], X[N][N], Y[N][N], T[N][N], v1[N], v2[N], v[N];
+  load_mat<N>(Xi.A, N, i, Zi);
+  load_mat<N>(Xj.A, 2 * N, j, Jj);
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+      X[q][p] = at<N>(Xj.A, p, q, j); /* Aj^T */
+      Y[q][p] = at<N>(Xi.A, q, p, i);
+    }
+  bool ok = solve_thread<N>(Zi, Jj, X);
+  ok = solve_thread<N>(Jj, Zi, Y) && ok;
+  /* bi + Zi ej, ej - Jj bi */
+#pragma unroll
+  for (int k = 0; k < N; ++k) v1[k] = at<N>(Xi.A, 3 * N, k, i), v2[k] = at<N>(Xj.A, 3 * N + 1, k, j);
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = -v1[k];
+  {
+    double e[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) e[k] = v2[k];
+    matvec<N>(Zi, e, v1);
+    matvec<N>(Jj, v, v2);
+  }
+  double bn[N], en[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) bn[k] = at<N>(Xj.A, 3 * N, k, j), en[k] = at<N>(Xi.A, 3 * N + 1, k, i);
+  matvec<N>(X, v1, bn);
+  matvec<N>(Y, v2, en);
+  store_col<N>(O.A, 3 * N, o, bn);
+  store_col<N>(O.A, 3 * N + 1, o, en);
+  /* J = Y (Jj Ai) + Ji: Jj has been read */
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    double t[N], out[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = at<N>(Xi.A, q, k, i), t[k] = 0.0, out[k] = at<N>(Xi.A, 2 * N + q, k, i);
+    matvec<N>(Jj, v, t);
+    matvec<N>(Y, t, out);
+    store_col<N>(O.A, 2 * N + q, o, out);
+  }
+  /* Z = (X Zi) Aj^T + Zj, then A = X Ai */
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) T[q][k] = 0.0;
+    matvec<N>(X, Zi[q], T[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    double out[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = at<N>(Xj.A, k, q, j), out[k] = at<N>(Xj.A, N + q, k, j);
+    matvec<N>(T, v, out);
+    store_col<N>(O.A, N + q, o, out);
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    double out[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = at<N>(Xi.A, q, k, i), out[k] = 0.0;
+    matvec<N>(X, v, out);
+    store_col<N>(O.A, q, o, out);
+  }
+  return ok;
+}
+
+template <int N>
+__device__ __forceinline__ void combine_smooth_thread(const SElems& Xi, int64_t i, const SElems& Xj, int64_t j,
+                                                      const SElems& O, int64_t o)
+{
+  double E[N][N], T[N][N], v[N], out[N];
+  load_mat<N>(Xj.E, 0, j, E);
+#pragma unroll
+  for (int q = 0; q < N; ++q) { /* Ej Li, Ej Ei */
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = at<N>(Xi.E, N + q, k, i), T[q][k] = 0.0;
+    matvec<N>(E, v, T[q]);
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = at<N>(Xi.E, q, k, i), out[k] = 0.0;
+    matvec<N>(E, v, out);
+    store_col<N>(O.E, q, o, out);
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = at<N>(Xi.E, 2 * N, k, i), out[k] = at<N>(Xj.E, 2 * N, k, j);
+  matvec<N>(E, v, out);
+  store_col<N>(O.E, 2 * N, o, out);
+#pragma unroll
+  for (int q = 0; q < N; ++q) { /* (Ej Li) Ej^T + Lj */
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = E[k][q], out[k] = at<N>(Xj.E, N + q, k, j);
+    matvec<N>(T, v, out);
+    store_col<N>(O.E, N + q, o, out);
+  }
+}
+
+/* columns 0 .. cols - 1 of an element */
+template <int N>
+__device__ __forceinline__ void copy_thread(const Soa& X, int64_t s, const Soa& O, int64_t o, int cols)
+{
+  for (int c = 0; c < cols; ++c) copy<N>(X, s, O, o, c, true);
+}
+
+template <int N>
+__global__ void __launch_bounds__(kThreads) up_filter_thread(int T, ScanLevel lv, ScanLevel nx, FElems cur, FElems nxt,
+                                                             int* flag)
+{
+  const int64_t item = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (item >= lv.nup) return;
+  const int t = find_track(lv.up_items, T, item);
+  const int64_t p = item - lv.up_items[t], s0 = lv.start[t] + 2 * p, o = nx.start[t] + p;
+  if (2 * p + 1 >= lv.L[t]) copy_thread<N>(cur.A, s0, nxt.A, o, 3 * N + 2);
+  else if (!combine_thread<N>(cur, s0, cur, s0 + 1, nxt, o)) atomicOr(flag, 2);
+}
+template <int N>
+__global__ void __launch_bounds__(kThreads) down_filter_thread(int T, ScanLevel lv, ScanLevel nx, FElems cur, FElems nxt,
+                                                               int* flag)
+{
+  const int64_t item = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (item >= lv.ndown) return;
+  const int t = find_track(lv.down_items, T, item);
+  const int64_t p = item - lv.down_items[t], L = lv.L[t];
+  if (L < 2) return;
+  const int64_t s0 = lv.start[t] + 2 * p, b0 = nx.start[t] + p;
+  if (2 * p + 1 < L) copy_thread<N>(nxt.A, b0, cur.A, s0 + 1, 3 * N + 2);
+  if (p > 0 && !combine_thread<N>(nxt, b0 - 1, cur, s0, cur, s0)) atomicOr(flag, 2);
+}
+template <int N>
+__global__ void __launch_bounds__(kThreads) up_smooth_thread(int T, ScanLevel lv, ScanLevel nx, SElems cur, SElems nxt)
+{
+  const int64_t item = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (item >= lv.nup) return;
+  const int t = find_track(lv.up_items, T, item);
+  const int64_t p = item - lv.up_items[t], s0 = lv.start[t] + 2 * p, o = nx.start[t] + p;
+  if (2 * p + 1 >= lv.L[t]) copy_thread<N>(cur.E, s0, nxt.E, o, 2 * N + 1);
+  else combine_smooth_thread<N>(cur, s0, cur, s0 + 1, nxt, o);
+}
+template <int N>
+__global__ void __launch_bounds__(kThreads) down_smooth_thread(int T, ScanLevel lv, ScanLevel nx, SElems cur, SElems nxt)
+{
+  const int64_t item = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  if (item >= lv.ndown) return;
+  const int t = find_track(lv.down_items, T, item);
+  const int64_t p = item - lv.down_items[t], L = lv.L[t];
+  if (L < 2) return;
+  const int64_t s0 = lv.start[t] + 2 * p, b0 = nx.start[t] + p;
+  if (2 * p + 1 < L) copy_thread<N>(nxt.E, b0, cur.E, s0 + 1, 2 * N + 1);
+  if (p > 0) combine_smooth_thread<N>(nxt, b0 - 1, cur, s0, cur, s0);
+}
+
+/* the scan kernels of a state dimension; a level's launches by its items */
 struct Scans {
   void (*up_f)(int, ScanLevel, ScanLevel, FElems, FElems, int*) = nullptr;
   void (*down_f)(int, ScanLevel, ScanLevel, FElems, FElems, int*) = nullptr;
   void (*up_s)(int, ScanLevel, ScanLevel, SElems, SElems) = nullptr;
   void (*down_s)(int, ScanLevel, ScanLevel, SElems, SElems) = nullptr;
-  int smooth_per_block = 0;
+  int smooth_per_block = 0, filter_per_block = kWarps, block = 32 * kWarps;
 };
 template <int N>
-Scans scans_n()
+Scans scans_n(bool threads)
 {
   Scans s;
+  if constexpr (N <= 5)
+    if (threads) {
+      s.up_f = up_filter_thread<N>;
+      s.down_f = down_filter_thread<N>;
+      s.up_s = up_smooth_thread<N>;
+      s.down_s = down_smooth_thread<N>;
+      s.smooth_per_block = s.filter_per_block = s.block = kThreads;
+      return s;
+    }
   s.up_f = up_filter<N>;
   s.down_f = down_filter<N>;
   s.up_s = up_smooth<N>;
@@ -315,17 +566,23 @@ Scans scans_n()
   s.smooth_per_block = SmoothGroup<N>::per_block;
   return s;
 }
-inline Scans scans(int n)
+/* Lanes up to eight rounds of a warp a scheduler: there a thread's chain takes as
+ * long (10,000 steps, n = 1 to 5: by lanes alone 0.34, 0.48, 0.66, 0.89 and 1.20
+ * ms, with threads for the 5,000 combines of the first level 0.33, 0.47, 0.65,
+ * 0.88 and 1.21)                                                             */
+constexpr int64_t kLaneItems = 4864;
+inline Scans scans(int n, int64_t items)
 {
+  const bool threads = items > kLaneItems;
   switch (n) {
-    case 1: return scans_n<1>();
-    case 2: return scans_n<2>();
-    case 3: return scans_n<3>();
-    case 4: return scans_n<4>();
-    case 5: return scans_n<5>();
-    case 6: return scans_n<6>();
-    case 7: return scans_n<7>();
-    case 8: return scans_n<8>();
+    case 1: return scans_n<1>(threads);
+    case 2: return scans_n<2>(threads);
+    case 3: return scans_n<3>(threads);
+    case 4: return scans_n<4>(threads);
+    case 5: return scans_n<5>(threads);
+    case 6: return scans_n<6>(threads);
+    case 7: return scans_n<7>(threads);
+    case 8: return scans_n<8>(threads);
     default: return Scans();
   }
 }
