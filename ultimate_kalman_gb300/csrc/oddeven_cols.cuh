@@ -75,32 +75,42 @@ struct QrShared {
   T amb[2][2], inv[2][2]; /* its reflector (amb = 0: none) */
 };
 
-/* One step of a reduction for a thread whose column has the rows b below and
- * tk on top; panel: 0, or 1 for a second panel reduced at the same time; pivot:
- * this thread's column is the step's pivot.  on: the thread takes part.
- * Returns the top entry after the step.                                     */
+/* In FP64 a warp without a live column waits, instead of forming products for
+ * nothing on the pipe that bounds the kernel: 64 tracks of 100 steps, n = 33,
+ * pairs 17.6 -> 14.7 ms, n = 64 63.4 -> 55.4.  Up to 16 states there are two or
+ * three warps, and on the FP32 pipe the others hide it: the test costs 1 to 3 %
+ * more than it saves.                                                        */
 template <typename T, int NP>
-__device__ __forceinline__ T step(QrShared<T, NP>& sm, int k, int panel, bool on, bool pivot, int n, T tk, T (&b)[NP])
+__host__ __device__ constexpr bool skips() { return std::is_same<T, double>::value && NP >= 24; }
+/* One step of a reduction for a thread whose column has the rows b below and
+ * tk on top; panel: 0, or 1 for a second panel reduced at the same time; live:
+ * the column takes part; pivot: it is the step's pivot.  Returns the top entry
+ * after the step.                                                            */
+template <typename T, int NP>
+__device__ __forceinline__ T step(QrShared<T, NP>& sm, int k, int panel, bool live, bool pivot, int n, T tk, T (&b)[NP])
 {
   const int buf = k & 1;
   T* x = sm.x[buf][panel];
-  if (on && pivot)
+  if (live && pivot)
 #pragma unroll
     for (int i = 0; i < NP; ++i) x[i] = b[i];
   __syncthreads();
-  T d0 = T(0), d1 = T(0);
+  T dot = T(0);
+  if (!skips<T, NP>() || live) {
+    T d0 = T(0), d1 = T(0);
 #pragma unroll
-  for (int i = 0; i < NP; i += 4)
-    if (i < least<NP>() || i < n) { /* rows past n are zero; the same in every thread */
-      d0 = fma(x[i], b[i], d0);
-      d1 = fma(x[i + 1], b[i + 1], d1);
-      d0 = fma(x[i + 2], b[i + 2], d0);
-      d1 = fma(x[i + 3], b[i + 3], d1);
-    }
-  const T dot = d0 + d1;
+    for (int i = 0; i < NP; i += 4)
+      if (i < least<NP>() || i < n) { /* rows past n are zero; the same in every thread */
+        d0 = fma(x[i], b[i], d0);
+        d1 = fma(x[i + 1], b[i + 1], d1);
+        d0 = fma(x[i + 2], b[i + 2], d0);
+        d1 = fma(x[i + 3], b[i + 3], d1);
+      }
+    dot = d0 + d1;
+  }
   /* the pivot's own product is the tail: its warp alone forms the reflector (a
      fifth to a third of the FP64 instructions, were every warp to do it) */
-  if (on && pivot) {
+  if (live && pivot) {
     Refl<T> r;
     r.beta = tk;
     r.amb = r.inv = T(0);
@@ -111,7 +121,7 @@ __device__ __forceinline__ T step(QrShared<T, NP>& sm, int k, int panel, bool on
   }
   __syncthreads();
   const T amb = sm.amb[buf][panel], inv = sm.inv[buf][panel];
-  if (!on || pivot || amb == T(0)) return tk;
+  if (!live || pivot || amb == T(0)) return tk;
   const T d = fma(amb, tk, dot) * inv;
 #pragma unroll
   for (int i = 0; i < NP; i += 4)
@@ -149,7 +159,8 @@ __device__ __forceinline__ void reduce(QrShared<T, NP>& sm, int panel, bool act,
     T tk = next;
     if (on && k >= m) tk = shift<T, NP>(b);
     next = act && k + 1 < m ? load(k + 1) : T(0);
-    tk = step<T, NP>(sm, k, panel, on, c == k, n, tk, b);
+    /* what a pivot column holds below its own row is not read any more */
+    tk = step<T, NP>(sm, k, panel, on && c >= k, c == k, n, tk, b);
     if (on) store(k, tk);
   }
 }
