@@ -87,3 +87,33 @@ def test_associative_variances_up_and_down(n, m):
     assert st == 0
     X, S = native.smooth(P, "associative")
     assert oracle.rel_err_states(X, Xo) < 1e-7 and oracle.rel_err_covs(S, So) < 1e-7
+
+
+@pytest.mark.parametrize("n,m,cov", [(34, 34, "C"), (37, 1, "W"), (40, 20, "C"), (41, 13, "F"), (45, 44, "w"), (50, 50, "C"),
+                                     (51, 25, "W"), (56, 8, "F"), (57, 19, "C"), (61, 61, "w")])
+def test_sizes_above_32(n, m, cov):
+    """Above 32 states the block kernel weighs and the observations are
+    triangularized after; FP64 and double-float have register sizes of 40 (pairs,
+    even steps) and 56 (even steps to 50 states) besides 48 and 64."""
+    P = pb.random_dynamics([1, 2, 11, 14], n, m, seed=3 * n + m, K_type=cov, C_type=cov, missing=0.3, per_step=True)
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, S = native.smooth(P, "oddeven")
+    assert oracle.rel_err_states(X, Xo) < 1e-11 and oracle.rel_err_covs(S, So) < 1e-11
+    Xb, Sb = native.smooth(P.select_tracks([0, 1, 2, 3] * 60), "oddeven")
+    np.testing.assert_array_equal(Xb[-P.nsteps:], X)
+    np.testing.assert_array_equal(Sb[-P.nsteps:], S)
+    X, S = native.smooth(P, "oddeven", fp32_refine=True)
+    assert oracle.rel_err_states(X, Xo) < 1e-9 and oracle.rel_err_covs(S, So) < 1e-9
+    X, _ = native.smooth(P, "oddeven", covariance=False, fp32_refine=True, sweeps=3)
+    assert oracle.rel_err_states(X, Xo) < 1e-9
+
+
+@pytest.mark.parametrize("n,m", [(66, 66), (67, 1), (68, 30), (80, 80), (93, 46), (95, 12)])
+def test_wide_sizes_up_to_96(n, m):
+    """The precision form of 65 to 96 states (24 rows a lane) between its ends."""
+    P = pb.random_dynamics([1, 2, 7, 13], n, m, seed=n + m, missing=0.3, per_step=True)
+    st, Xo, _ = oracle.smooth(P, "oddeven")
+    assert st == 0
+    X, _ = native.smooth(P, "oddeven", covariance=False, fp32_refine=True, sweeps=3)
+    assert oracle.rel_err_states(X, Xo) < 1e-9

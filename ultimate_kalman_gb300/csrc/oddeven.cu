@@ -2606,7 +2606,7 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
   const cols::Kernels<T> CK = cols::kernels<T>(n, mx);
   const size_t ck_pair = cols::pair_smem<T>(n), ck_tail = cols::tail_smem<T>(n), ck_solve = cols::solve_smem<T>(n);
   if (CK.pair) {
-    ukg_allow_dynamic_smem((const void*)CK.weigh);
+    if (CK.weigh) ukg_allow_dynamic_smem((const void*)CK.weigh);
     ukg_allow_dynamic_smem((const void*)CK.pair);
     ukg_allow_dynamic_smem((const void*)CK.tail);
     if (CK.solve) ukg_allow_dynamic_smem((const void*)CK.solve);
@@ -2627,7 +2627,7 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     const int64_t rmax = std::max(n, p->mmax);
     const int64_t wneed = rmax * rmax + rmax * (2 * n + 1) + rmax * cta::NT;
     if (CK.weigh) {
-      UKG_LAUNCH(kWeigh, st, (CK.weigh<<<(unsigned)p->nsteps, CK.threads3, CK.weigh_smem, st>>>(a, raw)));
+      UKG_LAUNCH(kWeigh, st, (CK.weigh<<<(unsigned)p->nsteps, CK.weigh_threads, CK.weigh_smem, st>>>(a, raw)));
     } else if (2 * wneed <= a.scratch_per_cta) {
       a.scratch_per_cta /= 2;
       const unsigned g2 = (unsigned)std::max<int64_t>(1, std::min<int64_t>(p->nsteps, 2 * (int64_t)ncta));
@@ -2635,6 +2635,7 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     } else {
       UKG_LAUNCH(kWeigh, st, (ctak::weigh_cta<T><<<grid(p->nsteps), cta::NT, 0, st>>>(a, raw, p->nsteps)));
     }
+    if (CK.tri) UKG_LAUNCH(kWeigh, st, (CK.tri<<<(unsigned)p->nsteps, CK.tri_threads, 0, st>>>(a)));
     if constexpr (sizeof(T) == sizeof(float))
       if (WK.pair)
         UKG_LAUNCH(kWeigh, st, (WK.triangularize<<<(unsigned)((p->nsteps + 1) / 2), wide::NT, WK.smem, st>>>(a, p->nsteps)));
@@ -2678,7 +2679,7 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     common(a, l);
     if (lp[l].nsolve == 0) continue;
     if (CK.solve && want_cov)
-      UKG_LAUNCH(kSolve, st, (CK.solve<<<(unsigned)lp[l].nsolve, CK.threads3, ck_solve, st>>>(a)));
+      UKG_LAUNCH(kSolve, st, (CK.solve<<<(unsigned)lp[l].nsolve, CK.solve_threads, ck_solve, st>>>(a)));
     else if (CK.state && !want_cov)
       UKG_LAUNCH(kSolve, st, (CK.state<<<(unsigned)((lp[l].nsolve + 3) / 4), 128, 0, st>>>(a)));
     else

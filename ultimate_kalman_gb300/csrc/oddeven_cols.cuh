@@ -12,9 +12,9 @@
  * few items a level it is the chain of 2 n reflectors, 50 us.  Measured, ms,
  * pairs / back-substitution / weighing, before and now:
  *   16 tracks of 64 to 4,000 steps, n = 12  FP64   7.2 2.0 1.5    2.2 1.1 0.7
- *   2,000 steps, n = 48                     FP64   22.7 8.4 1.6   12.0 6.3 2.2
- *                                           df     16.6 9.9 1.0   5.7 6.6 1.8
- *   4,000 steps, n = 64, states             FP32   8.9 1.0 1.5    4.2 0.5 3.2
+ *   2,000 steps, n = 48                     FP64   22.7 8.4 1.6   10.8 6.2 2.3
+ *                                           df     16.6 9.9 1.0   4.9 6.5 1.2
+ *   4,000 steps, n = 64, states             FP32   8.9 1.0 1.5    4.1 0.4 1.7
  * (the weighing now includes the triangularization).
  *
  * Structure.  Every observation block is upper trapezoidal: the weighing
@@ -54,14 +54,14 @@ __host__ __device__ constexpr int threads3() { return (3 * NP + 2 + 31) / 32 * 3
 template <typename T, int NP>
 __host__ __device__ constexpr int blocks()
 {
-  return sizeof(T) == 8 ? (NP <= 12 ? 8 : NP <= 16 ? 6 : NP <= 24 ? 4 : NP <= 32 ? 2 : 1)
-                        : (NP <= 12 ? 12 : NP <= 16 ? 8 : NP <= 24 ? 5 : NP <= 32 ? 4 : NP <= 64 ? 2 : 1);
+  return sizeof(T) == 8 ? (NP <= 12 ? 8 : NP <= 16 ? 6 : NP <= 24 ? 4 : NP <= 40 ? 2 : 1)
+                        : (NP <= 12 ? 12 : NP <= 16 ? 8 : NP <= 24 ? 5 : NP <= 32 ? 4 : 2);
 }
 template <typename T, int NP>
 __host__ __device__ constexpr int blocks3()
 {
-  return sizeof(T) == 8 ? (NP <= 12 ? 8 : NP <= 16 ? 8 : NP <= 24 ? 5 : NP <= 32 ? 3 : NP <= 48 ? 2 : 1)
-                        : (NP <= 12 ? 12 : NP <= 16 ? 12 : NP <= 24 ? 6 : NP <= 32 ? 4 : NP <= 64 ? 2 : 1);
+  return sizeof(T) == 8 ? (NP <= 12 ? 8 : NP <= 16 ? 8 : NP <= 24 ? 5 : NP <= 32 ? 3 : NP <= 56 ? 2 : 1)
+                        : (NP <= 12 ? 12 : NP <= 16 ? 12 : NP <= 24 ? 6 : 4);
 }
 
 /* the fewest states an instantiation is used for; rows below it need no test
@@ -169,47 +169,9 @@ __device__ __forceinline__ void reduce(QrShared<T, NP>& sm, int panel, bool act,
  * level 0: weighing, and the triangularization of [W G | W o].
  * Threads 0..2n: columns of [H | -F | c]; threads 2n+1..3n+1: columns of [G | o].
  * ------------------------------------------------------------------------ */
-/* Lower Cholesky factors of the n x n matrices in L[0] and L[1] (column-major,
- * ld NP + 1; n[f] = 0: none) side by side, reciprocals of the diagonals in d.
- * Column j, scaled, waits in row j of the upper half, which nothing else
- * reads; whoever updates the next diagonal entry takes its root.  *bad is set
- * for a pivot that is not positive (replaced by 1).                          */
-template <typename T, int NP>
-__device__ __forceinline__ void cholesky2(T* const (&L)[2], T* const (&d)[2], const int (&n)[2], int* bad)
-{
-  constexpr int LD = NP + 1, NT = threads3<NP>();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  auto root = [&](int f, int j) {
-    const T s = L[f][j * LD + j];
-    if (!(s > T(0))) *bad = 1;
-    d[f][j] = s > T(0) ? inv_root(s) : T(1);
-  };
-  if (tid < 2 && n[tid] > 0) root(tid, 0);
-  __syncthreads();
-  const int top = n[0] > n[1] ? n[0] : n[1];
-  for (int j = 0; j + 1 < top; ++j) {
-#pragma unroll
-    for (int f = 0; f < 2; ++f)
-      for (int i = j + 1 + tid; i < n[f]; i += NT) L[f][i * LD + j] = L[f][j * LD + i] * d[f][j];
-    __syncthreads();
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      for (int k = j + 1 + warp; k < n[f]; k += NT / 32) {
-        const T lk = L[f][k * LD + j];
-        for (int i = k + lane; i < n[f]; i += 32) {
-          const T v = fma(-L[f][i * LD + j], lk, L[f][k * LD + i]);
-          L[f][k * LD + i] = v;
-          if (i == j + 1) root(f, j + 1);
-        }
-      }
-      for (int i = j + 1 + tid; i < n[f]; i += NT) L[f][j * LD + i] = L[f][i * LD + j];
-    }
-    __syncthreads();
-  }
-}
-
-/* The same for n <= 32 by one warp, row i on lane i, in registers; L and d in
- * shared memory as above (row i of the factor from lane i)                   */
+/* Lower Cholesky factor of the n x n matrix in L (column-major, ld NP + 1) by one
+ * warp, row i on lane i, in registers, the reciprocals of the diagonal in d;
+ * *bad is set for a pivot that is not positive (replaced by 1)               */
 template <typename T>
 __device__ __forceinline__ T bcast(T v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 template <>
@@ -290,17 +252,11 @@ __global__ void __launch_bounds__(threads3<NP>(), blocks3<T, NP>()) weigh_cols(C
   if (evol) fetch(kt, raw.K + g * nn, n, n, Lk, dk);
   if (m > 0) fetch(ct, raw.C + g * (int64_t)mm * mm, mm, m, Lc, dc);
   __syncthreads();
-  {
-    T* const L2[2] = {Lk, Lc};
-    T* const d2[2] = {dk, dc};
-    const int n2[2] = {evol && kt == 'C' ? n : 0, m > 0 && ct == 'C' ? m : 0};
-    if constexpr (NP <= 32) { /* K's factor in the first warp, C's in the second */
-      const int f = tid >> 5;
-      if (f < 2 && n2[f] > 0) cholesky_warp<T, NP>(L2[f], d2[f], n2[f], &bad);
-      __syncthreads();
-    } else if (n2[0] + n2[1] > 0) {
-      cholesky2<T, NP>(L2, d2, n2, &bad);
-    }
+  { /* K's factor in the first warp, C's in the second */
+    const bool second = tid >= 32;
+    if (tid < 64 && (second ? m > 0 && ct == 'C' : evol && kt == 'C'))
+      cholesky_warp<T, NP>(second ? Lc : Lk, second ? dc : dk, second ? m : n, &bad);
+    __syncthreads();
   }
   if (tid == 0) a.ce.m[q] = m;
   if (tid == 0 && bad) flag |= 1;
@@ -366,6 +322,29 @@ __global__ void __launch_bounds__(threads3<NP>(), blocks3<T, NP>()) weigh_cols(C
   T* out = tid < n ? &a.ce.G.at(tid * a.mx, q) : &a.ce.o.at(0, q);
   reduce<T, NP>(sm, 0, act, tid, m, 0, steps, steps, b, [](int) { return T(0); },
                 [&](int k, T v) { out[k] = tid < n && k > tid ? T(0) : v; });
+}
+/* Above 32 states ctak::weigh_cta weighs: a block a step here is one or two an
+ * SM, whose chain of n pivots and n reflectors nothing hides (6,400 steps, n = 49,
+ * m = 24: 14.2 ms, double-float 11.6; apart 7.2 and 4.3).
+ * Then the observations alone are triangularized.                            */
+template <int NP>
+__host__ __device__ constexpr int tri_threads() { return (NP + 1 + 31) / 32 * 32; }
+template <typename T, int NP>
+__global__ void __launch_bounds__(tri_threads<NP>(), sizeof(T) == 8 ? (NP <= 48 ? 6 : 4) : (NP <= 48 ? 8 : 5))
+    triangularize(CArgs<T> a)
+{
+  __shared__ QrShared<T, NP> sm;
+  const int n = a.n, tid = threadIdx.x;
+  const int64_t g = blockIdx.x;
+  const int t = find_track(a.track_start, a.ntracks, g);
+  const int64_t q = a.ct.slot[t] + (g - a.track_start[t]);
+  const int m = a.ce.m[q], steps = m < n ? m : n;
+  const bool act = tid <= n;
+  T* col = tid < n ? &a.ce.G.at(tid * a.mx, q) : &a.ce.o.at(0, q);
+  T b[NP];
+  load_rows<T, NP>(col, m, act, b);
+  reduce<T, NP>(sm, 0, act, tid, n, 0, steps, steps, b, [](int) { return T(0); },
+                [&](int k, T v) { col[k] = tid < n && k > tid ? T(0) : v; });
 }
 template <typename T, int NP>
 constexpr size_t weigh_smem() { return (size_t)(2 * NP * (NP + 1) + 2 * NP + (NP + 1) * NP) * sizeof(T); }
@@ -563,9 +542,10 @@ __global__ void __launch_bounds__(threads3<NP>(), blocks3<T, NP>()) solve_cols(C
   const int n = a.n, tid = threadIdx.x, nn = n * n;
   T* B = (T*)dyn;      /* [F~ | Y], column-major */
   T* R = B + 2 * nn;   /* column-major */
-  T* W = R + nn;       /* column-major, n x 2n; then M's columns are read from M */
-  T* M = W + 2 * nn;
-  T* dv = M + nn;
+  T* W = R + nn;       /* column-major, n x 2n; then X */
+  T* M = W + 2 * nn;   /* its lower triangle, column by column */
+  T* dv = M + n * (n + 1) / 2;
+  auto at_m = [&](int i, int c) { return c * n - c * (c - 1) / 2 + i - c; }; /* i >= c */
   const auto& Rr = a.cr;
   const int64_t item = blockIdx.x;
   const int t = find_track(a.ct.solve, a.ntracks, item);
@@ -656,20 +636,25 @@ __global__ void __launch_bounds__(threads3<NP>(), blocks3<T, NP>()) solve_cols(C
     if ((q1 - q0) & 1) s0 = fma(W[(q1 - 1) * n + i], B[(q1 - 1) * n + c], s0);
     T m = s0 + s1;
     if (i == c) m += T(1);
-    M[c * n + i] = M[i * n + c] = m;
+    M[at_m(i, c)] = m;
   }
-  __syncthreads();
+  __syncthreads(); /* W is in registers: X goes there */
   const int mc = tid - (2 * n + 1);
   const bool isM = mc >= 0 && mc < n;
-  if (isM) load_end<T, NP>(M + mc * n, n, true, b);
-  __syncthreads(); /* M's columns are in registers: X goes there */
+  T* X = W;
+  if (isM)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int r = i - NP + n;
+      b[i] = r < 0 ? T(0) : M[r >= mc ? at_m(r, mc) : at_m(mc, r)];
+    }
   {
     /* one substitution for the blocks -R^{-1} W, the state and X = R^{-1} M: the
        columns differ by where they go.  cov(x_{j-1}, x_j): row q of U;
        cov(x_j, x_{j+1}): column q                                            */
     const bool isU = isW && a.level > 0 && (tid < n ? hp : hn);
-    T* dst = isU ? (tid < n ? &Rr.U.at(q, a.ct.slot[t] + j) : &Rr.U.at(q * n, a.ct.slot[t] + j + 1)) : M + (isM ? mc : 0);
-    const int ds = isU && tid >= n ? 1 : n; /* X goes to M transposed: row mc */
+    T* dst = isU ? (tid < n ? &Rr.U.at(q, a.ct.slot[t] + j) : &Rr.U.at(q * n, a.ct.slot[t] + j + 1)) : X + (isM ? mc : 0);
+    const int ds = isU && tid >= n ? 1 : n; /* X transposed: row mc */
     if (isU || isx || isM)
       back_subst<T, NP>(R, dv, n, b, [&](int r, T v) {
         if (isx) a.state[oj * n + r] = ukg_df::widen(v);
@@ -678,7 +663,7 @@ __global__ void __launch_bounds__(threads3<NP>(), blocks3<T, NP>()) solve_cols(C
   }
   __syncthreads();
   if (isM) {
-    load_end<T, NP>(M + mc * n, n, true, b); /* X^T's column mc */
+    load_end<T, NP>(X + mc * n, n, true, b); /* X^T's column mc */
     double* So = a.cov + oj * nn;
     back_subst<T, NP>(R, dv, n, b, [&](int r, T v) {
       if (r >= mc) {
@@ -690,7 +675,7 @@ __global__ void __launch_bounds__(threads3<NP>(), blocks3<T, NP>()) solve_cols(C
   }
 }
 template <typename T>
-size_t solve_smem(int n) { return (size_t)(6 * n * n + n) * sizeof(T); }
+size_t solve_smem(int n) { return (size_t)(5 * n * n + n * (n + 1) / 2 + n) * sizeof(T); }
 
 /* the state alone, a warp per even step: lanes over the rows (row lane + 32 u) */
 template <typename T, int NP>
@@ -779,26 +764,45 @@ __global__ void __launch_bounds__(128) state_cols(CArgs<T> a)
 /* the kernels of a state dimension: the smallest instantiation that holds it */
 template <typename T>
 struct Kernels {
-  void (*weigh)(CArgs<T>, RawA) = nullptr;
+  void (*weigh)(CArgs<T>, RawA) = nullptr; /* or ctak::weigh_cta and tri */
+  void (*tri)(CArgs<T>) = nullptr;
   void (*pair)(CArgs<T>) = nullptr;
   void (*tail)(CArgs<T>) = nullptr;
   void (*solve)(CArgs<T>) = nullptr;
   void (*state)(CArgs<T>) = nullptr;
-  int threads = 0, threads3 = 0;
+  int threads = 0, weigh_threads = 0, tri_threads = 0, solve_threads = 0;
   size_t weigh_smem = 0;
 };
+template <typename T, int NP>
+void pairs_np(Kernels<T>& k)
+{
+  k.pair = pair_cols<T, NP>;
+  k.tail = tail_cols<T, NP>;
+  k.threads = threads<NP>();
+}
+template <typename T, int NP>
+void solve_np(Kernels<T>& k)
+{
+  if constexpr (sizeof(T) == 8) {
+    k.solve = solve_cols<T, NP>;
+    k.solve_threads = threads3<NP>();
+  }
+}
 template <typename T, int NP>
 Kernels<T> kernels_np()
 {
   Kernels<T> k;
-  k.weigh = weigh_cols<T, NP>;
-  k.pair = pair_cols<T, NP>;
-  k.tail = tail_cols<T, NP>;
-  if constexpr (sizeof(T) == 8) k.solve = solve_cols<T, NP>;
+  if constexpr (NP <= 32) {
+    k.weigh = weigh_cols<T, NP>;
+    k.weigh_threads = threads3<NP>();
+    k.weigh_smem = weigh_smem<T, NP>();
+  } else {
+    k.tri = triangularize<T, NP>;
+    k.tri_threads = tri_threads<NP>();
+  }
+  pairs_np<T, NP>(k);
+  solve_np<T, NP>(k);
   k.state = state_cols<T, NP>;
-  k.threads = threads<NP>();
-  k.threads3 = threads3<NP>();
-  k.weigh_smem = weigh_smem<T, NP>();
   return k;
 }
 template <typename T>
@@ -809,10 +813,21 @@ Kernels<T> kernels(int n, int mx)
   if (n <= 16) return kernels_np<T, 16>();
   if (n <= 24) return kernels_np<T, 24>();
   if (n <= 32) return kernels_np<T, 32>();
-  if (n <= 48) return kernels_np<T, 48>();
-  if (n <= 64) return kernels_np<T, 64>();
-  Kernels<T> k; /* above, the states' back-substitution alone */
-  k.state = state_cols<T, 128>;
+  Kernels<T> k;
+  if (n <= 64) {
+    k = n <= 48 ? kernels_np<T, 48>() : kernels_np<T, 64>();
+    /* Registers (and shared memory) for two blocks an SM instead of one: 64
+       tracks of 100 steps, n = 33, FP64, pairs 14.7 -> 10.0 ms (19.0 -> 12.8 at
+       n = 40); n = 49, even steps 19.2 -> 13.0, double-float 25.5 -> 14.3.  The
+       pairs of 41 states and more would spill, the even steps of 51 and more do
+       not fit the shared memory twice.                                       */
+    if constexpr (sizeof(T) == 8) {
+      if (n <= 40) pairs_np<T, 40>(k), solve_np<T, 40>(k);
+      if (n > 48 && n <= 50) solve_np<T, 56>(k);
+    }
+    return k;
+  }
+  k.state = state_cols<T, 128>; /* above, the states' back-substitution alone */
   return k;
 }
 
