@@ -71,3 +71,35 @@ def test_upper_levels_in_one_launch(n, k, sweeps):
         Xb, _ = native.smooth(P.select_tracks([0] * T), "oddeven", covariance=False, fp32_refine=True, sweeps=sweeps)
         for t in (0, T - 1):
             np.testing.assert_array_equal(Xb[k * t:k * t + k], X, err_msg=f"{T} tracks")
+
+
+@pytest.mark.parametrize("n,m,cov,missing", [(2, 2, "C", 0.0), (3, 1, "W", 0.3), (4, 2, "C", 0.1), (5, 5, "w", 0.2),
+                                             (6, 3, "F", 0.0), (6, 6, "C", 0.4), (8, 4, "C", 0.2)])
+def test_many_tails_same_bits(n, m, cov, missing):
+    """Tracks of odd length at a level: a warp each, up to 6 states a thread each
+    past 4,864 of them (level 0: 7,500 here, level 1: 5,000), with the same bits
+    in FP64, double-float and FP32."""
+    P = pb.random_dynamics([1, 2, 3, 5], n, m, seed=20 * n + m, K_type=cov, C_type=cov, missing=missing, per_step=True)
+    B = P.select_tracks([0, 1, 2, 3] * 2500)
+    k = P.nsteps
+    st, Xo, So = oracle.smooth(P, "oddeven")
+    assert st == 0
+    for kw, tol in ((dict(), 1e-11), (dict(fp32_refine=True), 1e-9), (dict(fp32_refine=True, covariance=False), 1e-9)):
+        X, S = native.smooth(P, "oddeven", **kw)
+        assert oracle.rel_err_states(X, Xo) < tol
+        assert S is None or oracle.rel_err_covs(S, So) < tol
+        Xb, Sb = native.smooth(B, "oddeven", **kw)
+        for t in (0, 1249, 2499):
+            np.testing.assert_array_equal(Xb[k * t:k * t + k], X)
+            if S is not None:
+                np.testing.assert_array_equal(Sb[k * t:k * t + k], S)
+
+
+def test_many_unobservable_tails_are_reported():
+    P = pb.random_dynamics([1, 3], 4, 1, seed=2, fold=False)
+    P.obs_rows[1:] = 0
+    B = P.select_tracks([0, 1] * 3000)
+    for kw in (dict(), dict(fp32_refine=True)):
+        with pytest.raises(native.KalmanError) as e:
+            native.smooth(B, "oddeven", **kw)
+        assert e.value.status == native.KALMAN_GPU_ESINGULAR

@@ -1985,6 +1985,7 @@ struct SmallKernels {
   void (*pair8)(Args<T, T>) = nullptr;
   void (*pair1)(Args<T, T>) = nullptr; /* null: eight lanes at every larger size */
   void (*tail)(Args<T, T>) = nullptr;
+  void (*tail1)(Args<T, T>) = nullptr; /* null: a warp for any number */
   void (*solve32)(Args<T, T>) = nullptr;
   void (*solve1)(Args<T, T>) = nullptr;
   void (*state)(Args<T, T>) = nullptr;
@@ -2024,6 +2025,11 @@ struct SmallLimits<double> {
   static constexpr int64_t pair32 = 1216, pair8 = 7296, solve32 = 7296;
 };
 
+/* Tails of a level (tracks of odd length) that a warp each takes: eight rounds of
+ * a warp a scheduler, where a thread's chain takes as long (4,000 and 8,000 tracks
+ * of 3 steps by warps, n = 4: tails 82 and 154 us, by threads 8,000 47)         */
+constexpr int64_t kLaneTails = 4864;
+
 template <typename T, int N>
 SmallKernels<T> small_kernels_n(int pair_bs)
 {
@@ -2033,6 +2039,7 @@ SmallKernels<T> small_kernels_n(int pair_bs)
   k.pair_bs = kPairThreadBS;
   if constexpr (std::is_same<T, double>::value && N <= 6) k.pair1 = small::pair_thread<T, N, kPairThreadBS, 2>;
   k.tail = small::tail_lanes<T, N>;
+  if constexpr (N <= 6) k.tail1 = small::tail_thread<T, N>;
   if constexpr (std::is_same<T, float>::value) {
     k.pair_bs = pair_bs;
     constexpr int per_sm = N <= 6 ? 512 : 256; /* threads per SM: 128 or 255 registers each */
@@ -2256,16 +2263,20 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
     if (l + 1 < nlev) a.ne = eqT(l + 1);
     const int64_t np = lp[l].npairs, nt = lp[l].ntail;
     if (SK.pair32) { /* n <= 8: lanes or threads per item */
-      if (np <= SmallLimits<T>::pair32) { /* with the tails */
+      const bool many = SK.tail1 && nt > kLaneTails;
+      if (np <= SmallLimits<T>::pair32 && !many) { /* with the tails */
         if (np + nt > 0)
           UKG_LAUNCH(kPair, st, (SK.pair32<<<grid(np + nt, lw), lt, 0, st>>>(a)));
         continue;
       }
-      if (np <= SmallLimits<T>::pair8 || !SK.pair1)
+      if (np > 0 && (np <= SmallLimits<T>::pair8 || !SK.pair1))
         UKG_LAUNCH(kPair, st, (SK.pair8<<<grid(np, 4 * lw), lt, 0, st>>>(a)));
-      else
+      else if (np > 0)
         UKG_LAUNCH(kPair, st, (SK.pair1<<<grid(np, SK.pair_bs), SK.pair_bs, 0, st>>>(a)));
-      if (nt > 0) UKG_LAUNCH(kTail, st, (SK.tail<<<grid(nt, lw), lt, 0, st>>>(a)));
+      if (many)
+        UKG_LAUNCH(kTail, st, (SK.tail1<<<grid(nt, small::kTailThreadBS), small::kTailThreadBS, 0, st>>>(a)));
+      else if (nt > 0)
+        UKG_LAUNCH(kTail, st, (SK.tail<<<grid(nt, lw), lt, 0, st>>>(a)));
       continue;
     }
     if (np > 0) UKG_LAUNCH(kPair, st, (pair_kernel<T, T><<<grid(np, bp), bp, bp * pt_pair, st>>>(a, rmax)));

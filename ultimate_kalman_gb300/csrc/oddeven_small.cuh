@@ -385,9 +385,10 @@ __device__ __forceinline__ void thread_qr_tri(T (&t)[N][N], T (&x)[N][N], T (&am
 {
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    T tail = T(0);
+    Dot<T> sq;
 #pragma unroll
-    for (int i = 0; i < N; ++i) tail = fma(x[k][i], x[k][i], tail);
+    for (int i = 0; i < N; ++i) sq.add(x[k][i], x[k][i]);
+    const T tail = sq.value();
     am[k] = iv[k] = T(0);
     if (tail == T(0)) continue;
     const Refl<T> r = reflector(t[k][k], tail);
@@ -396,10 +397,10 @@ __device__ __forceinline__ void thread_qr_tri(T (&t)[N][N], T (&x)[N][N], T (&am
     iv[k] = r.inv;
 #pragma unroll
     for (int c = k + 1; c < N; ++c) {
-      T d = T(0); /* FP64: as Dot */
+      Dot<T> xa;
 #pragma unroll
-      for (int i = 0; i < N; ++i) d = fma(x[k][i], x[c][i], d);
-      d = fma(r.amb, t[c][k], d) * r.inv;
+      for (int i = 0; i < N; ++i) xa.add(x[k][i], x[c][i]);
+      const T d = fma(r.amb, t[c][k], xa.value()) * r.inv;
       t[c][k] = fma(-d, r.amb, t[c][k]);
 #pragma unroll
       for (int i = 0; i < N; ++i) x[c][i] = fma(-d, x[k][i], x[c][i]);
@@ -412,10 +413,10 @@ __device__ __forceinline__ void thread_apply_tri(const T (&x)[N][N], const T (&a
 {
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    T d = T(0);
+    Dot<T> xa;
 #pragma unroll
-    for (int i = 0; i < N; ++i) d = fma(x[k][i], cb[i], d);
-    d = fma(am[k], ct[k], d) * iv[k];
+    for (int i = 0; i < N; ++i) xa.add(x[k][i], cb[i]);
+    const T d = fma(am[k], ct[k], xa.value()) * iv[k];
     ct[k] = fma(-d, am[k], ct[k]);
 #pragma unroll
     for (int i = 0; i < N; ++i) cb[i] = fma(-d, x[k][i], cb[i]);
@@ -429,9 +430,10 @@ __device__ __forceinline__ void thread_qr_full(T (&p)[N][R], T (&am)[N], T (&iv)
   for (int k = 0; k < N; ++k) {
     am[k] = iv[k] = T(0);
     if (k >= R) continue;
-    T tail = T(0);
+    Dot<T> sq;
 #pragma unroll
-    for (int i = k + 1; i < R; ++i) tail = fma(p[k][i], p[k][i], tail);
+    for (int i = k + 1; i < R; ++i) sq.add(p[k][i], p[k][i]);
+    const T tail = sq.value();
     if (tail == T(0) || k >= nref) continue;
     const Refl<T> r = reflector(p[k][k], tail);
     p[k][k] = r.beta;
@@ -439,10 +441,10 @@ __device__ __forceinline__ void thread_qr_full(T (&p)[N][R], T (&am)[N], T (&iv)
     iv[k] = r.inv;
 #pragma unroll
     for (int c = k + 1; c < N; ++c) {
-      T d = T(0);
+      Dot<T> xa;
 #pragma unroll
-      for (int i = k + 1; i < R; ++i) d = fma(p[k][i], p[c][i], d);
-      d = fma(r.amb, p[c][k], d) * r.inv;
+      for (int i = k + 1; i < R; ++i) xa.add(p[k][i], p[c][i]);
+      const T d = fma(r.amb, p[c][k], xa.value()) * r.inv;
       p[c][k] = fma(-d, r.amb, p[c][k]);
 #pragma unroll
       for (int i = k + 1; i < R; ++i) p[c][i] = fma(-d, p[k][i], p[c][i]);
@@ -455,10 +457,10 @@ __device__ __forceinline__ void thread_apply_full(const T (&p)[N][R], const T (&
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     if (k >= R) continue;
-    T d = T(0);
+    Dot<T> xa;
 #pragma unroll
-    for (int i = k + 1; i < R; ++i) d = fma(p[k][i], c[i], d);
-    d = fma(am[k], c[k], d) * iv[k];
+    for (int i = k + 1; i < R; ++i) xa.add(p[k][i], c[i]);
+    const T d = fma(am[k], c[k], xa.value()) * iv[k];
     c[k] = fma(-d, am[k], c[k]);
 #pragma unroll
     for (int i = k + 1; i < R; ++i) c[i] = fma(-d, p[k][i], c[i]);
@@ -682,6 +684,206 @@ __global__ void __launch_bounds__(BS, MINB) pair_thread(Args<T, T> a)
     else thread_c_full<T, N, 2 * N>(a, I);
     Nx.m[I.sn] = rC < N ? rC : N;
   }
+}
+
+/* ---------------------------------------------------------------------------
+ * odd-length tracks by one thread each, the operations of tail_item: for levels
+ * that end many tracks.  A warp a tail is 32 lanes for 2 N + 1 columns, and
+ * thousands of tracks of a few steps are little but tails: 20,000 tracks of 3
+ * steps, FP64, n = 4, the tails of both levels (with the pairs' launch) 461 us
+ * before, 126 now, n = 6 880 and 297.
+ * ------------------------------------------------------------------------ */
+constexpr int kTailThreadBS = 64;
+
+template <typename T, int N>
+__device__ __forceinline__ void load_cols(const Soa<T>& first, int e, int64_t s, int rows, T (&p)[N][N])
+{
+#pragma unroll
+  for (int c = 0; c < N; ++c)
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[c][i] = i < rows ? first.at(e + c * N + i, s) : T(0);
+}
+
+/* x = R^{-1} y, S = R^{-1} R^{-T} of a track's only step */
+template <typename T, int N>
+__device__ __forceinline__ void base_thread(const Args<T, T>& a, int tr, const T (&R)[N][N], T (&y)[N], PVc<T, kTailThreadBS> Ri)
+{
+  const int64_t os = orig_step(a.track_start, a.level, tr, 0);
+  double* x = a.state + os * N;
+  T dv[N];
+  bool bad = false;
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    bad |= R[c][c] == T(0);
+    dv[c] = recip(R[c][c]);
+    if (a.baseR.p)
+#pragma unroll
+      for (int i = 0; i < N; ++i) a.baseR.at(c * N + i, tr) = i <= c ? R[c][i] : T(0);
+  }
+  if (bad) atomicOr(a.flag, 2);
+  auto solve = [&](T (&v)[N], int top) {
+#pragma unroll
+    for (int j = N - 1; j >= 0; --j) {
+      if (j > top) continue;
+      v[j] = v[j] * dv[j];
+#pragma unroll
+      for (int i = 0; i < j; ++i) v[i] = fma(-v[j], R[j][i], v[i]);
+    }
+  };
+  solve(y, N - 1);
+#pragma unroll
+  for (int i = 0; i < N; ++i) x[i] = ukg_df::widen(y[i]);
+  if (!a.cov) return;
+  double* S = a.cov + os * (int64_t)N * N;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    T v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = i == q ? T(1) : T(0);
+    solve(v, q);
+#pragma unroll
+    for (int i = 0; i < N; ++i) Ri[q * N + i] = v[i];
+  }
+#pragma unroll 1
+  for (int j = 0; j < N; ++j)
+#pragma unroll 1
+    for (int i = 0; i < N; ++i) {
+      T sm = T(0);
+      for (int k = i > j ? i : j; k < N; ++k) sm = fma(Ri[k * N + i], Ri[k * N + j], sm);
+      S[j * N + i] = ukg_df::widen(sm);
+    }
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(kTailThreadBS) tail_thread(Args<T, T> a)
+{
+  __shared__ T buf[kTailThreadBS * (N + 1) * N];
+  const PVc<T, kTailThreadBS> Z{buf + threadIdx.x}; /* the rows left over, column by column; or R^{-1} */
+  const int64_t item = (int64_t)blockIdx.x * kTailThreadBS + threadIdx.x;
+  if (item >= a.ct.ntail) return;
+  using K = Col<N>;
+  const int tr = (int)a.ct.tail[item];
+  const Soa<T>&C = a.ce.F, &Nx = a.ne.F, &Rr = a.cr.R;
+  const int64_t L = a.ct.L[tr], s = a.ct.slot[tr] + L - 1;
+  const int mt = a.ce.m[s];
+  T p[N][N], v[N], am[N], iv[N];
+  load_cols<T, N>(C, K::G, s, mt, p);
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = i < mt ? C.at(K::o + i, s) : T(0);
+  if (a.level == 0) {
+    thread_qr_full<T, N, N>(p, am, iv, mt);
+    thread_apply_full<T, N, N>(p, am, iv, v);
+  }
+  if (L == 1) {
+    if (mt < N) {
+      const int64_t os = orig_step(a.track_start, a.level, tr, 0);
+      for (int i = 0; i < N; ++i) a.state[os * N + i] = NAN;
+      if (a.cov)
+        for (int i = 0; i < N * N; ++i) a.cov[os * N * N + i] = NAN;
+      atomicOr(a.flag, 2);
+    } else {
+      base_thread<T, N>(a, tr, p, v, Z);
+    }
+    return;
+  }
+  const int64_t es = a.ct.solve[tr] + (L - 1) / 2, sn = a.nt.slot[tr] + L / 2 - 1;
+  const bool tri = mt == N;
+  T q[N][N], w[N];
+  load_cols<T, N>(C, K::H, s, N, q);
+#pragma unroll
+  for (int i = 0; i < N; ++i) w[i] = C.at(K::c + i, s);
+#pragma unroll
+  for (int c = 0; c < N; ++c)
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i > c || i >= mt) p[c][i] = T(0);
+  /* [R~ | o' | 0; H_s | c_s | F_s], or H_s on top of the mt rows of R~ */
+  if (tri) {
+    thread_qr_tri<T, N>(p, q, am, iv);
+    thread_apply_tri<T, N>(q, am, iv, v, w);
+#pragma unroll
+    for (int i = 0; i < N; ++i) Rr.at(K::rhs + i, es) = v[i], Z[N * N + i] = w[i];
+#pragma unroll 1
+    for (int c = 0; c < N; ++c) {
+      T ft[N], fb[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) ft[i] = T(0), fb[i] = C.at(K::F + c * N + i, s);
+      thread_apply_tri<T, N>(q, am, iv, ft, fb);
+#pragma unroll
+      for (int i = 0; i < N; ++i) Rr.at(K::Ft + c * N + i, es) = ft[i], Z[c * N + i] = fb[i];
+    }
+  } else {
+    T g[N][2 * N], u[2 * N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      u[i] = w[i], u[N + i] = v[i];
+#pragma unroll
+      for (int c = 0; c < N; ++c) g[c][i] = q[c][i], g[c][N + i] = p[c][i];
+    }
+    thread_qr_full<T, N, 2 * N>(g, am, iv, N);
+    thread_apply_full<T, N, 2 * N>(g, am, iv, u);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      Rr.at(K::rhs + i, es) = u[i], Z[N * N + i] = u[N + i];
+#pragma unroll
+      for (int c = 0; c < N; ++c) p[c][i] = g[c][i];
+    }
+#pragma unroll 1
+    for (int c = 0; c < N; ++c) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) u[i] = C.at(K::F + c * N + i, s), u[N + i] = T(0);
+      thread_apply_full<T, N, 2 * N>(g, am, iv, u);
+#pragma unroll
+      for (int i = 0; i < N; ++i) Rr.at(K::Ft + c * N + i, es) = u[i], Z[c * N + i] = u[N + i];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < N; ++c)
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      Rr.at(K::R + c * N + i, es) = i <= c ? p[c][i] : T(0);
+      Rr.at(K::Y + c * N + i, es) = T(0);
+    }
+  /* fix-up: [G~ | o; Z | o''], mt rows of Z; stacked without a gap unless both are full */
+  const int gp = a.ne.m[sn], rF = gp + mt, nF = rF < N ? rF : N;
+  if (tri && gp == N) {
+    load_cols<T, N>(Nx, K::G, sn, N, p);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      v[i] = Nx.at(K::o + i, sn), w[i] = Z[N * N + i];
+#pragma unroll
+      for (int c = 0; c < N; ++c) q[c][i] = Z[c * N + i];
+    }
+    thread_qr_tri<T, N>(p, q, am, iv);
+    thread_apply_tri<T, N>(q, am, iv, v, w);
+  } else {
+    T g[N][2 * N], u[2 * N];
+#pragma unroll
+    for (int c = 0; c <= N; ++c)
+#pragma unroll
+      for (int r = 0; r < 2 * N; ++r) {
+        T x = T(0);
+        if (r < gp) x = Nx.at((c < N ? K::G + c * N : K::o) + r, sn);
+        else if (r < rF) x = Z[c * N + r - gp];
+        (c < N ? g[c < N ? c : 0][r] : u[r]) = x;
+      }
+    thread_qr_full<T, N, 2 * N>(g, am, iv, nF);
+    thread_apply_full<T, N, 2 * N>(g, am, iv, u);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      v[i] = u[i];
+#pragma unroll
+      for (int c = 0; c < N; ++c) p[c][i] = g[c][i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < nF) {
+      Nx.at(K::o + i, sn) = v[i];
+#pragma unroll
+      for (int c = 0; c < N; ++c) Nx.at(K::G + c * N + i, sn) = i <= c ? p[c][i] : T(0);
+    }
+  a.ne.m[sn] = nF;
 }
 
 /* ---------------------------------------------------------------------------
