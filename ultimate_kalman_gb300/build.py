@@ -21,6 +21,14 @@ LIB = os.path.join(HERE, "libukgpu.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["oddeven.cu", "associative.cu", "builder.cu", "filter.cu", "profiling.cu", "host_api.cpp", "matrix_ops.c"]
+# oddeven.cu's kernels by arithmetic type, a compilation each
+PARTS = {"oddeven.cu": [("f32", "float"), ("f64", "double"), ("df", "ukg_df::dd")]}
+# --split-compile=0: nvcc optimizes a translation unit's kernels in parallel on every
+# core.  That gives other registers and spills at every build of the same source (the
+# residual of 6 states took 46 or 63 us), and slower FP32 and double-float pairs (8.8
+# instead of 8.1 ms at 128 states), so those two are compiled without; the FP64
+# back-substitutions and scans are 15 to 25 % faster with it, build after build.
+SPLIT = ["--split-compile=0"]
 
 
 def nvcc():
@@ -30,13 +38,12 @@ def nvcc():
     raise FileNotFoundError("nvcc not found")
 
 
-def _compile(src, verbose):
-    out = os.path.join(BUILD, os.path.basename(src) + ".o")
+def _compile(unit, verbose):
+    src, name, flags = unit
+    out = os.path.join(BUILD, name + ".o")
     inc = ["-I", os.path.join(REPO, "include"), "-I", CSRC]
     if src.endswith(".cu"):
-        # --split-compile=0: nvcc optimizes the translation unit's kernels in parallel on every core
-        cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "--split-compile=0", "-Xcompiler", "-fPIC", *inc,
-               "-c", src, "-o", out]
+        cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", *inc, *flags, "-c", src, "-o", out]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
     elif src.endswith(".cpp"):
@@ -57,8 +64,14 @@ def build(verbose=False, force=False):
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= max(os.path.getmtime(d) for d in deps):
         return LIB
     os.makedirs(BUILD, exist_ok=True)
-    with cf.ThreadPoolExecutor(max_workers=len(srcs)) as ex:
-        results = list(ex.map(lambda s: _compile(s, verbose), srcs))
+    units = []
+    for src in srcs:
+        name = os.path.basename(src)
+        for tag, t in PARTS.get(name, []):
+            units.append((src, f"{name}.{tag}", [f"-DUKG_NAME={tag}", f"-DUKG_TYPE={t}"] + (SPLIT if tag == "f64" else [])))
+        units.append((src, name, SPLIT if src.endswith(".cu") else []))
+    with cf.ThreadPoolExecutor(max_workers=len(units)) as ex:
+        results = list(ex.map(lambda u: _compile(u, verbose), units))
     if verbose:
         for _, err in results:
             if err:

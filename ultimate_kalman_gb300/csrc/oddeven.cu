@@ -57,6 +57,11 @@
  *   base factors     baseR [n*n][tracks] (refinement only)
  *   outputs          state [nsteps][n], covariance [nsteps][n*n] (caller's layout)
  * Level l slot q of track t is original step track_start[t] + ((q+1) << l) - 1.
+ *
+ * The file is compiled four times, at once: for each arithmetic type (UKG_TYPE, a
+ * run of the kernels, ukg_oddeven_run_<UKG_NAME>) and without one for the host
+ * side, so that no compilation takes longer than a minute or two without nvcc's
+ * --split-compile (build.py says where that is used).
  */
 #include <cuda_runtime.h>
 
@@ -75,6 +80,24 @@
 
 #include "profiling.h"
 #include "ukgpu_internal.h"
+
+/* a smoothing on a prepared plan and workspace, by the arithmetic type */
+struct ukg_oddeven_run {
+  uint32_t options;
+  const kalman_gpu_problem_t* p;
+  cudaStream_t st;
+  const void* plan;                 /* Plan */
+  const int64_t *tab, *tab_dev;     /* the plan tables (run_plan) */
+  char* work;
+  void* scratch;                    /* thread blocks: scratch of per_cta doubles for each of ncta */
+  int64_t per_cta;
+  int ncta;
+  kalman_gpu_tuning_t tune;
+  bool cta, enqueue_only;
+};
+int ukg_oddeven_run_f32(const ukg_oddeven_run& r);
+int ukg_oddeven_run_f64(const ukg_oddeven_run& r);
+int ukg_oddeven_run_df(const ukg_oddeven_run& r);
 
 namespace {
 
@@ -1760,6 +1783,7 @@ struct RegSolves {
   void (*rt_level)(Args<float, float>, Soa<float>, Soa<float>, Soa<float>) = nullptr;
   void (*top)(TopArgs) = nullptr;
 };
+template <typename T> /* T: float, so that the other compilations have none of them */
 RegSolves reg_solves(int n)
 {
   RegSolves r;
@@ -1795,7 +1819,10 @@ struct DfKernels {
   void (*resid)(Args<float, float>, Eq<float>, Soa<float>, int64_t) = nullptr;
   int weigh_bs = kWeighBS;
 };
-DfKernels df_kernels(int n, int mmax, int weigh_bs = kWeighBS)
+/* the shapes that have them */
+bool df_shape(int n, int mmax) { return (n == 6 && (mmax == 2 || mmax == 3 || mmax == 6)) || (n == 4 && (mmax == 2 || mmax == 4)); }
+template <typename T> /* T: float */
+DfKernels df_kernels(int n, int mmax, int weigh_bs)
 {
   DfKernels k;
   const int mx = mmax > n ? mmax : n;
@@ -1812,19 +1839,6 @@ DfKernels df_kernels(int n, int mmax, int weigh_bs = kWeighBS)
 #undef UKG_DF
   if (!k.weigh || !k.resid) k = DfKernels(); /* both or neither */
   return k;
-}
-
-/* Launch tuning (kalman_gpu_set_tuning): process-wide, read once at the
- * start of every call.  Defaults: a thread per item below 9 states, a thread
- * block per item from 9 on; four CTAs per SM; the block sizes the FP32
- * kernels were written for.                                                  */
-kalman_gpu_tuning_t default_tuning() { return kalman_gpu_tuning_t{9, 4, kPairBP, kWeighBS}; }
-std::mutex g_tune_mu;
-kalman_gpu_tuning_t g_tune = default_tuning();
-kalman_gpu_tuning_t tuning_now()
-{
-  std::lock_guard<std::mutex> lock(g_tune_mu);
-  return g_tune;
 }
 
 struct LevelPlan {
@@ -1935,7 +1949,7 @@ size_t build_plan(const kalman_gpu_problem_t* p, bool want_cov, bool fp32, bool 
     /* the per-thread path refines with the double-float residual where it is
        compiled (low parts of the level-0 equations); the CTA path, and the
        per-thread path elsewhere, with the FP64 residual (its two arrays) */
-    if (!cta && df_kernels(n, p->mmax).resid) {
+    if (!cta && df_shape(n, p->mmax)) {
       P.o_eq0lo = take((size_t)P.S0 * eqd * sizeof(float));
     } else { /* the FP64 residual's intermediate arrays */
       P.o_rE = take((size_t)P.S0 * n * sizeof(double));
@@ -2102,7 +2116,7 @@ int finish_plan(cudaStream_t st, int* dflag)
  * (uploaded with cudaMemcpyAsync) */
 template <typename T>
 int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, const Plan& P, const int64_t* tab,
-             char* B, const int64_t* tab_dev = nullptr, bool enqueue_only = false)
+             char* B, const int64_t* tab_dev, bool enqueue_only, const kalman_gpu_tuning_t& tune)
 {
   const int n = p->n, T_ = p->ntracks, nlev = P.nlev;
   const int mx = p->mmax > n ? p->mmax : n;
@@ -2176,7 +2190,6 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
       pick_block(pt_solve, 64, &bs) || pick_block(pt_res, 128, &br))
     return ukg_set_error(KALMAN_GPU_EINVAL, "state dimension %d (observation rows %d) needs more shared memory per "
                          "thread than this build's odd-even kernels use", n, mx);
-  const kalman_gpu_tuning_t tune = tuning_now();
   ukg_allow_dynamic_smem((const void*)weigh_kernel<T>);
   if (staged)
     ukg_allow_dynamic_smem((const void*)weigh_staged_kernel<T>);
@@ -2194,7 +2207,7 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
 
   /* double-float level-0 weighing and refinement residual where compiled */
   DfKernels DK;
-  if constexpr (sizeof(T) == sizeof(float)) DK = df_kernels(n, p->mmax, tune.weigh_block);
+  if constexpr (sizeof(T) == sizeof(float)) DK = df_kernels<T>(n, p->mmax, tune.weigh_block);
   const bool use_df = DK.resid != nullptr && P.refine && P.o_eq0lo != 0;
   if (!use_df) DK = DfKernels();
   if (P.refine && !use_df && (P.o_rE == 0 || P.o_rO == 0)) /* offset 0 is the tables: never write there */
@@ -2202,7 +2215,7 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
   Eq<float> eq0lo;
   memset(&eq0lo, 0, sizeof(eq0lo));
   RegSolves RS; /* register-resident FP32 solves where compiled */
-  if constexpr (sizeof(T) == sizeof(float)) RS = reg_solves(n);
+  if constexpr (sizeof(T) == sizeof(float)) RS = reg_solves<T>(n);
   if (use_df) eq0lo = eq_at<float>(B, P.o_eq0lo, P.o_m0, P.S0, n, mx);
 
   /* ---- level 0: weighing ---- */
@@ -2413,87 +2426,6 @@ int run_plan(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, c
   return enqueue_only ? 0 : finish_plan(st, dflag);
 }
 
-/* cached device workspace and plan tables of the ordinary entry point */
-struct Workspace {
-  int device = -1;
-  void* dev = nullptr;
-  size_t dev_bytes = 0;
-};
-thread_local Workspace tl_ws; /* one cached device arena per host thread */
-
-/* page-locked, device-mapped host buffer for the plan tables (one per host
- * thread; every call waits for its kernels, so the next call may refill it) */
-struct MappedTables {
-  int64_t* host = nullptr;
-  int64_t* dev = nullptr;
-  size_t entries = 0;
-};
-thread_local MappedTables tl_mtab;
-
-int ensure_mapped_tables(size_t entries)
-{
-  MappedTables& m = tl_mtab;
-  if (m.entries < entries) {
-    if (m.host) cudaFreeHost(m.host);
-    m = MappedTables();
-    const size_t want = std::max<size_t>(entries, 1 << 16);
-    cudaError_t e = cudaHostAlloc((void**)&m.host, want * sizeof(int64_t), cudaHostAllocMapped);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&m.dev, m.host, 0);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      if (m.host) cudaFreeHost(m.host);
-      m = MappedTables();
-      return ukg_set_error(KALMAN_GPU_ENOMEM, "page-locked plan tables (%zu entries): %s", entries,
-                           cudaGetErrorString(e));
-    }
-    m.entries = want;
-  }
-  return 0;
-}
-
-/* The workspace grows by stream-ordered allocation on the call's stream
- * (cudaFreeAsync / cudaMallocAsync): cudaFree and cudaMalloc synchronize the
- * whole device, which would stall the calls other host threads have running
- * on their own streams.  Every call synchronizes its stream before returning,
- * so the next call, on any stream, finds the allocation complete.           */
-int ensure_workspace(size_t bytes, void** out, cudaStream_t st)
-{
-  int dev = 0;
-  cudaGetDevice(&dev);
-  Workspace& w = tl_ws;
-  if (w.dev && (w.dev_bytes < bytes || w.device != dev)) {
-    if (w.device == dev) cudaFreeAsync(w.dev, st);
-    else cudaFree(w.dev);
-    w.dev = nullptr;
-    w.dev_bytes = 0;
-  }
-  if (!w.dev) {
-    size_t want = ukg_with_slack(bytes);
-    const cudaError_t e = (cudaError_t)ukg_malloc_async(&w.dev, want, st);
-    if (e != cudaSuccess) {
-      w.dev = nullptr;
-      return ukg_set_error(KALMAN_GPU_ENOMEM, "cudaMalloc of %zu bytes of workspace failed: %s", want,
-                           cudaGetErrorString(e));
-    }
-    w.dev_bytes = want;
-    w.device = dev;
-  }
-  *out = w.dev;
-  return 0;
-}
-
-}  // namespace
-
-extern "C" int64_t ukg_oddeven_workspace_held(void) { return (int64_t)tl_ws.dev_bytes; }
-
-extern "C" void ukg_release_oddeven_workspace(void)
-{
-  if (tl_ws.dev) cudaFree(tl_ws.dev);
-  tl_ws = Workspace();
-  if (tl_mtab.host) cudaFreeHost(tl_mtab.host);
-  tl_mtab = MappedTables();
-}
-
 /* ---------------------------------------------------------------------------
  * larger state dimensions: one CTA per item (oddeven_cta.cuh), FP64
  * ------------------------------------------------------------------------ */
@@ -2501,38 +2433,9 @@ constexpr int kCtaMaxN = 128;
 static_assert(kCtaMaxN <= 32 * ctak::kRtQ && kCtaMaxN <= cta::kMaxCov && 2 * kCtaMaxN <= cta::kMaxPanelRows,
               "CTA kernels: per-lane state registers, covariance and panel buffers");
 
-int64_t cta_scratch_per_cta(int n, int mmax)
-{
-  const int64_t rmax = std::max(n, mmax);
-  const int64_t weigh = rmax * rmax + rmax * (2 * n + 1) + rmax * cta::NT;
-  const int64_t tail = 7 * (int64_t)n * n + 5 * n + (int64_t)std::max(n, mmax) * (n + 1) + n;
-  const int64_t mx = rmax; /* max(n, mmax) */
-  const int64_t pair = std::max(std::max(2 * (int64_t)n * (3 * n + 1), (mx + n) * (2 * n + 1)), 2 * mx * (n + 1));
-  const int64_t solve = 7 * (int64_t)n * n + n;
-  return std::max(std::max(weigh, tail), std::max(pair, solve)) + 32;
-}
-
-/* thread blocks of the CTA kernels' persistent grid: per_sm on every SM */
-int cta_count(int per_sm)
-{
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(sms, 1) * std::max(per_sm, 1);
-}
-
-/* thread per item below tune.cta_min_n states (and up to 8 observation
- * rows), one thread block per item from there on                           */
-bool use_cta(const kalman_gpu_problem_t* p, const kalman_gpu_tuning_t& tune)
-{
-  const int mxp = p->mmax > p->n ? p->mmax : p->n;
-  return p->n >= tune.cta_min_n || mxp > 8;
-}
-
 template <typename T>
 int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t st, const Plan& P,
-                 const int64_t* tab_dev, char* B, void* scratch, int64_t per_cta, int ncta,
-                 bool enqueue_only = false)
+                 const int64_t* tab_dev, char* B, void* scratch, int64_t per_cta, int ncta, bool enqueue_only)
 {
   const int n = p->n, T_ = p->ntracks, nlev = P.nlev;
   const int mx = p->mmax > n ? p->mmax : n;
@@ -2622,7 +2525,8 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
     ukg_allow_dynamic_smem((const void*)CK.tail);
     if (CK.solve) ukg_allow_dynamic_smem((const void*)CK.solve);
   }
-  const wide::Kernels WK = sizeof(T) == sizeof(float) ? wide::kernels(n, mx) : wide::Kernels();
+  wide::Kernels WK;
+  if constexpr (sizeof(T) == sizeof(float)) WK = wide::kernels<T>(n, mx);
   if (WK.pair) {
     ukg_allow_dynamic_smem((const void*)WK.triangularize);
     ukg_allow_dynamic_smem((const void*)WK.pair);
@@ -2772,6 +2676,151 @@ int run_plan_cta(uint32_t options, const kalman_gpu_problem_t* p, cudaStream_t s
   return 0;
 }
 
+}  // namespace
+
+#ifdef UKG_TYPE
+
+#define UKG_RUN_NAME(name) UKG_RUN_NAME2(name)
+#define UKG_RUN_NAME2(name) ukg_oddeven_run_##name
+int UKG_RUN_NAME(UKG_NAME)(const ukg_oddeven_run& r)
+{
+  const Plan& P = *(const Plan*)r.plan;
+  return r.cta ? run_plan_cta<UKG_TYPE>(r.options, r.p, r.st, P, r.tab_dev, r.work, r.scratch, r.per_cta, r.ncta,
+                                        r.enqueue_only)
+               : run_plan<UKG_TYPE>(r.options, r.p, r.st, P, r.tab, r.work, r.tab_dev, r.enqueue_only, r.tune);
+}
+
+#else /* the host side */
+
+namespace {
+
+/* Launch tuning (kalman_gpu_set_tuning): process-wide, read once at the
+ * start of every call.  Defaults: a thread per item below 9 states, a thread
+ * block per item from 9 on; four CTAs per SM; the block sizes the FP32
+ * kernels were written for.                                                  */
+kalman_gpu_tuning_t default_tuning() { return kalman_gpu_tuning_t{9, 4, kPairBP, kWeighBS}; }
+std::mutex g_tune_mu;
+kalman_gpu_tuning_t g_tune = default_tuning();
+kalman_gpu_tuning_t tuning_now()
+{
+  std::lock_guard<std::mutex> lock(g_tune_mu);
+  return g_tune;
+}
+
+/* cached device workspace and plan tables of the ordinary entry point */
+struct Workspace {
+  int device = -1;
+  void* dev = nullptr;
+  size_t dev_bytes = 0;
+};
+thread_local Workspace tl_ws; /* one cached device arena per host thread */
+
+/* page-locked, device-mapped host buffer for the plan tables (one per host
+ * thread; every call waits for its kernels, so the next call may refill it) */
+struct MappedTables {
+  int64_t* host = nullptr;
+  int64_t* dev = nullptr;
+  size_t entries = 0;
+};
+thread_local MappedTables tl_mtab;
+
+int ensure_mapped_tables(size_t entries)
+{
+  MappedTables& m = tl_mtab;
+  if (m.entries < entries) {
+    if (m.host) cudaFreeHost(m.host);
+    m = MappedTables();
+    const size_t want = std::max<size_t>(entries, 1 << 16);
+    cudaError_t e = cudaHostAlloc((void**)&m.host, want * sizeof(int64_t), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&m.dev, m.host, 0);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      if (m.host) cudaFreeHost(m.host);
+      m = MappedTables();
+      return ukg_set_error(KALMAN_GPU_ENOMEM, "page-locked plan tables (%zu entries): %s", entries,
+                           cudaGetErrorString(e));
+    }
+    m.entries = want;
+  }
+  return 0;
+}
+
+/* The workspace grows by stream-ordered allocation on the call's stream
+ * (cudaFreeAsync / cudaMallocAsync): cudaFree and cudaMalloc synchronize the
+ * whole device, which would stall the calls other host threads have running
+ * on their own streams.  Every call synchronizes its stream before returning,
+ * so the next call, on any stream, finds the allocation complete.           */
+int ensure_workspace(size_t bytes, void** out, cudaStream_t st)
+{
+  int dev = 0;
+  cudaGetDevice(&dev);
+  Workspace& w = tl_ws;
+  if (w.dev && (w.dev_bytes < bytes || w.device != dev)) {
+    if (w.device == dev) cudaFreeAsync(w.dev, st);
+    else cudaFree(w.dev);
+    w.dev = nullptr;
+    w.dev_bytes = 0;
+  }
+  if (!w.dev) {
+    size_t want = ukg_with_slack(bytes);
+    const cudaError_t e = (cudaError_t)ukg_malloc_async(&w.dev, want, st);
+    if (e != cudaSuccess) {
+      w.dev = nullptr;
+      return ukg_set_error(KALMAN_GPU_ENOMEM, "cudaMalloc of %zu bytes of workspace failed: %s", want,
+                           cudaGetErrorString(e));
+    }
+    w.dev_bytes = want;
+    w.device = dev;
+  }
+  *out = w.dev;
+  return 0;
+}
+
+int64_t cta_scratch_per_cta(int n, int mmax)
+{
+  const int64_t rmax = std::max(n, mmax);
+  const int64_t weigh = rmax * rmax + rmax * (2 * n + 1) + rmax * cta::NT;
+  const int64_t tail = 7 * (int64_t)n * n + 5 * n + (int64_t)std::max(n, mmax) * (n + 1) + n;
+  const int64_t mx = rmax; /* max(n, mmax) */
+  const int64_t pair = std::max(std::max(2 * (int64_t)n * (3 * n + 1), (mx + n) * (2 * n + 1)), 2 * mx * (n + 1));
+  const int64_t solve = 7 * (int64_t)n * n + n;
+  return std::max(std::max(weigh, tail), std::max(pair, solve)) + 32;
+}
+
+/* thread blocks of the CTA kernels' persistent grid: per_sm on every SM */
+int cta_count(int per_sm)
+{
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::max(sms, 1) * std::max(per_sm, 1);
+}
+
+/* thread per item below tune.cta_min_n states (and up to 8 observation
+ * rows), one thread block per item from there on                           */
+bool use_cta(const kalman_gpu_problem_t* p, const kalman_gpu_tuning_t& tune)
+{
+  const int mxp = p->mmax > p->n ? p->mmax : p->n;
+  return p->n >= tune.cta_min_n || mxp > 8;
+}
+
+int run(bool f32, bool df, const ukg_oddeven_run& r)
+{
+  return f32 ? ukg_oddeven_run_f32(r) : df ? ukg_oddeven_run_df(r) : ukg_oddeven_run_f64(r);
+}
+
+}  // namespace
+
+extern "C" int64_t ukg_oddeven_workspace_held(void) { return (int64_t)tl_ws.dev_bytes; }
+
+extern "C" void ukg_release_oddeven_workspace(void)
+{
+  if (tl_ws.dev) cudaFree(tl_ws.dev);
+  tl_ws = Workspace();
+  if (tl_mtab.host) cudaFreeHost(tl_mtab.host);
+  tl_mtab = MappedTables();
+}
+
 extern "C" int ukg_oddeven_device(uint32_t options, const kalman_gpu_problem_t* p, void* cuda_stream)
 {
   if (p->nsteps == 0) return 0;
@@ -2795,14 +2844,8 @@ extern "C" int ukg_oddeven_device(uint32_t options, const kalman_gpu_problem_t* 
     void* base = nullptr;
     if (int e = ensure_workspace(scratch_off + (size_t)ncta * per * sizeof(double), &base, (cudaStream_t)cuda_stream))
       return e;
-    if (f32)
-      return run_plan_cta<float>(options, p, (cudaStream_t)cuda_stream, P, tl_mtab.dev, (char*)base,
-                                 (char*)base + scratch_off, per, ncta);
-    if (dd)
-      return run_plan_cta<ukg_df::dd>(options, p, (cudaStream_t)cuda_stream, P, tl_mtab.dev, (char*)base,
-                                      (char*)base + scratch_off, per, ncta);
-    return run_plan_cta<double>(options, p, (cudaStream_t)cuda_stream, P, tl_mtab.dev, (char*)base,
-                                (char*)base + scratch_off, per, ncta);
+    return run(f32, dd, ukg_oddeven_run{options, p, (cudaStream_t)cuda_stream, &P, nullptr, tl_mtab.dev, (char*)base,
+                                        (char*)base + scratch_off, per, ncta, tune, true, false});
   }
   const bool dd = (options & KALMAN_GPU_FP32_REFINE) && want_cov; /* double-float with covariances */
   const bool fp32 = (options & KALMAN_GPU_FP32_REFINE) && !dd;
@@ -2814,9 +2857,8 @@ extern "C" int ukg_oddeven_device(uint32_t options, const kalman_gpu_problem_t* 
   build_plan(p, want_cov, fp32, fp32, P, tab, need, false);
   void* base = nullptr;
   if (int e = ensure_workspace(P.bytes, &base, (cudaStream_t)cuda_stream)) return e;
-  if (fp32) return run_plan<float>(options, p, (cudaStream_t)cuda_stream, P, tab, (char*)base, tl_mtab.dev);
-  if (dd) return run_plan<ukg_df::dd>(options, p, (cudaStream_t)cuda_stream, P, tab, (char*)base, tl_mtab.dev);
-  return run_plan<double>(options, p, (cudaStream_t)cuda_stream, P, tab, (char*)base, tl_mtab.dev);
+  return run(fp32, dd, ukg_oddeven_run{options, p, (cudaStream_t)cuda_stream, &P, tab, tl_mtab.dev, (char*)base, nullptr, 0,
+                                       0, tune, false, false});
 }
 
 /* Device bytes the ordinary odd-even entry point caches for problem p under
@@ -2968,8 +3010,9 @@ extern "C" int kalman_gpu_smooth_oddeven_noalloc(uint32_t options, const kalman_
   /* the per-thread kernels at every shape, also n >= 9 or mmax > 8 where the
      ordinary entry point switches to CTA kernels (their per-CTA panels are
      not part of this fixed scratch) */
-  const int status = run_plan<double>(options, p, (cudaStream_t)cuda_stream, P, g_noalloc_tab,
-                                      (char*)g_noalloc_addr[dev]);
+  const int status = run(false, false, ukg_oddeven_run{options, p, (cudaStream_t)cuda_stream, &P, g_noalloc_tab, nullptr,
+                                                       (char*)g_noalloc_addr[dev], nullptr, 0, 0, tuning_now(), false,
+                                                       false});
   ukg_prof_resume(prof);
   return status;
 }
@@ -3067,22 +3110,8 @@ extern "C" kalman_gpu_plan_t* kalman_gpu_plan_create(uint32_t options, const kal
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
   if (e == cudaSuccess) {
     const int prof = ukg_prof_pause(); /* no profiling events inside the graph */
-    int st;
-    if (cta && fp32)
-      st = run_plan_cta<float>(options, p, cs, P, nullptr, (char*)pl->work, (char*)pl->work + scratch_off, per, ncta,
-                               true);
-    else if (cta && dd)
-      st = run_plan_cta<ukg_df::dd>(options, p, cs, P, nullptr, (char*)pl->work, (char*)pl->work + scratch_off, per,
-                                    ncta, true);
-    else if (dd)
-      st = run_plan<ukg_df::dd>(options, p, cs, P, nullptr, (char*)pl->work, nullptr, true);
-    else if (cta)
-      st = run_plan_cta<double>(options, p, cs, P, nullptr, (char*)pl->work, (char*)pl->work + scratch_off, per, ncta,
-                                true);
-    else if (fp32)
-      st = run_plan<float>(options, p, cs, P, nullptr, (char*)pl->work, nullptr, true);
-    else
-      st = run_plan<double>(options, p, cs, P, nullptr, (char*)pl->work, nullptr, true);
+    const int st = run(fp32, dd, ukg_oddeven_run{options, p, cs, &P, nullptr, nullptr, (char*)pl->work,
+                                                 (char*)pl->work + scratch_off, per, ncta, tune, cta, true});
     ukg_prof_resume(prof);
     cudaGraph_t g = nullptr;
     const cudaError_t ee = cudaStreamEndCapture(cs, &g);
@@ -3129,3 +3158,5 @@ extern "C" int kalman_gpu_plan_status(kalman_gpu_plan_t* pl)
   if (hflag & 2) return ukg_set_error(KALMAN_GPU_ESINGULAR, "zero pivot: the smoothing problem is not observable");
   return 0;
 }
+
+#endif /* the host side */

@@ -537,7 +537,8 @@ Kernels kernels_rj(int n)
   k.smem = smem<RJ>(n);
   return k;
 }
-inline Kernels kernels(int n, int mx)
+template <typename T> /* T: float, so that the other arithmetics' compilations have none of them */
+Kernels kernels(int n, int mx)
 {
   if (n != mx || n < 65 || n > 128) return Kernels();
   return n <= 96 ? kernels_rj<24>(n) : kernels_rj<32>(n);
