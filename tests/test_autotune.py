@@ -41,6 +41,25 @@ def test_candidates_follow_the_mapping():
     assert autotune.candidates("cta_min_n", 12, 6, False, True, d) == [9]  # past 8 states: blocks only
 
 
+@pytest.mark.parametrize("n,m,kw,scratch", [
+    (9, 9, {}, False), (12, 6, {}, False), (32, 32, dict(fp32_refine=True), False),  # columns in registers throughout
+    (12, 6, dict(fp32_refine=True, covariance=False), True),  # the FP64 residual
+    (33, 4, {}, True), (48, 24, dict(fp32_refine=True), True), (100, 50, {}, True), (12, 20, {}, True)])
+def test_scratch_where_a_kernel_uses_it(n, m, kw, scratch):
+    """The workspace holds ctas_per_sm blocks' scratch only where a kernel has its panels there."""
+    P = pb.empty_problem(n, max(n, m), [100])
+    s = native.ProblemStruct()
+    s.n, s.mmax, s.ntracks, s.location, s.nsteps = n, max(n, m), 1, native.KALMAN_GPU_DEVICE, 100
+    s.track_start = P.track_start.ctypes.data
+    for f in ("H", "F", "c", "K", "K_type", "G", "o", "C", "C_type", "obs_rows", "state", "covariance"):
+        setattr(s, f, 1)  # only their presence matters
+    bytes_ = []
+    for c in (1, 16):
+        native.set_tuning(ctas_per_sm=c)
+        bytes_.append(native.oddeven_workspace_bytes(s, **dict(dict(covariance=True), **kw)))
+    assert 0 < bytes_[0] and (bytes_[1] > bytes_[0]) == scratch
+
+
 def test_cache_round_trip(tmp_path):
     cache = str(tmp_path / "t.json")
     e = {"key": autotune.class_key(4, 4, [64] * 8, True, False), "tuning": {"cta_min_n": 5, "ctas_per_sm": 4,

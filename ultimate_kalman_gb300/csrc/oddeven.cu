@@ -2804,6 +2804,14 @@ bool use_cta(const kalman_gpu_problem_t* p, const kalman_gpu_tuning_t& tune)
   return p->n >= tune.cta_min_n || mxp > 8;
 }
 
+/* bytes of scratch of the thread-block kernels: none in FP64 and double-float for
+ * 9 to 32 states and no more observation rows, whose kernels (oddeven_cols.cuh)
+ * hold all in registers and shared memory; from 33 on the weighing uses it      */
+size_t cta_scratch_bytes(const kalman_gpu_problem_t* p, bool f32, const kalman_gpu_tuning_t& tune)
+{
+  if (!f32 && p->n >= 9 && p->n <= 32 && p->mmax <= p->n) return 0;
+  return (size_t)cta_count(tune.ctas_per_sm) * cta_scratch_per_cta(p->n, p->mmax) * sizeof(double);
+}
 int run(bool f32, bool df, const ukg_oddeven_run& r)
 {
   return f32 ? ukg_oddeven_run_f32(r) : df ? ukg_oddeven_run_df(r) : ukg_oddeven_run_f64(r);
@@ -2842,7 +2850,7 @@ extern "C" int ukg_oddeven_device(uint32_t options, const kalman_gpu_problem_t* 
     const int64_t per = cta_scratch_per_cta(p->n, p->mmax);
     const size_t scratch_off = align_up(P.bytes, 256);
     void* base = nullptr;
-    if (int e = ensure_workspace(scratch_off + (size_t)ncta * per * sizeof(double), &base, (cudaStream_t)cuda_stream))
+    if (int e = ensure_workspace(scratch_off + cta_scratch_bytes(p, f32, tune), &base, (cudaStream_t)cuda_stream))
       return e;
     return run(f32, dd, ukg_oddeven_run{options, p, (cudaStream_t)cuda_stream, &P, nullptr, tl_mtab.dev, (char*)base,
                                         (char*)base + scratch_off, per, ncta, tune, true, false});
@@ -2904,9 +2912,7 @@ extern "C" int64_t kalman_gpu_oddeven_workspace_bytes(uint32_t options, const ka
     return -1;
   }
   size_t bytes = P.bytes;
-  if (cta)
-    bytes = align_up(P.bytes, 256) +
-            (size_t)cta_count(tune.ctas_per_sm) * cta_scratch_per_cta(p->n, p->mmax) * sizeof(double);
+  if (cta) bytes = align_up(P.bytes, 256) + cta_scratch_bytes(p, f32, tune);
   return (int64_t)ukg_with_slack(bytes);
 }
 
@@ -3094,7 +3100,7 @@ extern "C" kalman_gpu_plan_t* kalman_gpu_plan_create(uint32_t options, const kal
   const int ncta = cta ? cta_count(tune.ctas_per_sm) : 0;
   const int64_t per = cta ? cta_scratch_per_cta(p->n, p->mmax) : 0;
   const size_t scratch_off = align_up(P.bytes, 256);
-  const size_t bytes = cta ? scratch_off + (size_t)ncta * per * sizeof(double) : P.bytes;
+  const size_t bytes = cta ? scratch_off + cta_scratch_bytes(p, fp32, tune) : P.bytes;
   cudaError_t e = cudaMalloc(&pl->work, bytes);
   if (e == cudaSuccess)
     e = cudaMemcpy((char*)pl->work + P.o_tab, tab.data(), need * sizeof(int64_t), cudaMemcpyHostToDevice);
