@@ -261,10 +261,12 @@ int64_t kalman_gpu_workspace_held(void);
  *                item (a step pair, a tail, an even step) instead of one
  *                thread; 1..129 (129: never below 129 states), default 9.
  *                Shapes with more than 8 observation rows always use blocks.
- *   ctas_per_sm  thread blocks per SM of the block-per-item kernels'
- *                persistent grid, 1..16, default 4.
- *   pair_block   threads per block of the FP32 register-tile pair kernel
- *                (precision form, n = 4 and 6): 32, 64 or 128, default 64.
+ *   ctas_per_sm  thread blocks per SM of the persistent grids of the
+ *                block-per-item kernels with panels in global scratch, 1..16,
+ *                default 4 (none of them with 9 to 32 states in FP64 or
+ *                double-float and no more observation rows than states).
+ *   pair_block   threads per block of the FP32 thread-per-pair kernel
+ *                (precision form, n = 2 to 8): 32, 64 or 128, default 64.
  *   weigh_block  steps per block of the double-float weighing kernel
  *                (precision form, n = 4 and 6): 64, 128 or 256, default 128.
  * kalman_gpu_set_tuning(NULL) restores the defaults; values outside these

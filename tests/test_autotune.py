@@ -41,6 +41,23 @@ def test_candidates_follow_the_mapping():
     assert autotune.candidates("cta_min_n", 12, 6, False, True, d) == [9]  # past 8 states: blocks only
 
 
+def test_candidates_reach_a_kernel():
+    d = {"cta_min_n": 9, "ctas_per_sm": 4, "pair_block": 64, "weigh_block": 128}
+    for n in (9, 12, 32):  # panels in registers; the FP32 form's residual has a grid
+        assert autotune.candidates("ctas_per_sm", n, n, False, True, d) == [4]
+        assert autotune.candidates("ctas_per_sm", n, n, True, True, d) == [4]
+        assert autotune.candidates("ctas_per_sm", n, n, True, False, d) == autotune.SPACE["ctas_per_sm"]
+        assert autotune.candidates("ctas_per_sm", n, n + 1, False, True, d) == autotune.SPACE["ctas_per_sm"]
+    for n in (33, 64, 128):
+        assert autotune.candidates("ctas_per_sm", n, n, False, True, d) == autotune.SPACE["ctas_per_sm"]
+    for n in (2, 3, 5, 7, 8):
+        assert autotune.candidates("pair_block", n, n, True, False, d) == [32, 64, 128]
+        assert autotune.candidates("weigh_block", n, n, True, False, d) == [128]
+        assert autotune.candidates("pair_block", n, n + 1, True, False, d) == [64]
+    assert autotune.candidates("weigh_block", 4, 4, True, False, d) == [64, 128, 256]
+    assert autotune.candidates("pair_block", 1, 1, True, False, d) == [64]
+
+
 @pytest.mark.parametrize("n,m,kw,scratch", [
     (9, 9, {}, False), (12, 6, {}, False), (32, 32, dict(fp32_refine=True), False),  # columns in registers throughout
     (12, 6, dict(fp32_refine=True, covariance=False), True),  # the FP64 residual

@@ -2,10 +2,11 @@
 
 The library exposes its launch choices as kalman_gpu_tuning_t
 (include/kalman_gpu.h): whether a work item (step pair, tail, even step) goes
-to one thread or to one thread block (cta_min_n), how many blocks per SM the
-block-per-item kernels' persistent grid keeps (ctas_per_sm), and the block
-sizes of the precision form's register-tile pair kernel (pair_block) and
-double-float weighing kernel (weigh_block).  Which choice is fastest depends
+to one thread (or a few lanes) or to one thread block (cta_min_n), how many
+blocks per SM the persistent grids of the block-per-item kernels with panels in
+global scratch keep (ctas_per_sm), and the block sizes of the precision form's
+thread-per-pair kernel (pair_block) and double-float weighing kernel
+(weigh_block).  Which choice is fastest depends
 on the problem class -- state dimension, observation rows, precision, whether
 covariances are wanted, and how much parallel work the tracks offer -- so
 this module measures them on the GPU and keeps the winners.
@@ -16,8 +17,8 @@ tune() times the candidates by coordinate descent (every value of one knob
 with the others fixed at the best so far, knobs in turn, until a full pass
 changes nothing), each candidate as the mean of `reps` smoothings after a
 warm-up, with CUDA events on the launching stream; knobs that cannot affect
-the class (the FP32 block sizes in FP64, the grid in the thread mapping) are
-not searched.  The result and the whole table go into a JSON cache
+the class (the FP32 block sizes in FP64, the grid in the thread mapping and
+where every kernel keeps its panels in registers) are not searched.  The result and the whole table go into a JSON cache
 (tuning_gb300.json beside this file), which apply() reads.  The reference's
 only tuning knob is the TBB grain (c/parallel_tbb.cpp:31,39-43, set through
 parallel_set_blocksize, c/parallel.h:31-32).
@@ -57,9 +58,12 @@ def candidates(knob, n, mmax, fp32_refine, covariance, current):
     blocks = current["cta_min_n"] <= n or not thread_ok
     if knob == "cta_min_n":
         return [n + 1, n] if thread_ok else [current["cta_min_n"]]
-    if knob == "ctas_per_sm":
-        return SPACE[knob] if blocks else [current[knob]]
-    fp32_thread = fp32_refine and not covariance and not blocks and n == max(n, mmax) and n in (4, 6)
+    fp32 = fp32_refine and not covariance
+    if knob == "ctas_per_sm":  # 9 to 32 states: the FP32 form's residual alone has a persistent grid
+        columns = 9 <= n <= 32 and mmax <= n and not fp32
+        return SPACE[knob] if blocks and not columns else [current[knob]]
+    # the thread-per-pair kernel from 2 states on, the double-float weighing at 4 and 6
+    fp32_thread = fp32 and not blocks and mmax <= n and n in (range(2, 9) if knob == "pair_block" else (4, 6))
     return SPACE[knob] if fp32_thread else [current[knob]]
 
 

@@ -2695,9 +2695,9 @@ int UKG_RUN_NAME(UKG_NAME)(const ukg_oddeven_run& r)
 namespace {
 
 /* Launch tuning (kalman_gpu_set_tuning): process-wide, read once at the
- * start of every call.  Defaults: a thread per item below 9 states, a thread
- * block per item from 9 on; four CTAs per SM; the block sizes the FP32
- * kernels were written for.                                                  */
+ * start of every call.  Defaults: lanes or a thread per item below 9 states, a
+ * thread block per item from 9 on; four CTAs per SM where a kernel has a
+ * persistent grid; the block sizes the FP32 kernels were written for.        */
 kalman_gpu_tuning_t default_tuning() { return kalman_gpu_tuning_t{9, 4, kPairBP, kWeighBS}; }
 std::mutex g_tune_mu;
 kalman_gpu_tuning_t g_tune = default_tuning();
