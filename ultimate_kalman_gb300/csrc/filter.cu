@@ -1,13 +1,15 @@
 /*
  * filter.cu -- filtered estimates on the device: the sequential UltimateKalman
  * filter (c/kalman_ultimate.c: evolve 140-345, observe 347-557 with its
- * estimate 508-545) run for every track of a packed problem at once, one
- * thread block per track (kalman_gpu_filter_packed).  The reference keeps the
- * covariance as the factor R (its covariance_type 'W'); here P = R^{-1} R^{-T}
- * is written explicitly, as the smoothers write theirs.
+ * estimate 508-545) run for every track of a packed problem at once
+ * (kalman_gpu_filter_packed): a warp per track and three kernels up to 8 states
+ * and observation rows (below), a thread block per track (filter_cta) from there
+ * on.  The reference keeps the covariance as the factor R (its covariance_type
+ * 'W'); here P = R^{-1} R^{-T} is written explicitly, as the smoothers write
+ * theirs.
  *
- * Per track the block keeps the factor of the current state's information,
- * an upper-trapezoidal R (z rows, z <= n) and its right-hand side y:
+ * Kept per track is the factor of the current state's information, an
+ * upper-trapezoidal R (z rows, z <= n) and its right-hand side y:
  *   evolve to step i   QR, eliminating x_{i-1}, of
  *                        [ R        0     | y    ]   (z rows)
  *                        [ -V F_i   V H_i | V c_i ]   (n rows; V from K_i)
@@ -17,8 +19,8 @@
  *                      z = min(z + m_i, n) rows;
  *   estimate           x_{i|i} = R^{-1} y and P_{i|i} = R^{-1} R^{-T} once
  *                      z = n (NaN before, as the reference's estimate).
- * The QR reductions, weighing and triangular solves are the CTA routines of
- * the smoothers (cta_linalg.cuh).  FP64.
+ * filter_cta's QR reductions, weighing and triangular solves are the CTA
+ * routines of the smoothers (cta_linalg.cuh).  FP64.
  */
 #include <algorithm>
 #include <cmath>
@@ -242,7 +244,7 @@ struct ThreadWeights {
         for (int k = 0; k < j; ++k) s = fma(-L[k][j], L[k][j], s);
         const bool pd = s > 0.0;
         if (j < rows && !pd) ok = false;
-        d[j] = !pd ? 1.0 : lanes::series_range(s) ? lanes::rsqrt_series(s) : 1.0 / sqrt(s);
+        d[j] = pd ? lanes::inv_root(s) : 1.0;
 #pragma unroll
         for (int i = j + 1; i < R; ++i) {
           double x = L[j][i];

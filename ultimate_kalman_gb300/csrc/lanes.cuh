@@ -1,8 +1,8 @@
 /*
  * lanes.cuh -- Householder QR of a small panel whose columns lie on the lanes
- * of a warp (or of an eighth or a quarter of one), in registers, for FP64 and
- * double-float: shared by the odd-even smoother, the associative smoother and
- * the filter for up to 8 states.
+ * of a warp (or of a quarter of one), in registers, for FP64, double-float and
+ * FP32: shared by the odd-even smoother, the associative smoother and the filter
+ * for up to 8 states.
  *
  * On GB300 an FP64 instruction of a warp occupies its scheduler's quarter of
  * the SM for 64 cycles, whether 1 or 32 lanes take part (measured), so what
@@ -49,7 +49,7 @@ __device__ __forceinline__ T inv_root(T s) { return T(1) / sqrt(s); }
 template <>
 __device__ __forceinline__ double inv_root<double>(double s)
 {
-  return series_range(s) ? rsqrt_series(s) : 1.0 / sqrt(s);
+  return series_range(s) ? rsqrt_series(s) : rsqrt(s); /* either within one unit in the last place */
 }
 
 /* The reflector that maps (alpha, x) to (beta, 0), tail = x^T x != 0, as
