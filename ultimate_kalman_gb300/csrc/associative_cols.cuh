@@ -130,7 +130,7 @@ __device__ bool solve_half(double* dyn, SquareShared<NP>& sm, int n, int which, 
 #pragma unroll
     for (int r = 0; r < NP; ++r) b[r] = r < n ? p[r * st] : 0.0;
   }
-  qr_square<NP>(sm, 0, act, g ? n + q : q, n, b);
+  qr_square<NP>(sm, act, g ? n + q : q, n, b);
   bool bad = false;
   if (g == 0) {
     put_end<NP>(R + q * n, n, b);
@@ -340,7 +340,7 @@ __device__ __noinline__ bool explicit_rows(char kt, const double* K, int n, doub
   bool bad = false;
   if (kt == 'W') { /* K = (W^T W)^{-1} = U U^T, U = (W's R factor)^{-1} */
     load_rows<double, NP>(K + (int64_t)q * n, n, g == 0, b);
-    qr_square<NP>(sm, 0, g == 0, q, n, b);
+    qr_square<NP>(sm, g == 0, q, n, b);
     if (g == 0) put_end<NP>(S + q * n, n, b);
     if (g == 0) {
       const double d = S[q * n + q];
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(threads2<NP>(), NP <= 32 ? blocks2<NP>() : NP 
   if (act) matvec_half<NP>(S, n, g, b, [&](int l) { return F[(int64_t)l * n + q]; });
   join<NP>(w, n, act, g, b);
   if (g == 1) load_rows<double, NP>(S + q * n, n, true, b);
-  qr_square<NP>(sm, 0, act, g == 1 ? n + q : q, n, b);
+  qr_square<NP>(sm, act, g == 1 ? n + q : q, n, b);
   if (g == 0) {
     put_end<NP>(R + q * n, n, b);
     const double d = R[q * n + q];

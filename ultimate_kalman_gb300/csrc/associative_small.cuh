@@ -1,8 +1,8 @@
 /*
  * associative_small.cuh -- the scans of the associative smoother for up to 8
  * states, a warp (or half of one) per combine, up to 5 states a thread where
- * there are many.  Included by associative.cu (it
- * uses that file's FElems, SElems, ScanLevel and find_track).
+ * there are many.  Included by associative.cu (it uses that file's FElems,
+ * SElems, ScanLevel and find_track).
  *
  * A thread that combines two elements alone is a chain of some 2,700 FP64
  * instructions of 64 cycles (175 us a level, whatever its size); with a matrix

@@ -83,16 +83,16 @@ __device__ __forceinline__ void matvec(const double* M, int n, double (&b)[NP], 
   }
 }
 
-/* Householder QR of square panels (n x n pivots on the columns 0..n-1 of up to
- * two panels), FP64.  Row k is the first of b at step k; done, it goes to the
+/* Householder QR of a square panel (n x n pivots on the columns 0..n-1 and
+ * further columns), FP64.  Row k is the first of b at step k; done, it goes to the
  * end, so after n steps a column's entries are in order, aligned to the end:
  * R (whose entries below the diagonal mean nothing) and Q^T of the others.   */
 template <int NP>
 struct SquareShared {
-  double x[2][2][NP], amb[2][2], inv[2][2];
+  double x[2][NP], amb[2], inv[2]; /* by the step's parity */
 };
 template <int NP>
-__device__ __forceinline__ void qr_square(SquareShared<NP>& sm, int panel, bool act, int c, int n, double (&b)[NP])
+__device__ __forceinline__ void qr_square(SquareShared<NP>& sm, bool act, int c, int n, double (&b)[NP])
 {
 #pragma unroll 1
   for (int k = 0; k < n; ++k) {
@@ -100,7 +100,7 @@ __device__ __forceinline__ void qr_square(SquareShared<NP>& sm, int panel, bool 
     double t = b[0];
 #pragma unroll
     for (int i = 0; i + 1 < NP; ++i) b[i] = b[i + 1];
-    double* x = sm.x[buf][panel];
+    double* x = sm.x[buf];
     const bool pivot = act && c == k;
     if (pivot)
 #pragma unroll
@@ -125,12 +125,12 @@ __device__ __forceinline__ void qr_square(SquareShared<NP>& sm, int panel, bool 
       r.beta = t;
       r.amb = r.inv = 0.0;
       if (dot != 0.0) r = lanes::reflector(t, dot);
-      sm.amb[buf][panel] = r.amb;
-      sm.inv[buf][panel] = r.inv;
+      sm.amb[buf] = r.amb;
+      sm.inv[buf] = r.inv;
       t = r.beta;
     }
     __syncthreads();
-    const double amb = sm.amb[buf][panel], inv = sm.inv[buf][panel];
+    const double amb = sm.amb[buf], inv = sm.inv[buf];
     if (on && !pivot && amb != 0.0) {
       const double d = fma(amb, t, dot) * inv;
       t = fma(-d, amb, t);

@@ -1,8 +1,8 @@
 /*
- * oddeven_small.cuh -- the odd-even smoother's FP64 and double-float kernels
- * for up to 8 states (and no more observation rows than states), in two
- * mappings with the same arithmetic, entry by entry.  Included by oddeven.cu
- * (it uses that file's Args, tables and views).
+ * oddeven_small.cuh -- the odd-even smoother's kernels for 2 to 8 states (and no
+ * more observation rows than states), in FP64, double-float and FP32 (whose
+ * solves are oddeven.cu's), in two mappings with the same arithmetic, entry by
+ * entry.  Included by oddeven.cu (it uses that file's Args, tables and views).
  *
  *   *_lanes   a group of LPI lanes (32 or 8) shares a work item, a column of
  *             the current panel per lane and slot, in registers; reflectors
