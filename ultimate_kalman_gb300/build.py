@@ -24,11 +24,13 @@ SOURCES = ["oddeven.cu", "associative.cu", "builder.cu", "filter.cu", "profiling
 # oddeven.cu's kernels by arithmetic type, a compilation each
 PARTS = {"oddeven.cu": [("f32", "float"), ("f64", "double"), ("df", "ukg_df::dd")]}
 # --split-compile=0: nvcc optimizes a translation unit's kernels in parallel on every
-# core.  That gives other registers and spills at every build of the same source (the
-# residual of 6 states took 46 or 63 us), and slower FP32 and double-float pairs (8.8
-# instead of 8.1 ms at 128 states), so those two are compiled without; the FP64
-# back-substitutions and scans are 15 to 25 % faster with it, build after build.
+# core.  That gives other code at every build of the same source (the residual of 6
+# states took 46 or 63 us, the scans of 48 states 50 or 60 ms), so what it does not speed
+# up every time is compiled without: the FP32 and double-float parts (pairs of 128
+# states 8.8 ms with, 8.1 without) and the associative smoother.  The FP64 part keeps it:
+# its back-substitutions of 16 states and of 65 and more are 20 % slower without.
 SPLIT = ["--split-compile=0"]
+WHOLE = ("associative.cu",)
 
 
 def nvcc():
@@ -69,7 +71,7 @@ def build(verbose=False, force=False):
         name = os.path.basename(src)
         for tag, t in PARTS.get(name, []):
             units.append((src, f"{name}.{tag}", [f"-DUKG_NAME={tag}", f"-DUKG_TYPE={t}"] + (SPLIT if tag == "f64" else [])))
-        units.append((src, name, SPLIT if src.endswith(".cu") else []))
+        units.append((src, name, SPLIT if src.endswith(".cu") and name not in WHOLE else []))
     with cf.ThreadPoolExecutor(max_workers=len(units)) as ex:
         results = list(ex.map(lambda u: _compile(u, verbose), units))
     if verbose:
