@@ -1,7 +1,8 @@
-"""The thread-per-column kernels (9 to 64 states, 96 in the precision form) at
-the edges of their register sizes (12, 16, 24, 32, 48, 64, 96 rows) against
-the oracle: every covariance type, unobserved steps (the trapezoids then run
-out of rows), odd and even lengths.  Bars as elsewhere: 1e-11 in FP64, 1e-9
+"""The thread-per-column kernels (9 to 64 states) at the edges of their register
+sizes (12, 16, 24, 32, 48, 64 rows) and the precision form's kernels of four
+columns by a quarter of the rows per thread (65 to 128 states; to 96 and to 128
+rows) against the oracle: every covariance type, unobserved steps (the
+trapezoids then run out of rows), odd and even lengths.  Bars as elsewhere: 1e-11 in FP64, 1e-9
 in the precision form and in double-float."""
 import numpy as np
 import pytest
@@ -62,7 +63,7 @@ def test_associative_register_sizes(n, m, cov):
 @pytest.mark.parametrize("n,m,cov", [(97, 97, "C"), (99, 1, "w"), (100, 40, "W"), (113, 112, "C"), (127, 20, "F"),
                                      (128, 128, "C"), (128, 64, "W"), (120, 128, "C")])
 def test_two_pass_sizes(n, m, cov):
-    """97 to 128 states in the precision form: pivots first, the other columns after."""
+    """97 to 128 states in the precision form: 32 rows a lane, three passes a pair."""
     P = pb.random_dynamics([1, 2, 7, 12, 13], n, m, seed=n + m, K_type=cov, C_type=cov, missing=0.3, per_step=True)
     st, Xo, So = oracle.smooth(P, "oddeven")
     assert st == 0

@@ -243,9 +243,10 @@ def test_bulk_structs_through_the_batched_reference_entry_equal_the_packed_path(
 
 @pytest.mark.parametrize("n,m", [(4, 2), (6, 3), (6, 6)])
 def test_register_tiled_covariance_solve_at_every_level(n, m, parity_log):
-    """n = 4 and 6 run the covariance back-substitution register-tiled
-    (solve_cov_reg_kernel): FP64 and double-float against the oracle at
-    every recursion parity pattern, with missing observations."""
+    """n = 4 and 6 run the covariance back-substitution in registers, by lanes
+    or by threads (small::solve_lanes, small::solve_thread): FP64 and
+    double-float against the oracle at every recursion parity pattern, with
+    missing observations."""
     lens = [1, 2, 3, 5, 8, 17, 33, 64, 129, 700]
     P = (pb.constant_velocity(lens, seed=51, missing=0.1) if (n, m) == (6, 3)
          else pb.random_dynamics(lens, n, m, seed=52 + n + m, missing=0.1))

@@ -11,7 +11,7 @@
  * warp instructions at n = 48 (a third of them the reductions); at 19 cycles an
  * SM each that bounds the large levels, and the chain of n reflectors and four
  * half products the small ones.  5,000 steps, n = 48, m = 24: scans 74.5 ms
- * before, 50.4 now, smoothing elements 9.9 and 7.5.
+ * before, 51.5 now, smoothing elements 9.9 and 8.2.
  */
 #pragma once
 #include "columns.cuh"
