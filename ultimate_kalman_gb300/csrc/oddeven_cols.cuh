@@ -12,9 +12,9 @@
  * few items a level it is the chain of 2 n reflectors, 50 us.  Measured, ms,
  * pairs / back-substitution / weighing, before and now:
  *   16 tracks of 64 to 4,000 steps, n = 12  FP64   7.2 2.0 1.5    2.2 1.1 0.7
- *   2,000 steps, n = 48                     FP64   22.7 8.4 1.6   10.8 6.2 2.3
- *                                           df     16.6 9.9 1.0   4.9 6.5 1.2
- *   4,000 steps, n = 64, states             FP32   8.9 1.0 1.5    4.1 0.4 1.7
+ *   2,000 steps, n = 48                     FP64   22.7 8.4 1.6   10.8 6.3 2.3
+ *                                           df     16.6 9.9 1.0   4.8 4.5 1.1
+ *   4,000 steps, n = 64, states             FP32   8.9 1.0 1.5    3.9 0.4 2.1
  * (the weighing now includes the triangularization).
  *
  * Structure.  Every observation block is upper trapezoidal: the weighing
