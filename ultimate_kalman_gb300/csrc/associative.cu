@@ -26,11 +26,12 @@
  * Up to 8 states an element is built by one thread, its n x n temporaries in
  * shared memory, interleaved across the block's threads (element e of thread t
  * at smem[e*blockDim + t]), and combined by a warp, or up to 5 states and with
- * many combines by a thread (associative_small.cuh); from 9 to 64 a combine and a smoothing element take a thread block with a
- * column per thread (associative_cols.cuh), filtering elements and larger states a
- * block with its panels in global scratch (associative_cta.cuh).  Up to 8 states
- * element arrays are element-major (SoA) so that consecutive threads touch
- * consecutive addresses.
+ * many combines by a thread (associative_small.cuh); from 9 to 64 a combine
+ * and a smoothing element take a thread block with a column per thread
+ * (associative_cols.cuh), filtering elements and larger states a block with its
+ * panels in global scratch (associative_cta.cuh).  Up to 8 states element
+ * arrays are element-major (SoA) so that consecutive threads touch consecutive
+ * addresses.
  */
 #include <cuda_runtime.h>
 
